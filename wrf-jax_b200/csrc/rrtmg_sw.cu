@@ -1139,12 +1139,15 @@ __constant__ int kSwGofsDev[kSwBands] = {0, 6, 18, 26, 34, 44, 54, 56, 66, 74, 8
 
 constexpr int kSweepCols = 2;                         // day columns per block
 constexpr int kSweepThreads = kSweepCols * kSwGpts;   // 224: one thread per g-point
-constexpr int kRing = 8;                              // levels of terms per ordered-sum round
+constexpr int kRingRows = 32;                         // level terms per ordered-sum round: (level, type, column)
+constexpr int kRingStride = kSwGpts + 4;              // floats per row: 29 16-byte chunks, odd, so that the lanes
+                                                      // of a 16-byte read of 32 rows meet no bank conflict
+static_assert(kRingStride % 4 == 0 && (kRingStride / 4) % 2 == 1, "ring rows");
 
-// Shared memory of a sweep block: the level terms of the last kRing levels of
-// the current pass, awaiting their g-ordered sums, and the sums themselves.
+// Shared memory of a sweep block: two buffers of level terms awaiting their
+// g-ordered sums (one is summed while the other fills), and the sums.
 struct SweepShared {
-  float ring[kRing][kSweepCols][4][kSwGpts];
+  float ring[2][kRingRows][kRingStride];
   float sums[kSweepCols][6][kMaxLev];  // type: fu, fd, cu, cd, fdir, cdir; level top-down
   uint32_t slotbits[2][kMaxLay / 32][kSweepThreads];  // per thread: cloudy slots, total = clear slots
 };
@@ -1157,26 +1160,34 @@ struct SwLevel {
   float4 dn;   // dbt, tdbt, tdn, rdnd
 };
 
-// Adds ring rounds into the sums: chain (column, type, level) adds the 112
-// terms of its level in g-point order, starting from zero as the
-// reference's ordered sums do (sw:153-177).  `levels[j]` is the level of ring
-// slot j, `types` the sums' type indices of the pass's ring types.
-__device__ __forceinline__ void sweep_flush(SweepShared &S, int count, int ntypes, const int *types, int level0,
-                                            int dir) {
+// Ordered sums of one full (or last) ring buffer: row (j, q, c) = level j of
+// the round, term type q, column c holds the 112 terms of one level sum, and
+// one lane adds them in g-point order, starting from zero as the reference's
+// ordered sums do (sw:153-177).  One warp per round does it, the block's warps
+// in turn, while the others fill the other buffer: the barrier here says that
+// this buffer is full and that the other one's sums (of the previous round)
+// are done, so a round costs one barrier.  Before: two barriers around a sum
+// by 32 or 64 threads, whose rows lay 112 floats apart, a 16-way bank conflict;
+// sweep of a 425 x 425 x 50 call 26.6 -> 25.9 ms, of a 64 x 64 x 44 call 0.62 ->
+// 0.60 ms.
+template <int NTYPES>
+__device__ __forceinline__ void sweep_flush(SweepShared &S, int round, int count, int type0, int level0, int dir) {
   __syncthreads();
-  const int chains = kSweepCols * ntypes * count;
-  for (int ch = threadIdx.x; ch < chains; ch += kSweepThreads) {
-    const int j = ch % count;
-    const int rest = ch / count;
-    const int q = rest % ntypes;
-    const int c = rest / ntypes;
-    const float *v = S.ring[j][c][q];
-    float acc = 0.0f;
-#pragma unroll 16
-    for (int G = 0; G < kSwGpts; ++G) acc = acc + v[G];
-    S.sums[c][types[q]][level0 + dir * j] = acc;
+  if (static_cast<int>(threadIdx.x >> 5) != round % (kSweepThreads / 32)) return;
+  const int row = threadIdx.x & 31;
+  const int c = row % kSweepCols, q = row / kSweepCols % NTYPES, j = row / (kSweepCols * NTYPES);
+  if (j >= count) return;
+  const float4 *v = reinterpret_cast<const float4 *>(S.ring[round & 1][row]);
+  float acc = 0.0f;
+#pragma unroll 7
+  for (int i = 0; i < kSwGpts / 4; ++i) {
+    const float4 x = v[i];
+    acc = acc + x.x;
+    acc = acc + x.y;
+    acc = acc + x.z;
+    acc = acc + x.w;
   }
-  __syncthreads();
+  S.sums[c][type0 + q][level0 + dir * j] = acc;
 }
 
 // Block = kSweepCols consecutive slots of the chunk; thread = (slot, g-point).
@@ -1230,12 +1241,15 @@ __global__ void __launch_bounds__(kSweepThreads, kSwSweepMinBlocks) sw_sweep_ker
   uint32_t cloudy_bits = 0, same_word = 0;
 
   // ---- top-down pass: layer optics, direct beam, downward adding (sw:6887-7041)
-  const int dtypes[2] = {4, 5};
   float tdbtc_nd = 1.0f, tdbt_nd = 1.0f;
   const float zincflx = ((C.adjflux * sflux_g) * mu) * 1.0f;
-  S.ring[0][cslot][0][G] = tdbt_nd * zincflx;
-  S.ring[0][cslot][1][G] = tdbtc_nd * zincflx;
-  int filled = 1, level0 = 0;
+  // ring position of this thread's terms: row (level * types + type) * columns + column
+  float *const ring0 = &S.ring[0][cslot][G];
+  constexpr int kTypeStep = kSweepCols * kRingStride, kBufStep = kRingRows * kRingStride;
+  constexpr int kDownLevels = kRingRows / (2 * kSweepCols), kUpLevels = kRingRows / (4 * kSweepCols);
+  ring0[0] = tdbt_nd * zincflx;
+  ring0[kTypeStep] = tdbtc_nd * zincflx;
+  int filled = 1, level0 = 0, round = 0;
   // carry of the downward recurrence: level r values of each path
   float c_tdbt = 1.0f, c_tdn = 1.0f, c_rdnd = 0.0f;
   float t_tdbt = 1.0f, t_tdn = 1.0f, t_rdnd = 0.0f;
@@ -1368,17 +1382,20 @@ __global__ void __launch_bounds__(kSweepThreads, kSwSweepMinBlocks) sw_sweep_ker
       cloudy_bits = 0;
       same_word = 0;
     }
-    S.ring[filled][cslot][0][G] = tdbt_nd * zincflx;
-    S.ring[filled][cslot][1][G] = tdbtc_nd * zincflx;
-    if (++filled == kRing || r == n - 1) {
-      sweep_flush(S, filled, 2, dtypes, level0, 1);
+    {
+      float *q = ring0 + (round & 1) * kBufStep + filled * (2 * kTypeStep);
+      q[0] = tdbt_nd * zincflx;
+      q[kTypeStep] = tdbtc_nd * zincflx;
+    }
+    if (++filled == kDownLevels || r == n - 1) {
+      sweep_flush<2>(S, round, filled, 4, level0, 1);
+      ++round;
       level0 += filled;
       filled = 0;
     }
   }
 
   // ---- bottom-up pass: upward adding and level fluxes (vrtqdr, sw:3655-3720)
-  const int utypes[4] = {0, 1, 2, 3};
   // surface albedos of this g-point's band: direct (albp) and diffuse (albd);
   // the Noah-MP fields, when given, for columns with xland < 1.5 (sw:2519-2530):
   // visible in bands 25-28, near infrared in 16-24 and 29 (sw:2120-2127)
@@ -1439,18 +1456,24 @@ __global__ void __launch_bounds__(kSweepThreads, kSwSweepMinBlocks) sw_sweep_ker
       fut = (t.dn.y * rupt + (t.dn.z - t.dn.y) * rupdt) * zreft;
       fdt = t.dn.y + (t.dn.z - t.dn.y + t.dn.y * rupt * t.dn.w) * zreft;
     }
-    S.ring[filled][cslot][0][G] = fut * zincflx;
-    S.ring[filled][cslot][1][G] = fdt * zincflx;
-    S.ring[filled][cslot][2][G] = fuc * zincflx;
-    S.ring[filled][cslot][3][G] = fdc * zincflx;
-    if (++filled == kRing || k == 0) {
-      sweep_flush(S, filled, 4, utypes, level0, -1);
+    {
+      float *q = ring0 + (round & 1) * kBufStep + filled * (4 * kTypeStep);
+      q[0] = fut * zincflx;
+      q[kTypeStep] = fdt * zincflx;
+      q[2 * kTypeStep] = fuc * zincflx;
+      q[3 * kTypeStep] = fdc * zincflx;
+    }
+    if (++filled == kUpLevels || k == 0) {
+      sweep_flush<4>(S, round, filled, 0, level0, -1);
+      ++round;
       level0 -= filled;
       filled = 0;
     }
     c = nc;
     t = nt;
   }
+
+  __syncthreads();  // the last round's sums
 
   // ---- outputs of the block's live columns (sw:2285-2301, 2536-2719)
   for (int q = threadIdx.x; q < kSweepCols * kMaxLay; q += kSweepThreads) {
