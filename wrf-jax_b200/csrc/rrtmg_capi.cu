@@ -37,6 +37,11 @@ struct rrtmg_ctx {
   std::vector<unsigned char> host_blob;
   std::map<std::string, Entry> entries;
   void *dev_blob = nullptr;
+  // the gas optics' tables in their padded layout (one allocation), and while
+  // the context is made the host copy and the pointers into it
+  float *dev_padded = nullptr;
+  std::vector<float> padded;
+  std::vector<std::pair<const float **, size_t>> padded_refs;
   Tables tables{};
   std::mutex mutex;
   std::string last_error;
@@ -211,6 +216,41 @@ const T *host_ptr(rrtmg_ctx *ctx, const std::string &name, int *count = nullptr)
   return reinterpret_cast<const T *>(ctx->host_blob.data() + it->second.offset);
 }
 
+// Appends table `name` to the padded tables and notes that *out points to it
+// (null where the blob has no such table); returns its rows.  The blob holds
+// (rows, ngc), or (ngc, columns) where `transposed`; the copy has rows of
+// `pad` g-points and `edge` copies of its first and last row on either side.
+int add_padded(rrtmg_ctx *ctx, const std::string &name, int ngc, int pad, const float **out, int edge = 0,
+               bool transposed = false) {
+  *out = nullptr;
+  int n = 0;
+  const float *src = host_ptr<float>(ctx, name, &n);
+  const int rows = n / ngc;
+  if (!src || rows == 0) return 0;
+  std::vector<float> &dst = ctx->padded;
+  const size_t base = (dst.size() + 63) / 64 * 64;
+  dst.resize(base + static_cast<size_t>(rows + 2 * edge) * pad, 0.0f);
+  for (int r = -edge; r < rows + edge; ++r) {
+    const int from = r < 0 ? 0 : (r >= rows ? rows - 1 : r);
+    for (int g = 0; g < ngc; ++g)
+      dst[base + static_cast<size_t>(r + edge) * pad + g] = transposed ? src[g * rows + from] : src[from * ngc + g];
+  }
+  ctx->padded_refs.emplace_back(out, base + static_cast<size_t>(edge) * pad);
+  return rows;
+}
+
+// Copies the padded tables to the device and sets the pointers to them.
+cudaError_t upload_padded(rrtmg_ctx *ctx) {
+  const size_t bytes = ctx->padded.size() * sizeof(float);
+  cudaError_t e = cudaMalloc(&ctx->dev_padded, bytes);
+  if (e == cudaSuccess) e = cudaMemcpy(ctx->dev_padded, ctx->padded.data(), bytes, cudaMemcpyHostToDevice);
+  if (e != cudaSuccess) return e;
+  for (auto &ref : ctx->padded_refs) *ref.first = ctx->dev_padded + ref.second;
+  std::vector<float>().swap(ctx->padded);
+  ctx->padded_refs.clear();
+  return cudaSuccess;
+}
+
 // Ozone climatology work profile (module_ra_rrtmg_common.py:343-372), binary32.
 void o3_work_profile(rrtmg_ctx *ctx, float *o3wrk, float *ppwrkh) {
   const float *o3sum = host_ptr<float>(ctx, "o3sum");
@@ -239,31 +279,30 @@ bool fill_tables(rrtmg_ctx *ctx, std::string &err) {
   for (int b = 0; b < kLwBands; ++b) {
     const std::string p = "lw" + std::to_string(b + 1) + ".";
     LwBand &B = T.lw[b];
-    int n = 0;
-    B.ka = dev_ptr<float>(ctx, p + "ka", &n);
-    B.ka_rows = n / lw_ngc[b];
-    B.kb = dev_ptr<float>(ctx, p + "kb", &n);
-    B.kb_rows = B.kb ? n / lw_ngc[b] : 0;
-    B.fracrefa = dev_ptr<float>(ctx, p + "fracrefa");
-    B.fracrefb = dev_ptr<float>(ctx, p + "fracrefb");
-    B.selfref = dev_ptr<float>(ctx, p + "selfref");
-    B.forref = dev_ptr<float>(ctx, p + "forref");
-    B.ka_mn2 = dev_ptr<float>(ctx, p + "ka_mn2");
-    B.kb_mn2 = dev_ptr<float>(ctx, p + "kb_mn2");
-    B.ka_mn2o = dev_ptr<float>(ctx, p + "ka_mn2o");
-    B.kb_mn2o = dev_ptr<float>(ctx, p + "kb_mn2o");
-    B.ka_mo3 = dev_ptr<float>(ctx, p + "ka_mo3");
-    B.kb_mo3 = dev_ptr<float>(ctx, p + "kb_mo3");
-    B.ka_mco2 = dev_ptr<float>(ctx, p + "ka_mco2");
-    B.kb_mco2 = dev_ptr<float>(ctx, p + "kb_mco2");
-    B.ka_mco = dev_ptr<float>(ctx, p + "ka_mco");
-    B.ka_mo2 = dev_ptr<float>(ctx, p + "ka_mo2");
-    B.kb_mo2 = dev_ptr<float>(ctx, p + "kb_mo2");
-    B.ccl4 = dev_ptr<float>(ctx, p + "ccl4");
-    B.cfc11adj = dev_ptr<float>(ctx, p + "cfc11adj");
-    B.cfc12 = dev_ptr<float>(ctx, p + "cfc12");
-    B.cfc22adj = dev_ptr<float>(ctx, p + "cfc22adj");
-    if (!B.ka || !B.fracrefa || !B.selfref || !B.forref) {
+    auto add = [&](const char *name, const float **out, int edge = 0, bool transposed = false) {
+      return add_padded(ctx, p + name, lw_ngc[b], lw_pad(b), out, edge, transposed);
+    };
+    B.ka_rows = add("ka", &B.ka, kPadRows);
+    B.kb_rows = add("kb", &B.kb, kPadRows);
+    const bool have_fracs = add("fracrefa", &B.fracrefa, 0, true) > 0;
+    add("fracrefb", &B.fracrefb, 0, true);
+    const bool have_continuum = (add("selfref", &B.selfref) > 0) & (add("forref", &B.forref) > 0);
+    add("ka_mn2", &B.ka_mn2);
+    add("kb_mn2", &B.kb_mn2);
+    add("ka_mn2o", &B.ka_mn2o);
+    add("kb_mn2o", &B.kb_mn2o);
+    add("ka_mo3", &B.ka_mo3);
+    add("kb_mo3", &B.kb_mo3);
+    add("ka_mco2", &B.ka_mco2);
+    add("kb_mco2", &B.kb_mco2);
+    add("ka_mco", &B.ka_mco);
+    add("ka_mo2", &B.ka_mo2);
+    add("kb_mo2", &B.kb_mo2);
+    add("ccl4", &B.ccl4);
+    add("cfc11adj", &B.cfc11adj);
+    add("cfc12", &B.cfc12);
+    add("cfc22adj", &B.cfc22adj);
+    if (B.ka_rows == 0 || !have_fracs || !have_continuum) {
       err = "table blob lacks longwave band " + std::to_string(b + 1);
       return false;
     }
@@ -426,6 +465,13 @@ rrtmg_status finish_create(rrtmg_ctx *ctx, int device, rrtmg_ctx **out) {
     delete ctx;
     return fail(nullptr, RRTMG_BAD_ARG, err);
   }
+  e = upload_padded(ctx);
+  if (e != cudaSuccess) {
+    cudaFree(ctx->dev_padded);
+    cudaFree(ctx->dev_blob);
+    delete ctx;
+    return cuda_fail(nullptr, e, "cudaMalloc(padded tables)");
+  }
   cudaMemPoolProps props{};
   props.allocType = cudaMemAllocationTypePinned;
   props.location.type = cudaMemLocationTypeDevice;
@@ -437,6 +483,7 @@ rrtmg_status finish_create(rrtmg_ctx *ctx, int device, rrtmg_ctx **out) {
   }
   if (e != cudaSuccess) {
     if (ctx->pool) cudaMemPoolDestroy(ctx->pool);
+    cudaFree(ctx->dev_padded);
     cudaFree(ctx->dev_blob);
     delete ctx;
     return cuda_fail(nullptr, e, "cudaMemPoolCreate(scratch pool)");
@@ -519,6 +566,7 @@ void rrtmg_destroy(rrtmg_ctx *ctx) {
   for (float *p : ctx->retired_ozone) cudaFree(p);
   for (uint32_t *p : ctx->status_buf) cudaFree(p);
   for (uint32_t *p : ctx->retired_status) cudaFree(p);
+  cudaFree(ctx->dev_padded);
   cudaFree(ctx->dev_blob);
   if (ctx->pool) cudaMemPoolDestroy(ctx->pool);
   for (auto &side : ctx->events)

@@ -23,6 +23,19 @@ constexpr int kMaxBuf = 40;       // LW buffer layers above the model top
 constexpr int kLwMaskWords = 5;   // ceil(140 / 32)
 constexpr int kSwMaskWords = 4;   // ceil(112 / 32)
 
+// Padded table layout of the gas optics, built once per context: each row's
+// g-points are padded with zeros to a multiple of four, and the absorption
+// tables ka / kb repeat their first and last row kPadRows times on either
+// side, so that rows r .. r + 11 of a row index clamped to [-kPadRows, rows]
+// are the reference's rows clamped one by one.
+constexpr int kPadRows = 12;
+__host__ __device__ constexpr int lw_pad(int band) {
+  constexpr int pad[kLwBands] = {12, 12, 16, 16, 16, 8, 12, 8, 12, 8, 8, 8, 4, 4, 4, 4};
+  return pad[band];
+}
+
+// Longwave band tables in the padded layout; the Planck fractions of several
+// species ratios as (ratio, g-point).
 struct LwBand {
   const float *fracrefa, *fracrefb, *ka, *kb, *selfref, *forref;
   const float *ka_mn2, *kb_mn2, *ka_mn2o, *kb_mn2o, *ka_mo3, *kb_mo3;
