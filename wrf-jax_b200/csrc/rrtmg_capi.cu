@@ -359,6 +359,18 @@ bool fill_tables(rrtmg_ctx *ctx, std::string &err) {
   T.lw_ntbl = n - 1;
   T.lw_pade_exp = dev_ptr<float>(ctx, "lw.pade_exp_tbl");
   T.lw_pade_tfn = dev_ptr<float>(ctx, "lw.pade_tfn_tbl");
+  {
+    const float *ex = host_ptr<float>(ctx, "lw.pade_exp_tbl"), *tfn = host_ptr<float>(ctx, "lw.pade_tfn_tbl");
+    if (ex && tfn && n > 0) {
+      const size_t base = (ctx->padded.size() + 63) / 64 * 64;
+      ctx->padded.resize(base + 2 * static_cast<size_t>(n));
+      for (int i = 0; i < n; ++i) {
+        ctx->padded[base + 2 * i] = 1.0f - ex[i];
+        ctx->padded[base + 2 * i + 1] = tfn[i];
+      }
+      ctx->padded_refs.emplace_back(reinterpret_cast<const float **>(&T.lw_pade), base);
+    }
+  }
   const float *bp = host_ptr<float>(ctx, "lw.pade_bpade");
   T.lw_bpade = bp ? bp[0] : 0.0f;
   T.sw_preflog = dev_ptr<float>(ctx, "sw.preflog");
@@ -387,6 +399,10 @@ bool fill_tables(rrtmg_ctx *ctx, std::string &err) {
       !T.sw_preflog || !T.extliq1 || !T.extice3 || !T.sw_pade_exp || !T.retab || !T.pprof || !T.tprof ||
       !T.logf_tab || !lp || !T.expf_tab || !ep || !host_ptr<float>(ctx, "o3sum")) {
     err = "table blob is missing required tables";
+    return false;
+  }
+  if (T.lw_ntbl > kLwPadeMax) {
+    err = "longwave Pade tables have too many positions";
     return false;
   }
   T.logf_ln2 = lp[0];

@@ -22,6 +22,7 @@ constexpr int kMaxLay = 128;      // layers per column the kernels accept
 constexpr int kMaxBuf = 40;       // LW buffer layers above the model top
 constexpr int kLwMaskWords = 5;   // ceil(140 / 32)
 constexpr int kSwMaskWords = 4;   // ceil(112 / 32)
+constexpr int kLwPadeMax = 32767;  // highest Pade table position (the tables of RRTMG have 10,000)
 
 // Padded table layout of the gas optics, built once per context: each row's
 // g-points are padded with zeros to a multiple of four, and the absorption
@@ -59,6 +60,7 @@ struct Tables {
   const float *lw_preflog, *lw_tref, *chi_mls, *totplnk;
   const float *absice3, *absliq1;
   const float *lw_pade_tau, *lw_pade_exp, *lw_pade_tfn;
+  const float2 *lw_pade;  // (1 - exp, tfn) of each position
   float lw_bpade;
   int lw_ntbl;
   // shortwave reference atmosphere, cloud optics, Pade table

@@ -43,16 +43,20 @@ namespace {
 
 // Layer record (kLwRec floats): taug of each band's g-points from a 16-byte
 // boundary (kLwPadOfs), the Planck fractions likewise from kLwRecFracs, per
-// band (blay, dplankup, dplankdn, cloud optical depth) from kLwRecBand, and
-// the layer's cloud flag at kLwRecFlags.
+// band (blay, dplankup, dplankdn, cloud optical depth along the diffusivity
+// angle) from kLwRecBand and the cloud's absorptance from kLwRecEfcl, and from
+// kLwRecFlags the layer's cloud flag and McICA mask words.  The sweep's
+// downward pass leaves its transfer-table positions in place of the optical
+// depths for the upward pass (lw_down).
 constexpr int kLwPadOfs[kLwBands] = {0, 12, 24, 40, 56, 72, 80, 92, 100, 112, 120, 128, 136, 140, 144, 148};
 constexpr int kLwPadG = 152;
 static_assert(kLwPadOfs[kLwBands - 1] + lw_pad(kLwBands - 1) == kLwPadG, "padded g-points");
-constexpr int kLwRecFracs = kLwPadG, kLwRecBand = 2 * kLwPadG, kLwRecFlags = kLwRecBand + 4 * kLwBands;
-constexpr int kLwRec = kLwRecFlags + 4;
-static_assert(kLwRec % 4 == 0, "layer records are float4 aligned");
+constexpr int kLwRecFracs = kLwPadG, kLwRecBand = 2 * kLwPadG, kLwRecEfcl = kLwRecBand + 4 * kLwBands;
+constexpr int kLwRecFlags = kLwRecEfcl + kLwBands;
+constexpr int kLwRec = kLwRecFlags + 8;
+static_assert(kLwRec % 8 == 0 && 1 + kLwMaskWords <= 8, "layer records are whole sectors");
 __constant__ int kLwPadOfsDev[kLwBands] = {0, 12, 24, 40, 56, 72, 80, 92, 100, 112, 120, 128, 136, 140, 144, 148};
-__constant__ int kNgcDev[kLwBands] = {10, 12, 16, 14, 16, 8, 12, 8, 12, 6, 8, 8, 4, 2, 2, 2};
+__constant__ int kLwPadDev[kLwBands] = {12, 12, 16, 16, 16, 8, 12, 8, 12, 8, 8, 8, 4, 4, 4, 4};
 __constant__ int kGofsDev[kLwBands] = {0, 10, 22, 38, 52, 68, 76, 88, 96, 108, 114, 122, 130, 134, 136, 138};
 
 // The Layer fields taumol reads, stored field by field ([field][layer][column]).
@@ -167,20 +171,35 @@ __global__ void __launch_bounds__(128, kLwLayerMinBlocks) lw_layer_kernel(Tables
   const bool cloudy = load_mask(a, l, col, mask);
   float4 *rec = reinterpret_cast<float4 *>(layer_records(a) + (static_cast<size_t>(lc) * a.nlay + l) * kLwRec);
   const int iceflag = C.iceflg;
+  const float *secdiff = col_records(a)[lc].secdiff;
 #pragma unroll 1
-  for (int b = 0; b < kLwBands; ++b) {
-    const float blay = planck(T, L.indlay, L.tlayfrac, b);
-    const float dplankup = planck(T, L.indlev1, L.tlev1frac, b) - blay;
-    const float dplankdn = planck(T, L.indlev0, L.tlev0frac, b) - blay;
-    float teff = 0.0f;
-    if (cloudy) {
-      bool active = false;
-      const float tauc = cloud_tau(T, L, b, iceflag, active);
-      teff = active ? tauc : 0.0f;
+  for (int b4 = 0; b4 < kLwBands; b4 += 4) {
+    float efcl[4];
+#pragma unroll
+    for (int e = 0; e < 4; ++e) {
+      const int b = b4 + e;
+      const float blay = planck(T, L.indlay, L.tlayfrac, b);
+      const float dplankup = planck(T, L.indlev1, L.tlev1frac, b) - blay;
+      const float dplankdn = planck(T, L.indlev0, L.tlev0frac, b) - blay;
+      // a cloudy g-point's optical depth and absorptance (lw:5562-5565): the
+      // same for all g-points of the band, so its binary64 exponential is
+      // evaluated here, once per band and not once per g-point and direction
+      float odcld = 0.0f;
+      efcl[e] = 0.0f;
+      if (cloudy) {
+        bool active = false;
+        const float tauc = cloud_tau(T, L, b, iceflag, active);
+        odcld = secdiff[b] * (active ? tauc : 0.0f);
+        efcl[e] = (1.0f - glibc_expf(T, -odcld)) * 1.0f;
+      }
+      rec[kLwRecBand / 4 + b] = make_float4(blay, dplankup, dplankdn, odcld);
     }
-    rec[kLwRecBand / 4 + b] = make_float4(blay, dplankup, dplankdn, teff);
+    rec[kLwRecEfcl / 4 + b4 / 4] = make_float4(efcl[0], efcl[1], efcl[2], efcl[3]);
   }
-  rec[kLwRecFlags / 4] = make_float4(cloudy ? 1.0f : 0.0f, 0.0f, 0.0f, 0.0f);
+  static_assert(kLwMaskWords == 5, "mask words of a record");
+  rec[kLwRecFlags / 4] = make_float4(cloudy ? 1.0f : 0.0f, __uint_as_float(mask[0]), __uint_as_float(mask[1]),
+                                     __uint_as_float(mask[2]));
+  rec[kLwRecFlags / 4 + 1] = make_float4(__uint_as_float(mask[3]), __uint_as_float(mask[4]), 0.0f, 0.0f);
 }
 
 // 16-byte pieces of a warp's stage: optical depths, then fractions, of 32 rows of up to 5
@@ -272,157 +291,267 @@ __global__ void __launch_bounds__(128, kLwGasMinBlocks) lw_gas_kernel(Tables T, 
   }
 }
 
-// One g-point of band_sums: the new radiances (rA, rB) after one layer, from
-// the g-point's gas optical depth tg and Planck fraction fr, its band's
-// (blay, dplankup, dplankdn, cloud optical depth) bq, its McICA bit cld and
-// the layer's cloud flag.
-template <bool kDown>
-__device__ __forceinline__ void lw_step(const Tables &T, float tg, float fr, float4 bq, bool cld, bool cloudy_layer,
-                                        float secdiff, float &rA, float &rB, bool sep_clear) {
-  float odepth = secdiff * tg;
-  if (odepth < 0.0f) odepth = 0.0f;
-  float odcld = 0.0f, efcl = 0.0f;
-  if (cld) {
-    const float odcld_raw = secdiff * bq.w;
-    const float abscld = 1.0f - glibc_expf(T, -odcld_raw);
-    odcld = odcld_raw;
-    efcl = abscld * 1.0f;
-  }
-  const Terms tm = layer_terms(T, cloudy_layer, odepth, odcld, fr, bq.x, bq.z, bq.y);
-  const float cf = cld ? 1.0f : 0.0f;
-  const float r = rA, rc = rB;
-  float rn;
-  if constexpr (kDown) {
-    if (cloudy_layer) {
-      rn = r - r * (tm.a + efcl * (1.0f - tm.a)) + tm.gassrc + cf * (tm.bbdtot * tm.atot - tm.gassrc);
-    } else {
-      rn = r + (tm.bbdgas - r) * tm.a;
-    }
-    rB = sep_clear ? rc + (tm.bbdgas - rc) * tm.a : rn;
+// ---------------------------------------------------------------------------
+// One g-point of one layer of rtrnmc (_rtrnmc_clear_terms / _rtrnmc_cloudy_terms,
+// lw:5157-5262, and the radiance updates).  (a, x) are the layer's absorptance
+// and the Planck interpolation factor of an optical depth: from the series
+// where it is thin, else from the Pade tables, which the context holds as
+// pairs (1 - exp, tfn).  The operations and their order are layer_terms' of
+// the fused schedule; branches of it that give the same statements are merged,
+// and the total-sky part is left out where the g-point has no cloud, since its
+// weight there is zero.
+// ---------------------------------------------------------------------------
+struct LwGas {
+  float a, x;
+};
+
+__device__ __forceinline__ LwGas lw_thin(float od) { return {od - (0.5f * od) * od, 0.166667f * od}; }
+
+__device__ __forceinline__ LwGas lw_table(const Tables &T, int it) {
+  const float2 v = __ldg(T.lw_pade + it);
+  return {v.x, v.y};
+}
+
+// What the upward pass needs of a layer's transfer terms, in 32 bits: the gas
+// optical depth itself where the series serves (sign bit clear), else the
+// gas's table position, and above it (kLwTotShift) the cloudy total's.
+constexpr uint32_t kLwTableBit = 0x80000000u;
+constexpr int kLwTotShift = 15;
+static_assert(kLwPadeMax < (1 << kLwTotShift), "table positions fit their bits");
+
+// Total-sky (a, x) of a cloudy g-point whose gas is thin.
+__device__ __forceinline__ LwGas lw_total_thin(const Tables &T, float odtot) {
+  return odtot < 0.06f ? lw_thin(odtot) : lw_table(T, pade_index(T, odtot));
+}
+
+// New radiance of a g-point: rA total sky, rB clear sky.  src: the gas's
+// source, tot: the cloudy total's.
+__device__ __forceinline__ float lw_cloudy_radiance(float r, float a, float efcl, float src, float tot) {
+  return r - r * (a + efcl * (1.0f - a)) + src + (tot - src);
+}
+
+// Downward: returns the word for the upward pass.
+__device__ __forceinline__ uint32_t lw_down(const Tables &T, float tg, float fr, float4 bq, float efcl, bool cld,
+                                            bool cloudy_layer, float secdiff, float &rA, float &rB, bool sep_clear) {
+  float od = secdiff * tg;
+  if (od <= 0.0f) od = 0.0f;
+  const float odtot = od + bq.w;
+  const bool thin = od <= 0.06f || (cloudy_layer && cld && odtot < 0.06f);
+  LwGas g;
+  uint32_t word;
+  int ig = 0;
+  if (thin) {
+    g = lw_thin(od);
+    word = __float_as_uint(od);
   } else {
-    if (cloudy_layer) {
-      const float gas = tm.bbugas * tm.a;
-      rn = r - r * (tm.a + efcl * (1.0f - tm.a)) + gas + cf * (tm.bbutot * tm.atot - gas);
-    } else {
-      rn = r + (tm.bbugas - r) * tm.a;
-    }
-    rB = sep_clear ? rc + (tm.bbugas - rc) * tm.a : rn;
+    ig = pade_index(T, od);
+    g = lw_table(T, ig);
+    word = kLwTableBit | static_cast<uint32_t>(ig);
   }
-  rA = rn;
+  const float planck_dn = bq.x + g.x * bq.z;
+  const float bbdgas = fr * planck_dn;
+  if (cloudy_layer) {
+    const float gassrc = thin ? bbdgas * g.a : (g.a * fr) * planck_dn;
+    if (cld) {
+      LwGas t;
+      if (thin) {
+        t = lw_total_thin(T, odtot);
+      } else {
+        const int it = pade_index(T, ld(T.lw_pade_tau + ig) + bq.w);
+        t = lw_table(T, it);
+        word |= static_cast<uint32_t>(it) << kLwTotShift;
+      }
+      const float bbdtot = fr * (bq.x + t.x * bq.z);
+      rA = lw_cloudy_radiance(rA, g.a, efcl, gassrc, bbdtot * t.a);
+    } else {
+      rA = rA - rA * g.a + gassrc;
+    }
+    rB = rB + (bbdgas - rB) * g.a;
+  } else {
+    const float rn = rA + (bbdgas - rA) * g.a;
+    rB = sep_clear ? rB + (bbdgas - rB) * g.a : rn;
+    rA = rn;
+  }
+  return word;
+}
+
+__device__ __forceinline__ void lw_up(const Tables &T, uint32_t word, float fr, float4 bq, float efcl, bool cld,
+                                      bool cloudy_layer, float &rA, float &rB, bool sep_clear) {
+  const bool thin = (word & kLwTableBit) == 0u;
+  const float od = __uint_as_float(word);
+  constexpr uint32_t kPos = (1u << kLwTotShift) - 1u;
+  const LwGas g = thin ? lw_thin(od) : lw_table(T, static_cast<int>(word & kPos));
+  const float bbugas = fr * (bq.x + g.x * bq.y);
+  if (cloudy_layer) {
+    const float gas = bbugas * g.a;
+    if (cld) {
+      const LwGas t = thin ? lw_total_thin(T, od + bq.w)
+                           : lw_table(T, static_cast<int>((word >> kLwTotShift) & kPos));
+      const float bbutot = fr * (bq.x + t.x * bq.y);
+      rA = lw_cloudy_radiance(rA, g.a, efcl, gas, bbutot * t.a);
+    } else {
+      rA = rA - rA * g.a + gas;
+    }
+    rB = rB + (bbugas - rB) * g.a;
+  } else {
+    const float rn = rA + (bbugas - rA) * g.a;
+    rB = sep_clear ? rB + (bbugas - rB) * g.a : rn;
+    rA = rn;
+  }
 }
 
 constexpr int kLwSweepCols = 2;                            // columns per block
 constexpr int kLwSweepThreads = 288;                       // 2 x 140 g-points in 9 warps; 8 padding threads
-constexpr int kLwRing = 8;                                 // levels of radiances per ordered-sum round
+constexpr int kLwRing = 4;                                 // levels of radiances per ordered-sum round
+constexpr int kLwRows = kLwRing * 2 * kLwSweepCols;        // (level, total / clear, column) rows of a round
+constexpr int kLwRowStride = kLwPadG + 4;                  // an odd number of 16-byte pieces: no bank conflicts
 static_assert(kLwSweepThreads >= kLwSweepCols * kLwGpts && kLwSweepThreads % 32 == 0, "sweep block shape");
+static_assert(kLwRows == 16 && kLwBands == 16 && kLwSweepThreads / 32 == 9, "sum chains of a round: two bands a warp");
+static_assert(kLwRowStride % 4 == 0 && (kLwRowStride / 4) % 2 == 1, "ring rows");
 
 struct LwSweepShared {
-  float ring[kLwRing][kLwSweepCols][2][kLwGpts];      // total, clear radiance of each g-point
-  float bands[kLwRing][kLwSweepCols][2][kLwBands];    // each band's radiance sum
-  float flux[kLwSweepCols][4][kMaxLay + 1];           // up total, up clear, down total, down clear per level
+  float ring[2][kLwRows][kLwRowStride];        // radiances of each g-point, bands padded with zeros
+  float bands[2][kLwRows][kLwBands + 1];       // each band's radiance sum
+  float flux[kLwSweepCols][4][kMaxLay + 1];    // up total, up clear, down total, down clear per level
 };
 
-// Sums the ring's levels in two rounds of independent chains: (column,
-// total/clear, level, band) adds the band's radiances in g-point order, then
-// (column, total/clear, level) adds the band terms (bandsum * 0.5) * delwave in
-// band order (band_step, lw:170-199) and multiplies by fluxfac.  The
-// operations and their order are those of one sequential sum per level.
-__device__ __forceinline__ void lw_flush(LwSweepShared &S, int count, int type0, int level0, int dir) {
-  __syncthreads();
+// One round of levels awaiting its sums.
+struct LwRound {
+  int count, type0, level0, dir;
+};
+
+// bands of the two half warps of warp w < 8, of like length
+__constant__ int kLwSumBand[2][8] = {{0, 2, 4, 8, 7, 10, 12, 14}, {1, 3, 6, 5, 9, 11, 13, 15}};
+
+// Band terms (bandsum * 0.5) * delwave added in band order (lw:170-199) and
+// multiplied by fluxfac: one lane per row of round `number`.
+__device__ __forceinline__ void lw_band_terms(LwSweepShared &S, int number, const LwRound &r) {
   const float pi = 3.1415926535897932384626433832795f;
   const float fluxfac = pi * 2.0e4f;
-  const int band_chains = kLwSweepCols * 2 * count * kLwBands;
-  for (int ch = threadIdx.x; ch < band_chains; ch += kLwSweepThreads) {
-    const int b = ch % kLwBands;
-    const int rest = ch / kLwBands;
-    const int j = rest % count;
-    const int cq = rest / count;  // column * 2 + total/clear
-    const float *v = S.ring[j][cq >> 1][cq & 1] + kGofsDev[b];
-    const int ngc = kNgcDev[b];
-    float bandsum = 0.0f;
-    for (int g = 0; g < ngc; ++g) bandsum = bandsum + v[g];
-    S.bands[j][cq >> 1][cq & 1][b] = bandsum;
-  }
-  __syncthreads();
-  const int chains = kLwSweepCols * 2 * count;
-  for (int ch = threadIdx.x; ch < chains; ch += kLwSweepThreads) {
-    const int j = ch % count;
-    const int cq = ch / count;
-    const float *bs = S.bands[j][cq >> 1][cq & 1];
-    float total = 0.0f;
+  const int row = threadIdx.x & 31;
+  if (row >= 2 * kLwSweepCols * r.count) return;
+  const float *bs = S.bands[number & 1][row];
+  float total = 0.0f;
 #pragma unroll
-    for (int b = 0; b < kLwBands; ++b) total = total + (bs[b] * 0.5f) * kDelwave[b];
-    S.flux[cq >> 1][type0 + (cq & 1)][level0 + dir * j] = total * fluxfac;
-  }
-  __syncthreads();
+  for (int b = 0; b < kLwBands; ++b) total = total + (bs[b] * 0.5f) * kDelwave[b];
+  const int c = row % kLwSweepCols, type = row / kLwSweepCols % 2, j = row / (2 * kLwSweepCols);
+  S.flux[c][r.type0 + type][r.level0 + r.dir * j] = total * fluxfac;
 }
 
-// Block = kLwSweepCols consecutive columns of the chunk.  A column past the
-// chunk or the live count repeats the block's first column so that every
-// thread takes the same barriers; its results are not written.
+// Ordered sums of a round whose radiances have just been stored: warps 0-7
+// add each band's radiances in g-point order (a half warp per band, a lane per
+// row; the zero padding of a band adds nothing), and warp 8 adds the previous
+// round's band terms.  The next round fills the other ring buffer meanwhile,
+// so a round of four levels costs one barrier.  The operations and their order
+// are those of one sequential sum per level.
+__device__ __forceinline__ void lw_sum_round(LwSweepShared &S, int number, const LwRound &prev) {
+  __syncthreads();
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  if (warp == 8) {
+    if (number > 0) lw_band_terms(S, number - 1, prev);
+    return;
+  }
+  const int row = lane & 15, b = kLwSumBand[lane >> 4][warp];
+  const float4 *v = reinterpret_cast<const float4 *>(S.ring[number & 1][row] + kLwPadOfsDev[b]);
+  const int quads = kLwPadDev[b] / 4;
+  float sum = 0.0f;
+  for (int q = 0; q < quads; ++q) {
+    const float4 x = v[q];
+    sum = sum + x.x;
+    sum = sum + x.y;
+    sum = sum + x.z;
+    sum = sum + x.w;
+  }
+  S.bands[number & 1][row][b] = sum;
+}
+
+// Block = kLwSweepCols consecutive columns of the chunk.  Threads without a
+// column of their own (padding threads, a column past the chunk or the live
+// count) only take the barriers and their part of the sums.
+// Bound by instruction issue and the latency of record loads and table gathers.
+// 425 x 425 x 50 (180,625 columns of 63 layers): 27.6 ms before the cloud's
+// exponential moved to the layer kernel, the upward pass reused the downward
+// pass's table positions, and the sums took 16-byte reads of padded bands with
+// one barrier in four levels (before, three in eight and 4-byte reads); 22.4 ms
+// now.
 __global__ void __launch_bounds__(kLwSweepThreads, kLwSweepMinBlocks) lw_sweep_kernel(Tables T, LwArgs a) {
   __shared__ __align__(16) LwSweepShared S;
   const int lc0 = blockIdx.x * kLwSweepCols;
   if (lc0 >= a.chunk_count || dead_column(a.live, a.chunk_first + lc0)) return;  // whole block
   const int tid = threadIdx.x;
-  const bool writer = tid < kLwSweepCols * kLwGpts;
-  const int cslot = writer ? tid / kLwGpts : kLwSweepCols - 1;
-  const int G = writer ? tid - cslot * kLwGpts : kLwGpts - 1;
-  const int lc_own = lc0 + cslot;
-  const bool live = lc_own < a.chunk_count && !dead_column(a.live, a.chunk_first + lc_own);
-  const int lc = live ? lc_own : lc0;
+  const bool slot = tid < kLwSweepCols * kLwGpts;
+  const int cslot = slot ? tid / kLwGpts : kLwSweepCols - 1;
+  const int G = slot ? tid - cslot * kLwGpts : kLwGpts - 1;
+  const int lc = lc0 + cslot;
+  const bool live = slot && lc < a.chunk_count && !dead_column(a.live, a.chunk_first + lc);
   const int col = a.chunk_first + lc;
   int band = kLwBands - 1;
   while (G < kGofsDev[band]) --band;
   const int P = kLwPadOfsDev[band] + (G - kGofsDev[band]);
-  const ColRec &R = col_records(a)[lc];
+  const ColRec &R = col_records(a)[live ? lc : lc0];
   const float sd = R.secdiff[band];
   const bool has_cloud = R.has_cloud != 0;
   const int nlay = a.nlay, nk = a.nk;
-  const float *recs = layer_records(a) + static_cast<size_t>(lc) * nlay * kLwRec;
-  const uint32_t *mword = a.mask + col + static_cast<size_t>(G >> 5) * a.ncol;
-  const size_t mstride = static_cast<size_t>(kLwMaskWords) * a.ncol;
+  float *const recs = layer_records(a) + static_cast<size_t>(lc) * nlay * kLwRec;
+  const int PB = kLwRecBand + 4 * band, PE = kLwRecEfcl + band, PW = kLwRecFlags + 1 + (G >> 5);
   const uint32_t bit = 1u << (G & 31);
   const float pi = 3.1415926535897932384626433832795f;
   const float fluxfac = pi * 2.0e4f;
+  for (int q = tid; q < 2 * kLwRows * kLwRowStride; q += kLwSweepThreads) (&S.ring[0][0][0])[q] = 0.0f;
   if (tid < kLwSweepCols * 2) S.flux[tid >> 1][2 + (tid & 1)][nlay] = 0.0f * fluxfac;  // no downward flux at the top
+  __syncthreads();
+  // this thread's radiances in the ring: row (level * 2 + total / clear) * columns + column
+  float *const ring0 = &S.ring[0][cslot][P];
+  constexpr int kTypeStep = kLwSweepCols * kLwRowStride, kBufStep = kLwRows * kLwRowStride;
+  auto put = [&](int number, int filled, float total, float clear) {
+    float *q = ring0 + (number & 1) * kBufStep + filled * (2 * kTypeStep);
+    q[0] = total;
+    q[kTypeStep] = clear;
+  };
+  struct Next {
+    float tg, fr, efcl, flag;
+    float4 bq;
+    uint32_t word;
+  } nx{};
+  auto load = [&](int l) {
+    const float *q = recs + static_cast<size_t>(l) * kLwRec;
+    nx.tg = q[P];
+    nx.fr = q[kLwRecFracs + P];
+    nx.bq = *reinterpret_cast<const float4 *>(q + PB);
+    nx.efcl = q[PE];
+    nx.flag = q[kLwRecFlags];
+    nx.word = __float_as_uint(q[PW]);
+  };
 
   // downward sweep, top to bottom: layer l gives level l; next layer loaded ahead
   float rA = 0.0f, rB = 0.0f;
   bool iclddn = false;
-  int filled = 0, level0 = nlay - 1;
-  const float *q = recs + static_cast<size_t>(nlay - 1) * kLwRec;
-  float nx_tg = q[P], nx_fr = q[kLwRecFracs + P];
-  float4 nx_bq = *reinterpret_cast<const float4 *>(q + kLwRecBand + 4 * band);
-  float nx_flag = q[kLwRecFlags];
-  uint32_t nx_word = mword[static_cast<size_t>(nlay - 1) * mstride];
+  int filled = 0, number = 0;
+  LwRound round{0, 2, nlay - 1, -1}, prev = round;
+  if (live) load(nlay - 1);
   for (int l = nlay - 1; l >= 0; --l) {
-    const float tg = nx_tg, fr = nx_fr, flag = nx_flag;
-    const float4 bq = nx_bq;
-    const uint32_t word = nx_word;
-    if (l > 0) {
-      q = recs + static_cast<size_t>(l - 1) * kLwRec;
-      nx_tg = q[P];
-      nx_fr = q[kLwRecFracs + P];
-      nx_bq = *reinterpret_cast<const float4 *>(q + kLwRecBand + 4 * band);
-      nx_flag = q[kLwRecFlags];
-      nx_word = mword[static_cast<size_t>(l - 1) * mstride];
-    }
-    const bool cloudy = flag != 0.0f;
-    iclddn = iclddn || cloudy;
-    lw_step<true>(T, tg, fr, bq, (word & bit) != 0u, cloudy, sd, rA, rB, iclddn);
-    if (writer) {
-      S.ring[filled][cslot][0][G] = rA;
-      S.ring[filled][cslot][1][G] = rB;
+    if (live) {
+      const Next cur = nx;
+      if (l > 0) load(l - 1);
+      const bool cloudy = cur.flag != 0.0f;
+      iclddn = iclddn || cloudy;
+      const uint32_t up = lw_down(T, cur.tg, cur.fr, cur.bq, cur.efcl, (cur.word & bit) != 0u, cloudy, sd, rA, rB,
+                                  iclddn);
+      recs[static_cast<size_t>(l) * kLwRec + P] = __uint_as_float(up);
+      put(number, filled, rA, rB);
     }
     if (++filled == kLwRing || l == 0) {
-      lw_flush(S, filled, 2, level0, -1);
-      level0 -= filled;
+      round.count = filled;
+      lw_sum_round(S, number, prev);
+      prev = round;
+      round.level0 -= filled;
+      ++number;
       filled = 0;
     }
   }
   // surface emission and reflection: level 0 upward (surface_sums, lw:5648-5655)
-  {
+  round = LwRound{0, 0, 0, 1};
+  if (live) {
     const float bt = R.C.tsfc - 159.0f;
     const int indbound = clampi(static_cast<int>(bt), 1, 180);
     const float tbndfrac = bt - static_cast<float>(indbound);
@@ -431,43 +560,31 @@ __global__ void __launch_bounds__(kLwSweepThreads, kLwSweepMinBlocks) lw_sweep_k
     const float rad0 = recs[kLwRecFracs + P] * plankbnd;
     rA = rad0 + reflect * rA;
     rB = rad0 + reflect * rB;
-    if (writer) {
-      S.ring[0][cslot][0][G] = rA;
-      S.ring[0][cslot][1][G] = rB;
-    }
-    filled = 1;
-    level0 = 0;
+    put(number, 0, rA, rB);
+    load(0);
   }
+  filled = 1;
   // upward sweep, bottom to top: layer l gives level l + 1
-  q = recs;
-  nx_tg = q[P];
-  nx_fr = q[kLwRecFracs + P];
-  nx_bq = *reinterpret_cast<const float4 *>(q + kLwRecBand + 4 * band);
-  nx_flag = q[kLwRecFlags];
-  nx_word = mword[0];
   for (int l = 0; l < nlay; ++l) {
-    const float tg = nx_tg, fr = nx_fr, flag = nx_flag;
-    const float4 bq = nx_bq;
-    const uint32_t word = nx_word;
-    if (l + 1 < nlay) {
-      q = recs + static_cast<size_t>(l + 1) * kLwRec;
-      nx_tg = q[P];
-      nx_fr = q[kLwRecFracs + P];
-      nx_bq = *reinterpret_cast<const float4 *>(q + kLwRecBand + 4 * band);
-      nx_flag = q[kLwRecFlags];
-      nx_word = mword[static_cast<size_t>(l + 1) * mstride];
-    }
-    lw_step<false>(T, tg, fr, bq, (word & bit) != 0u, flag != 0.0f, sd, rA, rB, has_cloud);
-    if (writer) {
-      S.ring[filled][cslot][0][G] = rA;
-      S.ring[filled][cslot][1][G] = rB;
+    if (live) {
+      const Next cur = nx;
+      if (l + 1 < nlay) load(l + 1);
+      lw_up(T, __float_as_uint(cur.tg), cur.fr, cur.bq, cur.efcl, (cur.word & bit) != 0u, cur.flag != 0.0f, rA, rB,
+            has_cloud);
+      put(number, filled, rA, rB);
     }
     if (++filled == kLwRing || l == nlay - 1) {
-      lw_flush(S, filled, 0, level0, 1);
-      level0 += filled;
+      round.count = filled;
+      lw_sum_round(S, number, prev);
+      prev = round;
+      round.level0 += filled;
+      ++number;
       filled = 0;
     }
   }
+  __syncthreads();
+  if (tid >> 5 == 8) lw_band_terms(S, number - 1, prev);
+  __syncthreads();
 
   // heating rates and theta tendencies (lw:5706-5712, 7040-7057) and the 2-D
   // outputs (lw:7059-7077) of the block's live columns
@@ -496,7 +613,7 @@ __global__ void __launch_bounds__(kLwSweepThreads, kLwSweepMinBlocks) lw_sweep_k
     a.rthraten[rbase + static_cast<size_t>(l) * a.ny] = (htr / 86400.0f) / pi3d;
     a.rthratenc[rbase + static_cast<size_t>(l) * a.ny] = (htrc / 86400.0f) / pi3d;
   }
-  if (G == 0 && writer && live) {
+  if (G == 0 && live) {
     const float(*fx)[kMaxLay + 1] = S.flux[cslot];
     const float uflt = fx[0][nlay], ufltc = fx[1][nlay];
     const float dflt = 0.0f * fluxfac;
