@@ -45,16 +45,16 @@ namespace {
 // boundary (kLwPadOfs), the Planck fractions likewise from kLwRecFracs, per
 // band (blay, dplankup, dplankdn, cloud optical depth along the diffusivity
 // angle) from kLwRecBand and the cloud's absorptance from kLwRecEfcl, and from
-// kLwRecFlags the layer's cloud flag and McICA mask words.  The sweep's
+// kLwRecMask the layer's McICA mask words.  The sweep's
 // downward pass leaves its transfer-table positions in place of the optical
 // depths for the upward pass (lw_down).
 constexpr int kLwPadOfs[kLwBands] = {0, 12, 24, 40, 56, 72, 80, 92, 100, 112, 120, 128, 136, 140, 144, 148};
 constexpr int kLwPadG = 152;
 static_assert(kLwPadOfs[kLwBands - 1] + lw_pad(kLwBands - 1) == kLwPadG, "padded g-points");
 constexpr int kLwRecFracs = kLwPadG, kLwRecBand = 2 * kLwPadG, kLwRecEfcl = kLwRecBand + 4 * kLwBands;
-constexpr int kLwRecFlags = kLwRecEfcl + kLwBands;
-constexpr int kLwRec = kLwRecFlags + 8;
-static_assert(kLwRec % 8 == 0 && 1 + kLwMaskWords <= 8, "layer records are whole sectors");
+constexpr int kLwRecMask = kLwRecEfcl + kLwBands;
+constexpr int kLwRec = kLwRecMask + 8;
+static_assert(kLwRec % 8 == 0 && kLwMaskWords <= 8, "layer records are whole sectors");
 __constant__ int kLwPadOfsDev[kLwBands] = {0, 12, 24, 40, 56, 72, 80, 92, 100, 112, 120, 128, 136, 140, 144, 148};
 __constant__ int kLwPadDev[kLwBands] = {12, 12, 16, 16, 16, 8, 12, 8, 12, 8, 8, 8, 4, 4, 4, 4};
 __constant__ int kGofsDev[kLwBands] = {0, 10, 22, 38, 52, 68, 76, 88, 96, 108, 114, 122, 130, 134, 136, 138};
@@ -75,7 +75,7 @@ constexpr int kLwGasFields = 0 RRTMG_LW_GAS_FLOATS(RRTMG_LW_COUNT) RRTMG_LW_GAS_
 struct ColRec {
   Col C;
   float secdiff[kLwBands];
-  int has_cloud;
+  uint32_t cloud[kMaxLay / 32];  // bit l % 32 of word l / 32: layer l is cloudy in some g-point
 };
 constexpr size_t kColRecFloats = (sizeof(ColRec) + 15) / 16 * 4;
 
@@ -116,17 +116,22 @@ __global__ void __launch_bounds__(128) lw_colprep_kernel(Tables T, LwArgs a) {
   column_setup<true>(T, a, C, lane, s_tlev[w], s_o3[w]);
   const int nlay = C.nlay;
   int trop_count = 0;
-  bool cloud = false;
-  for (int l = lane; l < nlay; l += 32) {
-    bool trop;
-    column_layer(T, a, C, l, trop, s_cd[w][l], s_wk[w][l]);
-    trop_count += trop;
-    uint32_t mask[kLwMaskWords];
-    cloud = load_mask(a, l, col, mask) || cloud;
+#pragma unroll 1
+  for (int i = 0; i < kMaxLay / 32; ++i) {
+    const int l = 32 * i + lane;
+    bool cloud = false;
+    if (l < nlay) {
+      bool trop;
+      column_layer(T, a, C, l, trop, s_cd[w][l], s_wk[w][l]);
+      trop_count += trop;
+      uint32_t mask[kLwMaskWords];
+      cloud = load_mask(a, l, col, mask);
+    }
+    const uint32_t word = __ballot_sync(0xffffffffu, cloud);
+    if (lane == 0) reinterpret_cast<ColRec *>(a.scratch)[lc].cloud[i] = word;
   }
 #pragma unroll
   for (int o = 16; o > 0; o >>= 1) trop_count += __shfl_xor_sync(0xffffffffu, trop_count, o);
-  const bool has_cloud = __any_sync(0xffffffffu, cloud);
   __syncwarp();
   float amttl = 0.0f, wvttl = 0.0f;
   for (int l = 0; l < nlay; ++l) {
@@ -136,8 +141,12 @@ __global__ void __launch_bounds__(128) lw_colprep_kernel(Tables T, LwArgs a) {
   C.laytrop = trop_count;
   C.pwvcm = column_pwvcm(a, C, amttl, wvttl);
   column_secdiff(T, C, r.secdiff);
-  r.has_cloud = has_cloud ? 1 : 0;
-  if (lane == 0) reinterpret_cast<ColRec *>(a.scratch)[lc] = r;
+  if (lane == 0) {
+    ColRec &out = reinterpret_cast<ColRec *>(a.scratch)[lc];
+    out.C = r.C;
+#pragma unroll
+    for (int b = 0; b < kLwBands; ++b) out.secdiff[b] = r.secdiff[b];
+  }
 }
 
 // thread = (layer, chunk column), columns fastest
@@ -197,9 +206,9 @@ __global__ void __launch_bounds__(128, kLwLayerMinBlocks) lw_layer_kernel(Tables
     rec[kLwRecEfcl / 4 + b4 / 4] = make_float4(efcl[0], efcl[1], efcl[2], efcl[3]);
   }
   static_assert(kLwMaskWords == 5, "mask words of a record");
-  rec[kLwRecFlags / 4] = make_float4(cloudy ? 1.0f : 0.0f, __uint_as_float(mask[0]), __uint_as_float(mask[1]),
-                                     __uint_as_float(mask[2]));
-  rec[kLwRecFlags / 4 + 1] = make_float4(__uint_as_float(mask[3]), __uint_as_float(mask[4]), 0.0f, 0.0f);
+  rec[kLwRecMask / 4] = make_float4(__uint_as_float(mask[0]), __uint_as_float(mask[1]), __uint_as_float(mask[2]),
+                                    __uint_as_float(mask[3]));
+  rec[kLwRecMask / 4 + 1] = make_float4(__uint_as_float(mask[4]), 0.0f, 0.0f, 0.0f);
 }
 
 // 16-byte pieces of a warp's stage: optical depths, then fractions, of 32 rows of up to 5
@@ -413,6 +422,7 @@ struct LwSweepShared {
   float ring[2][kLwRows][kLwRowStride];        // radiances of each g-point, bands padded with zeros
   float bands[2][kLwRows][kLwBands + 1];       // each band's radiance sum
   float flux[kLwSweepCols][4][kMaxLay + 1];    // up total, up clear, down total, down clear per level
+  uint32_t cloud[kLwSweepCols][kMaxLay / 32];  // the columns' cloudy layers
 };
 
 // One round of levels awaiting its sums.
@@ -444,25 +454,38 @@ __device__ __forceinline__ void lw_band_terms(LwSweepShared &S, int number, cons
 // round's band terms.  The next round fills the other ring buffer meanwhile,
 // so a round of four levels costs one barrier.  The operations and their order
 // are those of one sequential sum per level.
-__device__ __forceinline__ void lw_sum_round(LwSweepShared &S, int number, const LwRound &prev) {
-  __syncthreads();
+// chain: the lane's band sum of every round (warps 0-7), found once.
+struct LwChain {
+  const float4 *v;  // its radiances in ring buffer 0
+  float *sum;       // its place in bands[0]
+  int quads;
+};
+
+__device__ __forceinline__ LwChain lw_chain(LwSweepShared &S) {
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  if (warp == 8) {
+  const int row = lane & 15, b = kLwSumBand[lane >> 4][warp & 7];
+  return {reinterpret_cast<const float4 *>(S.ring[0][row] + kLwPadOfsDev[b]), &S.bands[0][row][b], kLwPadDev[b] / 4};
+}
+
+__device__ __forceinline__ void lw_sum_round(LwSweepShared &S, const LwChain &chain, int number, const LwRound &prev) {
+  __syncthreads();
+  if (threadIdx.x >= 256) {
     if (number > 0) lw_band_terms(S, number - 1, prev);
     return;
   }
-  const int row = lane & 15, b = kLwSumBand[lane >> 4][warp];
-  const float4 *v = reinterpret_cast<const float4 *>(S.ring[number & 1][row] + kLwPadOfsDev[b]);
-  const int quads = kLwPadDev[b] / 4;
+  const float4 *v = chain.v + (number & 1) * (kLwRows * kLwRowStride / 4);
   float sum = 0.0f;
-  for (int q = 0; q < quads; ++q) {
-    const float4 x = v[q];
-    sum = sum + x.x;
-    sum = sum + x.y;
-    sum = sum + x.z;
-    sum = sum + x.w;
+#pragma unroll
+  for (int q = 0; q < 4; ++q) {
+    if (q < chain.quads) {
+      const float4 x = v[q];
+      sum = sum + x.x;
+      sum = sum + x.y;
+      sum = sum + x.z;
+      sum = sum + x.w;
+    }
   }
-  S.bands[number & 1][row][b] = sum;
+  chain.sum[(number & 1) * (kLwRows * (kLwBands + 1))] = sum;
 }
 
 // Block = kLwSweepCols consecutive columns of the chunk.  Threads without a
@@ -472,8 +495,10 @@ __device__ __forceinline__ void lw_sum_round(LwSweepShared &S, int number, const
 // 425 x 425 x 50 (180,625 columns of 63 layers): 27.6 ms before the cloud's
 // exponential moved to the layer kernel, the upward pass reused the downward
 // pass's table positions, and the sums took 16-byte reads of padded bands with
-// one barrier in four levels (before, three in eight and 4-byte reads); 22.4 ms
-// now.
+// one barrier in four levels (before, three in eight and 4-byte reads): 22.4 ms;
+// with four levels unrolled (no register moves of the layer loaded ahead) and
+// records addressed by 32-bit offsets from the block's first: 20.6 ms.  At 5
+// blocks per SM (40 registers) 21.9 ms.
 __global__ void __launch_bounds__(kLwSweepThreads, kLwSweepMinBlocks) lw_sweep_kernel(Tables T, LwArgs a) {
   __shared__ __align__(16) LwSweepShared S;
   const int lc0 = blockIdx.x * kLwSweepCols;
@@ -490,16 +515,23 @@ __global__ void __launch_bounds__(kLwSweepThreads, kLwSweepMinBlocks) lw_sweep_k
   const int P = kLwPadOfsDev[band] + (G - kGofsDev[band]);
   const ColRec &R = col_records(a)[live ? lc : lc0];
   const float sd = R.secdiff[band];
-  const bool has_cloud = R.has_cloud != 0;
   const int nlay = a.nlay, nk = a.nk;
-  float *const recs = layer_records(a) + static_cast<size_t>(lc) * nlay * kLwRec;
-  const int PB = kLwRecBand + 4 * band, PE = kLwRecEfcl + band, PW = kLwRecFlags + 1 + (G >> 5);
   const uint32_t bit = 1u << (G & 31);
   const float pi = 3.1415926535897932384626433832795f;
   const float fluxfac = pi * 2.0e4f;
   for (int q = tid; q < 2 * kLwRows * kLwRowStride; q += kLwSweepThreads) (&S.ring[0][0][0])[q] = 0.0f;
   if (tid < kLwSweepCols * 2) S.flux[tid >> 1][2 + (tid & 1)][nlay] = 0.0f * fluxfac;  // no downward flux at the top
+  bool has_cloud = false;
+  if (live) {
+#pragma unroll
+    for (int w = 0; w < kMaxLay / 32; ++w) {
+      const uint32_t word = 32 * w < nlay ? R.cloud[w] : 0u;
+      has_cloud = has_cloud || word != 0u;
+      if (G == 0) S.cloud[cslot][w] = word;
+    }
+  }
   __syncthreads();
+  const LwChain chain = lw_chain(S);
   // this thread's radiances in the ring: row (level * 2 + total / clear) * columns + column
   float *const ring0 = &S.ring[0][cslot][P];
   constexpr int kTypeStep = kLwSweepCols * kLwRowStride, kBufStep = kLwRows * kLwRowStride;
@@ -508,82 +540,94 @@ __global__ void __launch_bounds__(kLwSweepThreads, kLwSweepMinBlocks) lw_sweep_k
     q[0] = total;
     q[kTypeStep] = clear;
   };
+  // the block's layer records, addressed from one base by 32-bit byte offsets
+  char *const base = reinterpret_cast<char *>(layer_records(a) + static_cast<size_t>(lc0) * nlay * kLwRec);
+  constexpr uint32_t kStep = kLwRec * sizeof(float);
+  const uint32_t column = static_cast<uint32_t>(cslot * nlay) * kStep;
+  const uint32_t off_tau = column + 4u * P, off_band = column + 4u * (kLwRecBand + 4 * band);
+  const uint32_t off_efcl = column + 4u * (kLwRecEfcl + band), off_mask = column + 4u * (kLwRecMask + (G >> 5));
+  auto at = [&](uint32_t off) -> float & { return *reinterpret_cast<float *>(base + off); };
   struct Next {
-    float tg, fr, efcl, flag;
+    float tg, fr, efcl;
     float4 bq;
     uint32_t word;
+    bool cloudy;
   } nx{};
   auto load = [&](int l) {
-    const float *q = recs + static_cast<size_t>(l) * kLwRec;
-    nx.tg = q[P];
-    nx.fr = q[kLwRecFracs + P];
-    nx.bq = *reinterpret_cast<const float4 *>(q + PB);
-    nx.efcl = q[PE];
-    nx.flag = q[kLwRecFlags];
-    nx.word = __float_as_uint(q[PW]);
+    const uint32_t step = static_cast<uint32_t>(l) * kStep;
+    nx.tg = at(off_tau + step);
+    nx.fr = at(off_tau + step + 4 * kLwRecFracs);
+    nx.bq = *reinterpret_cast<const float4 *>(base + off_band + step);
+    nx.cloudy = (S.cloud[cslot][l >> 5] >> (l & 31)) & 1u;
+    if (nx.cloudy) {
+      nx.efcl = at(off_efcl + step);
+      nx.word = __float_as_uint(at(off_mask + step));
+    }
   };
 
   // downward sweep, top to bottom: layer l gives level l; next layer loaded ahead
   float rA = 0.0f, rB = 0.0f;
   bool iclddn = false;
-  int filled = 0, number = 0;
+  int number = 0;
   LwRound round{0, 2, nlay - 1, -1}, prev = round;
   if (live) load(nlay - 1);
-  for (int l = nlay - 1; l >= 0; --l) {
+  for (int l0 = nlay - 1; l0 >= 0; l0 -= kLwRing) {
     if (live) {
-      const Next cur = nx;
-      if (l > 0) load(l - 1);
-      const bool cloudy = cur.flag != 0.0f;
-      iclddn = iclddn || cloudy;
-      const uint32_t up = lw_down(T, cur.tg, cur.fr, cur.bq, cur.efcl, (cur.word & bit) != 0u, cloudy, sd, rA, rB,
-                                  iclddn);
-      recs[static_cast<size_t>(l) * kLwRec + P] = __uint_as_float(up);
-      put(number, filled, rA, rB);
+#pragma unroll
+      for (int j = 0; j < kLwRing; ++j) {
+        const int l = l0 - j;
+        if (l < 0) break;
+        const Next cur = nx;
+        if (l > 0) load(l - 1);
+        iclddn = iclddn || cur.cloudy;
+        const uint32_t up = lw_down(T, cur.tg, cur.fr, cur.bq, cur.efcl, (cur.word & bit) != 0u, cur.cloudy, sd, rA,
+                                    rB, iclddn);
+        at(off_tau + static_cast<uint32_t>(l) * kStep) = __uint_as_float(up);
+        put(number, j, rA, rB);
+      }
     }
-    if (++filled == kLwRing || l == 0) {
-      round.count = filled;
-      lw_sum_round(S, number, prev);
-      prev = round;
-      round.level0 -= filled;
-      ++number;
-      filled = 0;
-    }
+    round.count = l0 + 1 < kLwRing ? l0 + 1 : kLwRing;
+    lw_sum_round(S, chain, number, prev);
+    prev = round;
+    round.level0 -= kLwRing;
+    ++number;
   }
-  // surface emission and reflection: level 0 upward (surface_sums, lw:5648-5655)
+  // upward sweep, bottom to top: level 0 from the surface, then layer l gives level l + 1
   round = LwRound{0, 0, 0, 1};
-  if (live) {
-    const float bt = R.C.tsfc - 159.0f;
-    const int indbound = clampi(static_cast<int>(bt), 1, 180);
-    const float tbndfrac = bt - static_cast<float>(indbound);
-    const float reflect = 1.0f - R.C.semiss;
-    const float plankbnd = R.C.semiss * planck(T, indbound, tbndfrac, band);
-    const float rad0 = recs[kLwRecFracs + P] * plankbnd;
-    rA = rad0 + reflect * rA;
-    rB = rad0 + reflect * rB;
-    put(number, 0, rA, rB);
-    load(0);
-  }
-  filled = 1;
-  // upward sweep, bottom to top: layer l gives level l + 1
-  for (int l = 0; l < nlay; ++l) {
+  for (int l0 = 0; l0 <= nlay; l0 += kLwRing) {
     if (live) {
-      const Next cur = nx;
-      if (l + 1 < nlay) load(l + 1);
-      lw_up(T, __float_as_uint(cur.tg), cur.fr, cur.bq, cur.efcl, (cur.word & bit) != 0u, cur.flag != 0.0f, rA, rB,
-            has_cloud);
-      put(number, filled, rA, rB);
+#pragma unroll
+      for (int j = 0; j < kLwRing; ++j) {
+        const int level = l0 + j;
+        if (level > nlay) break;
+        if (j == 0 && level == 0) {
+          // surface emission and reflection (surface_sums, lw:5648-5655)
+          const float bt = R.C.tsfc - 159.0f;
+          const int indbound = clampi(static_cast<int>(bt), 1, 180);
+          const float tbndfrac = bt - static_cast<float>(indbound);
+          const float reflect = 1.0f - R.C.semiss;
+          const float plankbnd = R.C.semiss * planck(T, indbound, tbndfrac, band);
+          load(0);
+          const float rad0 = nx.fr * plankbnd;
+          rA = rad0 + reflect * rA;
+          rB = rad0 + reflect * rB;
+        } else {
+          const Next cur = nx;
+          if (level < nlay) load(level);
+          lw_up(T, __float_as_uint(cur.tg), cur.fr, cur.bq, cur.efcl, (cur.word & bit) != 0u, cur.cloudy, rA, rB,
+                has_cloud);
+        }
+        put(number, j, rA, rB);
+      }
     }
-    if (++filled == kLwRing || l == nlay - 1) {
-      round.count = filled;
-      lw_sum_round(S, number, prev);
-      prev = round;
-      round.level0 += filled;
-      ++number;
-      filled = 0;
-    }
+    round.count = nlay + 1 - l0 < kLwRing ? nlay + 1 - l0 : kLwRing;
+    lw_sum_round(S, chain, number, prev);
+    prev = round;
+    round.level0 += kLwRing;
+    ++number;
   }
   __syncthreads();
-  if (tid >> 5 == 8) lw_band_terms(S, number - 1, prev);
+  if (tid >= 256) lw_band_terms(S, number - 1, prev);
   __syncthreads();
 
   // heating rates and theta tendencies (lw:5706-5712, 7040-7057) and the 2-D
