@@ -311,27 +311,29 @@ bool fill_tables(rrtmg_ctx *ctx, std::string &err) {
     const std::string p = "sw" + std::to_string(b + 16) + ".";
     SwBand &B = T.sw[b];
     int n = 0;
-    B.ka = dev_ptr<float>(ctx, p + "ka");
-    B.kb = dev_ptr<float>(ctx, p + "kb");
-    B.selfref = dev_ptr<float>(ctx, p + "selfref");
-    B.forref = dev_ptr<float>(ctx, p + "forref", &n);
-    B.forref_rows = B.forref ? n / sw_ngc[b] : 0;
+    auto add = [&](const char *name, const float **out, bool transposed = false) {
+      return add_padded(ctx, p + name, sw_ngc[b], sw_pad(b), out, 0, transposed);
+    };
+    add("ka", &B.ka);
+    add("kb", &B.kb);
+    add("selfref", &B.selfref);
+    B.forref_rows = add("forref", &B.forref);
     B.sfluxref = dev_ptr<float>(ctx, p + "sfluxref", &n);
     B.sflux_cols = B.sfluxref ? n / sw_ngc[b] : 0;
-    B.rayla = dev_ptr<float>(ctx, p + "rayla");
-    B.raylb = dev_ptr<float>(ctx, p + "raylb");
-    B.absch4 = dev_ptr<float>(ctx, p + "absch4");
-    B.abso3a = dev_ptr<float>(ctx, p + "abso3a");
-    B.abso3b = dev_ptr<float>(ctx, p + "abso3b");
-    B.absh2o = dev_ptr<float>(ctx, p + "absh2o");
-    B.absco2 = dev_ptr<float>(ctx, p + "absco2");
+    add("rayla", &B.rayla, true);
+    add("raylb", &B.raylb);
+    add("absch4", &B.absch4);
+    add("abso3a", &B.abso3a);
+    add("abso3b", &B.abso3b);
+    add("absh2o", &B.absh2o);
+    add("absco2", &B.absco2);
     const float *rayl = host_ptr<float>(ctx, p + "rayl", &n);
     if (rayl && n == 1) {
       B.rayl = rayl[0];
       B.rayl_g = nullptr;
     } else {
       B.rayl = 0.0f;
-      B.rayl_g = dev_ptr<float>(ctx, p + "rayl");
+      add("rayl", &B.rayl_g);
     }
     auto scalar = [&](const char *f) {
       const float *v = host_ptr<float>(ctx, p + f);

@@ -35,6 +35,11 @@ __host__ __device__ constexpr int lw_pad(int band) {
   return pad[band];
 }
 
+__host__ __device__ constexpr int sw_pad(int band) {
+  constexpr int pad[kSwBands] = {8, 12, 8, 8, 12, 12, 4, 12, 8, 8, 8, 8, 8, 12};
+  return pad[band];
+}
+
 // Longwave band tables in the padded layout; the Planck fractions of several
 // species ratios as (ratio, g-point).
 struct LwBand {
@@ -45,6 +50,8 @@ struct LwBand {
   int ka_rows, kb_rows;
 };
 
+// Shortwave band tables, in the padded layout except the solar source; rayla as
+// (species ratio, g-point).
 struct SwBand {
   const float *ka, *kb, *selfref, *forref, *sfluxref, *rayla, *raylb, *rayl_g;
   const float *absch4, *abso3a, *abso3b, *absh2o, *absco2;
@@ -95,6 +102,28 @@ __device__ __forceinline__ int jrow(int r, int n) {
 __device__ __forceinline__ float ld(const float *p) { return __ldg(p); }
 
 __device__ __forceinline__ float interpf(float lo, float hi, float f) { return lo + f * (hi - lo); }
+
+// ---------------------------------------------------------------------------
+// four g-points at a time: one binary32 operation per component and statement
+// ---------------------------------------------------------------------------
+__device__ __forceinline__ float4 add4(float4 a, float4 b) {
+  return make_float4(a.x + b.x, a.y + b.y, a.z + b.z, a.w + b.w);
+}
+__device__ __forceinline__ float4 mul4(float s, float4 a) { return make_float4(s * a.x, s * a.y, s * a.z, s * a.w); }
+__device__ __forceinline__ float4 mul4(float4 a, float4 b) {
+  return make_float4(a.x * b.x, a.y * b.y, a.z * b.z, a.w * b.w);
+}
+// interpf per component
+__device__ __forceinline__ float4 interp4(float4 lo, float4 hi, float f) {
+  return make_float4(lo.x + f * (hi.x - lo.x), lo.y + f * (hi.y - lo.y), lo.z + f * (hi.z - lo.z),
+                     lo.w + f * (hi.w - lo.w));
+}
+
+// Row `row`, quad q of a padded table with rows of PAD g-points.
+template <int PAD>
+__device__ __forceinline__ float4 row4(const float *tab, int row, int q) {
+  return __ldg(reinterpret_cast<const float4 *>(tab + row * PAD) + q);
+}
 
 // Pa -> hPa: the reference's binary64 quotient rounded once to binary32
 // (module_ra_rrtmg_common.py:70-82), identical to a binary32 division.

@@ -38,28 +38,6 @@ struct Layer {
   float cldfrac, clwp, ciwp, cswp, rel, rei, res;
 };
 
-// ---------------------------------------------------------------------------
-// four g-points at a time: one binary32 operation per component and statement
-// ---------------------------------------------------------------------------
-__device__ __forceinline__ float4 add4(float4 a, float4 b) {
-  return make_float4(a.x + b.x, a.y + b.y, a.z + b.z, a.w + b.w);
-}
-__device__ __forceinline__ float4 mul4(float s, float4 a) { return make_float4(s * a.x, s * a.y, s * a.z, s * a.w); }
-__device__ __forceinline__ float4 mul4(float4 a, float4 b) {
-  return make_float4(a.x * b.x, a.y * b.y, a.z * b.z, a.w * b.w);
-}
-// interpf per component
-__device__ __forceinline__ float4 interp4(float4 lo, float4 hi, float f) {
-  return make_float4(lo.x + f * (hi.x - lo.x), lo.y + f * (hi.y - lo.y), lo.z + f * (hi.z - lo.z),
-                     lo.w + f * (hi.w - lo.w));
-}
-
-// Row `row`, quad q of a padded table with rows of PAD g-points.
-template <int PAD>
-__device__ __forceinline__ float4 row4(const float *tab, int row, int q) {
-  return __ldg(reinterpret_cast<const float4 *>(tab + row * PAD) + q);
-}
-
 struct Spec {
   float sc, sp, fs;
   int js;

@@ -57,6 +57,10 @@ struct SLayer {
 #define RRTMG_SW_COUNT(name) +1
 constexpr int kSwLayerFields = 1 RRTMG_SW_LAYER_FLOATS(RRTMG_SW_COUNT) RRTMG_SW_LAYER_INTS(RRTMG_SW_COUNT);  // + cloud-water flag
 #undef RRTMG_SW_COUNT
+#define RRTMG_SW_INDEX(name) kSwField_##name,
+enum SwField { RRTMG_SW_LAYER_FLOATS(RRTMG_SW_INDEX) RRTMG_SW_LAYER_INTS(RRTMG_SW_INDEX) kSwField_cloud_water };
+#undef RRTMG_SW_INDEX
+static_assert(kSwField_cloud_water + 1 == kSwLayerFields, "layer fields");
 
 __device__ __forceinline__ float in3(const float *p, const Col &C, int k) {
   return ld(p + (static_cast<size_t>(C.i) * C.nk + k) * C.ny + C.j);
@@ -231,14 +235,17 @@ __device__ SLayer make_layer(const Tables &T, const SwArgs &a, const Col &C, int
 }
 
 // ---------------------------------------------------------------------------
-// taumol16..29 helpers
+// taumol16..29 (sw:4043-6675), four g-points at a time from the padded tables
+// (rrtmg_device.cuh): the set-up of a band once, its quads in a loop that is
+// not unrolled (unrolled over single g-points the 14 bands' code overran the
+// instruction caches: 10 of 26 stall cycles per instruction).
 // ---------------------------------------------------------------------------
 struct SwSpec {
-  float sc, fs, f[8];
+  float sc, fs;
   int js0;
 };
 
-__device__ __forceinline__ SwSpec sw_species(float primary, float ratio_secondary, const SLayer &L, float scale, int cap) {
+__device__ __forceinline__ SwSpec sw_species(float primary, float ratio_secondary, float scale, int cap) {
   SwSpec s;
   s.sc = primary + ratio_secondary;
   const float q = primary / s.sc;
@@ -246,60 +253,80 @@ __device__ __forceinline__ SwSpec sw_species(float primary, float ratio_secondar
   const float sm = scale * sp;
   const int js = 1 + static_cast<int>(sm);
   s.fs = sm - floorf(sm);
-  const float comp = 1.0f - s.fs;
   s.js0 = clampi(js - 1, 0, cap);
-  s.f[0] = comp * L.fac00;
-  s.f[1] = s.fs * L.fac00;
-  s.f[2] = comp * L.fac10;
-  s.f[3] = s.fs * L.fac10;
-  s.f[4] = comp * L.fac01;
-  s.f[5] = s.fs * L.fac01;
-  s.f[6] = comp * L.fac11;
-  s.f[7] = s.fs * L.fac11;
   return s;
 }
 
-__device__ __forceinline__ float k8(const float *tab, int ngc, int ns, int js0, int jt0, int jt10, int jp0, int jp1,
-                                    const float *f, int g) {
-  auto R = [&](int js, int jt, int jp) { return ld(tab + (((jp) * 5 + (jt)) * ns + (js)) * ngc + g); };
-  float s = f[0] * R(js0, jt0, jp0);
-  s = s + f[1] * R(js0 + 1, jt0, jp0);
-  s = s + f[2] * R(js0, jt0 + 1, jp0);
-  s = s + f[3] * R(js0 + 1, jt0 + 1, jp0);
-  s = s + f[4] * R(js0, jt10, jp1);
-  s = s + f[5] * R(js0 + 1, jt10, jp1);
-  s = s + f[6] * R(js0, jt10 + 1, jp1);
-  s = s + f[7] * R(js0 + 1, jt10 + 1, jp1);
-  return s;
-}
-
-__device__ __forceinline__ float k4(const float *tab, int ngc, int jt0, int jt10, int jp0, int jp1, const SLayer &L, int g) {
-  float s = L.fac00 * ld(tab + (jp0 * 5 + jt0) * ngc + g);
-  s = s + L.fac10 * ld(tab + (jp0 * 5 + jt0 + 1) * ngc + g);
-  s = s + L.fac01 * ld(tab + (jp1 * 5 + jt10) * ngc + g);
-  s = s + L.fac11 * ld(tab + (jp1 * 5 + jt10 + 1) * ngc + g);
-  return s;
-}
-
-__device__ __forceinline__ float self_interp(const SwBand &B, int ngc, const SLayer &L, int g) {
-  const int i0 = clampi(L.indself - 1, 0, 8);
-  const float s0 = ld(B.selfref + i0 * ngc + g);
-  return s0 + L.selffrac * (ld(B.selfref + (i0 + 1) * ngc + g) - s0);
-}
-
-__device__ __forceinline__ float for_interp(const SwBand &B, int ngc, const SLayer &L, int g, int cap) {
-  const int i0 = clampi(L.indfor - 1, 0, cap);
-  const int i1 = jrow(i0 + 1, B.forref_rows);
-  const float f0 = ld(B.forref + i0 * ngc + g);
-  return f0 + L.forfrac * (ld(B.forref + i1 * ngc + g) - f0);
-}
-
-// Gas optical depth and Rayleigh depth of band B (0 = band 16) at one layer.
-// The species weights returned in sp8/sp4 feed the solar-source rules.
-template <int B>
-__device__ __forceinline__ void sw_taumol(const Tables &T, const SLayer &L, float *taug, float *taur, SwSpec &sp8, SwSpec &sp4) {
-  constexpr int ngc = kNgc[B];
+// The species ratio of band B (0 = band 16); its eight-interval form below
+// laytrop (kLow) or the four-interval one of the bands that have two there.
+template <int B, bool kLow, class Field>
+__device__ __forceinline__ SwSpec sw_band_species(const SwBand &K, Field field) {
   constexpr int bn = B + 16;
+  constexpr float scale = kLow ? 8.0f : 4.0f;
+  constexpr int cap = kLow ? 7 : 3;
+  if constexpr (bn == 16) return sw_species(field(kSwField_colh2o), K.strrat1 * field(kSwField_colch4), scale, cap);
+  if constexpr (bn == 17 || bn == 19 || bn == 21)
+    return sw_species(field(kSwField_colh2o), K.strrat * field(kSwField_colco2), scale, cap);
+  if constexpr (bn == 18) return sw_species(field(kSwField_colh2o), K.strrat * field(kSwField_colch4), scale, cap);
+  if constexpr (bn == 22)
+    return sw_species(field(kSwField_colh2o), (1.6f * K.strrat) * field(kSwField_colo2), scale, cap);
+  if constexpr (bn == 24) return sw_species(field(kSwField_colh2o), K.strrat * field(kSwField_colo2), scale, cap);
+  if constexpr (bn == 28) return sw_species(field(kSwField_colo3), K.strrat * field(kSwField_colo2), scale, cap);
+  return SwSpec{0.0f, 0.0f, 0};
+}
+
+// Two-species interpolation over pressure, temperature and species ratio:
+// rows r0, r0 + 1, r0 + NS, r0 + NS + 1 and the same from r1, in this order.
+struct SwRows8 {
+  float f[8];
+  int r0, r1;
+};
+
+template <int NS>
+__device__ __forceinline__ SwRows8 sw_rows8(const SwSpec &s, const SLayer &L, int jt0, int jt10, int jp0, int jp1) {
+  SwRows8 k;
+  const float comp = 1.0f - s.fs;
+  k.f[0] = comp * L.fac00;
+  k.f[1] = s.fs * L.fac00;
+  k.f[2] = comp * L.fac10;
+  k.f[3] = s.fs * L.fac10;
+  k.f[4] = comp * L.fac01;
+  k.f[5] = s.fs * L.fac01;
+  k.f[6] = comp * L.fac11;
+  k.f[7] = s.fs * L.fac11;
+  k.r0 = (jp0 * 5 + jt0) * NS + s.js0;
+  k.r1 = (jp1 * 5 + jt10) * NS + s.js0;
+  return k;
+}
+
+template <int PAD, int NS>
+__device__ __forceinline__ float4 sum8(const float *tab, const SwRows8 &k, int q) {
+  float4 s = mul4(k.f[0], row4<PAD>(tab, k.r0, q));
+  s = add4(s, mul4(k.f[1], row4<PAD>(tab, k.r0 + 1, q)));
+  s = add4(s, mul4(k.f[2], row4<PAD>(tab, k.r0 + NS, q)));
+  s = add4(s, mul4(k.f[3], row4<PAD>(tab, k.r0 + NS + 1, q)));
+  s = add4(s, mul4(k.f[4], row4<PAD>(tab, k.r1, q)));
+  s = add4(s, mul4(k.f[5], row4<PAD>(tab, k.r1 + 1, q)));
+  s = add4(s, mul4(k.f[6], row4<PAD>(tab, k.r1 + NS, q)));
+  s = add4(s, mul4(k.f[7], row4<PAD>(tab, k.r1 + NS + 1, q)));
+  return s;
+}
+
+// One-species interpolation, rows (pressure * 5 + temperature).
+template <int PAD>
+__device__ __forceinline__ float4 sum4(const float *tab, int r0, int r1, const SLayer &L, int q) {
+  float4 s = mul4(L.fac00, row4<PAD>(tab, r0, q));
+  s = add4(s, mul4(L.fac10, row4<PAD>(tab, r0 + 1, q)));
+  s = add4(s, mul4(L.fac01, row4<PAD>(tab, r1, q)));
+  s = add4(s, mul4(L.fac11, row4<PAD>(tab, r1 + 1, q)));
+  return s;
+}
+
+// Gas and Rayleigh optical depths of band B (0 = band 16) at one layer:
+// emit(q, taug, taur) for g-points 4 q .. 4 q + 3.  field: the layer fields.
+template <int B, class Field, class Emit>
+__device__ __forceinline__ void sw_quads(const Tables &T, const SLayer &L, Field field, Emit emit) {
+  constexpr int PAD = sw_pad(B), Q = PAD / 4, bn = B + 16;
   const SwBand &K = T.sw[B];
   const bool trop = L.trop;
   const int jp = L.jp;
@@ -307,120 +334,88 @@ __device__ __forceinline__ void sw_taumol(const Tables &T, const SLayer &L, floa
   const int jp0 = clampi(jp - 1, 0, 11), jp1 = jp0 + 1;
   const int kjp0 = clampi(jp - 13, 0, 45), kjp1 = clampi(jp - 12, 0, 46);
   const float colh2o = L.colh2o, colmol = L.colmol;
-  if constexpr (bn == 16) sp8 = sw_species(colh2o, K.strrat1 * L.colch4, L, 8.0f, 7);
-  if constexpr (bn == 17 || bn == 19 || bn == 21) sp8 = sw_species(colh2o, K.strrat * L.colco2, L, 8.0f, 7);
-  if constexpr (bn == 18) sp8 = sw_species(colh2o, K.strrat * L.colch4, L, 8.0f, 7);
-  if constexpr (bn == 22) sp8 = sw_species(colh2o, (1.6f * K.strrat) * L.colo2, L, 8.0f, 7);
-  if constexpr (bn == 24) sp8 = sw_species(colh2o, K.strrat * L.colo2, L, 8.0f, 7);
-  if constexpr (bn == 28) sp8 = sw_species(L.colo3, K.strrat * L.colo2, L, 8.0f, 7);
-  if constexpr (bn == 17 || bn == 21) sp4 = sw_species(colh2o, K.strrat * L.colco2, L, 4.0f, 3);
-  if constexpr (bn == 28) sp4 = sw_species(L.colo3, K.strrat * L.colo2, L, 4.0f, 3);
-#pragma unroll
-  for (int g = 0; g < ngc; ++g) {
-    float tg = 0.0f, tr = 0.0f;
-    if constexpr (bn == 16) {
+  // bands with two species below laytrop, and those with two above it too
+  constexpr bool two = bn == 16 || bn == 17 || bn == 18 || bn == 19 || bn == 21 || bn == 22 || bn == 24 || bn == 28;
+  constexpr bool two_above = bn == 17 || bn == 21 || bn == 28;
+  SwSpec sp8{0.0f, 0.0f, 0};
+  if constexpr (two) sp8 = sw_band_species<B, true>(K, field);
+  SwRows8 k8{};
+  if constexpr (two) {
+    if (trop) {
+      k8 = sw_rows8<9>(sp8, L, jt0, jt10, jp0, jp1);
+    } else if constexpr (two_above) {
+      k8 = sw_rows8<5>(sw_band_species<B, false>(K, field), L, jt0, jt10, kjp0, kjp1);
+    }
+  }
+  const int r0 = trop ? jp0 * 5 + jt0 : kjp0 * 5 + jt0, r1 = trop ? jp1 * 5 + jt10 : kjp1 * 5 + jt10;
+  const int is = clampi(L.indself - 1, 0, 8);
+  constexpr int fcap = bn == 16 || bn == 23 || bn == 24 ? 1 : 2;
+  const int if0 = clampi(L.indfor - 1, 0, fcap), if1 = jrow(if0 + 1, K.forref_rows);
+  const float selffrac = L.selffrac, forfrac = L.forfrac, selffac = L.selffac, forfac = L.forfac;
+  auto self = [&](int q) {
+    return mul4(selffac, interp4(row4<PAD>(K.selfref, is, q), row4<PAD>(K.selfref, is + 1, q), selffrac));
+  };
+  auto foreign_raw = [&](int q) {
+    return interp4(row4<PAD>(K.forref, if0, q), row4<PAD>(K.forref, if1, q), forfrac);
+  };
+  auto foreign = [&](int q) { return mul4(forfac, foreign_raw(q)); };
+  const float o2cont = bn == 22 ? (4.35e-4f * L.colo2) / (350.0f * 2.0f) : 0.0f;
+  const float ray = colmol * K.rayl;
+#pragma unroll 1
+  for (int q = 0; q < Q; ++q) {
+    float4 tg = make_float4(0.0f, 0.0f, 0.0f, 0.0f), tr = make_float4(ray, ray, ray, ray);
+    if constexpr (bn == 16 || bn == 17 || bn == 18 || bn == 19 || bn == 21 || bn == 22) {
       if (trop) {
-        const float ta = k8(K.ka, ngc, 9, sp8.js0, jt0, jt10, jp0, jp1, sp8.f, g);
-        const float cont = colh2o * (L.selffac * self_interp(K, ngc, L, g) + L.forfac * for_interp(K, ngc, L, g, 1));
-        tg = sp8.sc * ta + cont;
+        const float4 cont = mul4(colh2o, add4(self(q), foreign(q)));
+        tg = add4(mul4(sp8.sc, sum8<PAD, 9>(K.ka, k8, q)), cont);
+        if constexpr (bn == 22) tg = add4(tg, make_float4(o2cont, o2cont, o2cont, o2cont));
+      } else if constexpr (bn == 17 || bn == 21) {
+        const float4 cont = mul4(colh2o * forfac, foreign_raw(q));
+        tg = add4(mul4(sp8.sc, sum8<PAD, 5>(K.kb, k8, q)), cont);
+      } else if constexpr (bn == 22) {
+        tg = add4(mul4(L.colo2 * 1.6f, sum4<PAD>(K.kb, r0, r1, L, q)), make_float4(o2cont, o2cont, o2cont, o2cont));
       } else {
-        tg = L.colch4 * k4(K.kb, ngc, jt0, jt10, kjp0, kjp1, L, g);
+        tg = mul4(bn == 19 ? L.colco2 : L.colch4, sum4<PAD>(K.kb, r0, r1, L, q));
       }
-      tr = colmol * K.rayl;
-    } else if constexpr (bn == 17 || bn == 21) {
-      if (trop) {
-        const float ta = k8(K.ka, ngc, 9, sp8.js0, jt0, jt10, jp0, jp1, sp8.f, g);
-        const float cont = colh2o * (L.selffac * self_interp(K, ngc, L, g) + L.forfac * for_interp(K, ngc, L, g, 2));
-        tg = sp8.sc * ta + cont;
-      } else {
-        const float sa = k8(K.kb, ngc, 5, sp4.js0, jt0, jt10, kjp0, kjp1, sp4.f, g);
-        const float cont = (colh2o * L.forfac) * for_interp(K, ngc, L, g, 2);
-        tg = sp8.sc * sa + cont;
-      }
-      tr = colmol * K.rayl;
-    } else if constexpr (bn == 18 || bn == 19) {
-      if (trop) {
-        const float ta = k8(K.ka, ngc, 9, sp8.js0, jt0, jt10, jp0, jp1, sp8.f, g);
-        const float cont = colh2o * (L.selffac * self_interp(K, ngc, L, g) + L.forfac * for_interp(K, ngc, L, g, 2));
-        tg = sp8.sc * ta + cont;
-      } else {
-        const float col = bn == 18 ? L.colch4 : L.colco2;
-        tg = col * k4(K.kb, ngc, jt0, jt10, kjp0, kjp1, L, g);
-      }
-      tr = colmol * K.rayl;
     } else if constexpr (bn == 20) {
-      if (trop) {
-        const float ta = k4(K.ka, ngc, jt0, jt10, jp0, jp1, L, g);
-        const float inner = (ta + L.selffac * self_interp(K, ngc, L, g)) + L.forfac * for_interp(K, ngc, L, g, 2);
-        tg = colh2o * inner + L.colch4 * ld(K.absch4 + g);
-      } else {
-        const float sa = k4(K.kb, ngc, jt0, jt10, kjp0, kjp1, L, g);
-        const float inner = sa + L.forfac * for_interp(K, ngc, L, g, 2);
-        tg = colh2o * inner + L.colch4 * ld(K.absch4 + g);
-      }
-      tr = colmol * K.rayl;
-    } else if constexpr (bn == 22) {
-      const float o2cont = (4.35e-4f * L.colo2) / (350.0f * 2.0f);
-      if (trop) {
-        const float ta = k8(K.ka, ngc, 9, sp8.js0, jt0, jt10, jp0, jp1, sp8.f, g);
-        const float cont = colh2o * (L.selffac * self_interp(K, ngc, L, g) + L.forfac * for_interp(K, ngc, L, g, 2));
-        tg = (sp8.sc * ta + cont) + o2cont;
-      } else {
-        const float sa = k4(K.kb, ngc, jt0, jt10, kjp0, kjp1, L, g);
-        tg = (L.colo2 * 1.6f) * sa + o2cont;
-      }
-      tr = colmol * K.rayl;
+      float4 inner = sum4<PAD>(trop ? K.ka : K.kb, r0, r1, L, q);
+      if (trop) inner = add4(inner, self(q));
+      inner = add4(inner, foreign(q));
+      tg = add4(mul4(colh2o, inner), mul4(L.colch4, row4<PAD>(K.absch4, 0, q)));
     } else if constexpr (bn == 23) {
-      if (trop) {
-        const float ta = k4(K.ka, ngc, jt0, jt10, jp0, jp1, L, g);
-        const float sum = (K.givfac * ta + L.selffac * self_interp(K, ngc, L, g)) + L.forfac * for_interp(K, ngc, L, g, 1);
-        tg = colh2o * sum;
-      }
-      tr = colmol * ld(K.rayl_g + g);
+      if (trop)
+        tg = mul4(colh2o, add4(add4(mul4(K.givfac, sum4<PAD>(K.ka, r0, r1, L, q)), self(q)), foreign(q)));
+      tr = mul4(colmol, row4<PAD>(K.rayl_g, 0, q));
     } else if constexpr (bn == 24) {
       if (trop) {
-        const float ta = k8(K.ka, ngc, 9, sp8.js0, jt0, jt10, jp0, jp1, sp8.f, g);
-        const float cont = colh2o * (L.selffac * self_interp(K, ngc, L, g) + L.forfac * for_interp(K, ngc, L, g, 1));
-        tg = (sp8.sc * ta + L.colo3 * ld(K.abso3a + g)) + cont;
-        const float r0 = ld(K.rayla + g * 9 + sp8.js0), r1 = ld(K.rayla + g * 9 + sp8.js0 + 1);
-        tr = colmol * (r0 + sp8.fs * (r1 - r0));
+        const float4 cont = mul4(colh2o, add4(self(q), foreign(q)));
+        tg = add4(add4(mul4(sp8.sc, sum8<PAD, 9>(K.ka, k8, q)), mul4(L.colo3, row4<PAD>(K.abso3a, 0, q))), cont);
+        tr = mul4(colmol, interp4(row4<PAD>(K.rayla, sp8.js0, q), row4<PAD>(K.rayla, sp8.js0 + 1, q), sp8.fs));
       } else {
-        const float sa = k4(K.kb, ngc, jt0, jt10, kjp0, kjp1, L, g);
-        tg = L.colo2 * sa + L.colo3 * ld(K.abso3b + g);
-        tr = colmol * ld(K.raylb + g);
+        tg = add4(mul4(L.colo2, sum4<PAD>(K.kb, r0, r1, L, q)), mul4(L.colo3, row4<PAD>(K.abso3b, 0, q)));
+        tr = mul4(colmol, row4<PAD>(K.raylb, 0, q));
       }
     } else if constexpr (bn == 25) {
-      if (trop) {
-        const float ta = k4(K.ka, ngc, jt0, jt10, jp0, jp1, L, g);
-        tg = colh2o * ta + L.colo3 * ld(K.abso3a + g);
-      } else {
-        tg = L.colo3 * ld(K.abso3b + g);
-      }
-      tr = colmol * ld(K.rayl_g + g);
+      if (trop)
+        tg = add4(mul4(colh2o, sum4<PAD>(K.ka, r0, r1, L, q)), mul4(L.colo3, row4<PAD>(K.abso3a, 0, q)));
+      else
+        tg = mul4(L.colo3, row4<PAD>(K.abso3b, 0, q));
+      tr = mul4(colmol, row4<PAD>(K.rayl_g, 0, q));
     } else if constexpr (bn == 26) {
-      tg = 0.0f;
-      tr = colmol * ld(K.rayl_g + g);
+      tr = mul4(colmol, row4<PAD>(K.rayl_g, 0, q));
     } else if constexpr (bn == 27) {
-      const float ab = trop ? k4(K.ka, ngc, jt0, jt10, jp0, jp1, L, g) : k4(K.kb, ngc, jt0, jt10, kjp0, kjp1, L, g);
-      tg = L.colo3 * ab;
-      tr = colmol * ld(K.rayl_g + g);
+      tg = mul4(L.colo3, sum4<PAD>(trop ? K.ka : K.kb, r0, r1, L, q));
+      tr = mul4(colmol, row4<PAD>(K.rayl_g, 0, q));
     } else if constexpr (bn == 28) {
-      if (trop) tg = sp8.sc * k8(K.ka, ngc, 9, sp8.js0, jt0, jt10, jp0, jp1, sp8.f, g);
-      else tg = sp8.sc * k8(K.kb, ngc, 5, sp4.js0, jt0, jt10, kjp0, kjp1, sp4.f, g);
-      tr = colmol * K.rayl;
+      tg = mul4(sp8.sc, trop ? sum8<PAD, 9>(K.ka, k8, q) : sum8<PAD, 5>(K.kb, k8, q));
     } else {  // 29
-      if (trop) {
-        const float ta = k4(K.ka, ngc, jt0, jt10, jp0, jp1, L, g);
-        const float wat = (ta + L.selffac * self_interp(K, ngc, L, g)) + L.forfac * for_interp(K, ngc, L, g, 2);
-        tg = colh2o * wat + L.colco2 * ld(K.absco2 + g);
-      } else {
-        const float sa = k4(K.kb, ngc, jt0, jt10, kjp0, kjp1, L, g);
-        tg = L.colco2 * sa + colh2o * ld(K.absh2o + g);
-      }
-      tr = colmol * K.rayl;
+      const float4 k = sum4<PAD>(trop ? K.ka : K.kb, r0, r1, L, q);
+      if (trop)
+        tg = add4(mul4(colh2o, add4(add4(k, self(q)), foreign(q))), mul4(L.colco2, row4<PAD>(K.absco2, 0, q)));
+      else
+        tg = add4(mul4(L.colco2, k), mul4(colh2o, row4<PAD>(K.absh2o, 0, q)));
     }
-    taug[g] = tg;
-    taur[g] = tr;
+    emit(q, tg, tr);
   }
 }
 
@@ -710,11 +705,11 @@ __device__ __forceinline__ RT4 reftra(const Tables &T, float zg, float mu, float
 }
 
 // Solar source of band B (the per-band rules of sw:4430-4450): the source
-// layer from the layers' jp (jp(l)), the spectral interpolation (js0, fs) of
-// the layer (spec(ls, js0, fs), asked only when the band uses it), and the
-// source of each g-point.
-template <int B, class JpFn, class SpecFn>
-__device__ __forceinline__ void sw_source(const Tables &T, const Col &C, JpFn jp, SpecFn spec, float *sflux) {
+// layer from the layers' jp (jp(l)), the spectral interpolation of that layer
+// from its fields (field(f, l), where the band uses it), and the source of
+// each g-point.
+template <int B, class JpFn, class FieldFn>
+__device__ __forceinline__ void sw_source(const Tables &T, const Col &C, JpFn jp, FieldFn field, float *sflux) {
   constexpr int ngc = kNgc[B];
   constexpr int bn = B + 16;
   const int n = C.nlay;
@@ -770,7 +765,12 @@ __device__ __forceinline__ void sw_source(const Tables &T, const Col &C, JpFn jp
   if constexpr (bn == 18 || bn == 19 || bn == 21 || bn == 22 || bn == 24) have = C.laytrop > 0;
   float src_fs = 0.0f;
   int src_js0 = 0;
-  if (have && ls >= 0) spec(ls, src_js0, src_fs);
+  if (have && ls >= 0) {
+    constexpr bool low = !(bn == 17 || bn == 28);
+    const SwSpec sp = sw_band_species<B, low>(K, [&](SwField f) { return field(f, ls); });
+    src_js0 = sp.js0;
+    src_fs = sp.fs;
+  }
 #pragma unroll
   for (int g = 0; g < ngc; ++g) {
     float sz = 0.0f;
@@ -911,11 +911,10 @@ __device__ __forceinline__ void sw_column_outputs(const SwArgs &a, const Col &C,
 //   sw_colprep_kernel  warp = day slot: the column set-up once (laytrop by a
 //                      warp vote over the layers);
 //   sw_layer_kernel    thread = (day slot, layer): the layer set-up into
-//                      layer fields, and jp into the layer record;
+//                      layer fields;
 //   sw_optics_kernel   thread = (day slot, layer), block = one band: the
-//                      band's gas and Rayleigh depths of every g-point, its
-//                      cloud optics and the spectral interpolation its solar
-//                      source uses, into the layer record;
+//                      band's gas and Rayleigh depths of every g-point and its
+//                      cloud optics, into the layer record;
 //   sw_source_kernel   thread = (day slot, band): the band's solar source;
 //   sw_sweep_kernel    block = kSweepCols day slots x 112 g-points, thread =
 //                      one g-point: the top-down pass (delta-Eddington layers,
@@ -924,16 +923,16 @@ __device__ __forceinline__ void sw_column_outputs(const SwArgs &a, const Col &C,
 //                      per-level spectral sums in g-point order in shared
 //                      memory, then heating and the 2-D outputs.
 // Records: per chunk slot a column record, then nlay layer records of kSwRec
-// floats (1,376 bytes per layer, 70 KB per day column at nk = 50), then the
-// kSwLayerFields layer fields (124 bytes per layer).  Each
-// band's g-points start on a 16-byte boundary (kPadOfs) so the optics kernel
-// writes whole float4s: taug at [0, 128), taur at [128, 256), the cloud optics
-// (tau, ssa, asm, unscaled tau) of band B at 256 + 4 B, the solar-source
-// interpolation (js0, fs) of band B at 312 + 2 B, jp at 340.
-constexpr int kSwRec = 344;
-constexpr int kSwRecTaur = 128, kSwRecCloud = 256, kSwRecSpec = 312, kSwRecJp = 340;
+// floats (1,248 bytes per layer, 64 KB per day column at nk = 50), then the
+// kSwLayerFields layer fields (124 bytes per layer).  Each band's g-points
+// start on a 16-byte boundary (kPadOfs) so the optics kernel writes whole
+// float4s: taug at [0, 128), taur at [128, 256), the cloud optics (tau, ssa,
+// asm, unscaled tau) of band B at 256 + 4 B.
+constexpr int kSwRec = 312;
+constexpr int kSwRecTaur = 128, kSwRecCloud = 256;
 constexpr int kPadOfs[kSwBands] = {0, 8, 20, 28, 36, 48, 60, 64, 76, 84, 92, 100, 108, 116};
-static_assert(kSwRecJp < kSwRec && kSwRec % 4 == 0, "record layout");
+static_assert(kSwRecCloud + 4 * kSwBands == kSwRec && kSwRec % 8 == 0, "record layout");
+static_assert(kPadOfs[kSwBands - 1] + sw_pad(kSwBands - 1) == kSwRecTaur, "padded g-points");
 __constant__ int kPadOfsDev[kSwBands] = {0, 8, 20, 28, 36, 48, 60, 64, 76, 84, 92, 100, 108, 116};
 
 struct SwColRec {
@@ -969,46 +968,59 @@ __global__ void __launch_bounds__(128) sw_colprep_kernel(Tables T, SwArgs a) {
   if (lane == 0) sw_colrecs(a)[u].C = C;
 }
 
-// ngc values of v to float4s at dst (the tail padded with zeros).
-template <int NGC>
-__device__ __forceinline__ void store_padded(float4 *dst, const float *v) {
-#pragma unroll
-  for (int q = 0; q < (NGC + 3) / 4; ++q) {
-    const int g = 4 * q;
-    dst[q] = make_float4(v[g], g + 1 < NGC ? v[g + 1] : 0.0f, g + 2 < NGC ? v[g + 2] : 0.0f,
-                         g + 3 < NGC ? v[g + 3] : 0.0f);
-  }
-}
+// 16-byte pieces of a warp's stage: gas depths, then Rayleigh depths, of 32 rows of up to 3
+constexpr int kSwStage = 2 * 32 * 3;
 
-// Band B of one layer record: gas and Rayleigh depths of every g-point, the
-// band's cloud optics (cldprmc_sw only where the layer holds cloud water; a
-// layer without any has the reference's inactive values 0, 1, 0, 0), and the
-// spectral interpolation its solar source uses (into spec[2 B], spec[2 B + 1]).
+// Band B of the layer records of a warp's 32 (layer, slot) pairs: gas and
+// Rayleigh depths of every g-point, and the band's cloud optics (cldprmc_sw
+// only where the layer holds cloud water; a layer without any has the
+// reference's inactive values 0, 1, 0, 0).  The layer fields are read inside
+// the band's own code, so that each band loads only those it uses, and the
+// depths go through the warp's shared stage, so that neighbouring lanes write
+// neighbouring 16-byte pieces.  record: the lane's layer record, or -1.
 template <int B>
-__device__ __forceinline__ void sw_band_record(const Tables &T, const SLayer &L, bool cloud_water, int iceflg,
-                                               float4 *rec, float *spec) {
-  constexpr int ngc = kNgc[B], bn = B + 16, pofs = kPadOfs[B];
-  SwSpec sp8, sp4;
-  sp8.sc = 0.0f; sp8.fs = 0.0f; sp8.js0 = 0;
-  sp4 = sp8;
-  float tg[ngc], tr[ngc];
-  sw_taumol<B>(T, L, tg, tr, sp8, sp4);
-  store_padded<ngc>(rec + pofs / 4, tg);
-  store_padded<ngc>(rec + (kSwRecTaur + pofs) / 4, tr);
-  float4 cq = make_float4(0.0f, 1.0f, 0.0f, 0.0f);
-  if (cloud_water) {
-    const CloudOpt o = sw_cloud(T, L, B, iceflg);
-    cq = make_float4(o.tau, o.ssa, o.asm_, o.taor);
+__device__ __forceinline__ void sw_band_record(const Tables &T, const SwArgs &a, const float *fld, size_t fstride,
+                                               int record, float4 *stage) {
+  constexpr int Q = sw_pad(B) / 4, kRow = Q | 1;
+  const int lane = threadIdx.x & 31;
+  if (record >= 0) {
+    auto field = [&](SwField f) { return fld[static_cast<size_t>(f) * fstride]; };
+    SLayer L;
+#define RRTMG_SW_GET(name) L.name = field(kSwField_##name);
+#define RRTMG_SW_GETI(name) L.name = __float_as_int(field(kSwField_##name));
+    RRTMG_SW_LAYER_FLOATS(RRTMG_SW_GET)
+    RRTMG_SW_LAYER_INTS(RRTMG_SW_GETI)
+#undef RRTMG_SW_GET
+#undef RRTMG_SW_GETI
+    float4 *row = stage + lane * kRow;
+    sw_quads<B>(T, L, field, [&](int q, float4 tg, float4 tr) {
+      row[q] = tg;
+      row[q + kSwStage / 2] = tr;
+    });
+    float4 cq = make_float4(0.0f, 1.0f, 0.0f, 0.0f);
+    if (__float_as_int(field(kSwField_cloud_water)) != 0) {
+      const CloudOpt o = sw_cloud(T, L, B, a.iceflg);
+      cq = make_float4(o.tau, o.ssa, o.asm_, o.taor);
+    }
+    reinterpret_cast<float4 *>(sw_layrecs(a) + static_cast<size_t>(record) * kSwRec)[kSwRecCloud / 4 + B] = cq;
   }
-  rec[kSwRecCloud / 4 + B] = cq;
-  const SwSpec &sp = (bn == 17 || bn == 28) ? sp4 : sp8;
-  spec[2 * B] = __int_as_float(sp.js0);
-  spec[2 * B + 1] = sp.fs;
+  __syncwarp();
+  float *recs = sw_layrecs(a) + kPadOfs[B];
+#pragma unroll
+  for (int i = 0; i < Q; ++i) {
+    const int e = i * 32 + lane, r = e / Q, q = e - r * Q;
+    const int rec = __shfl_sync(0xffffffffu, record, r);
+    if (rec >= 0) {
+      float4 *out = reinterpret_cast<float4 *>(recs + static_cast<size_t>(rec) * kSwRec) + q;
+      out[0] = stage[r * kRow + q];
+      out[kSwRecTaur / 4] = stage[r * kRow + q + kSwStage / 2];
+    }
+  }
 }
 
 // sw_layer_kernel: thread = (layer, chunk slot), slots fastest: the layer
 // set-up (make_layer) and cldprmc_sw's activity test once, stored as layer
-// fields, and the layer's jp into its record.
+// fields.
 __global__ void __launch_bounds__(128) sw_layer_kernel(Tables T, SwArgs a) {
   const int n = a.nk + 1;
   const long long idx = static_cast<long long>(blockIdx.x) * blockDim.x + threadIdx.x;
@@ -1030,68 +1042,6 @@ __global__ void __launch_bounds__(128) sw_layer_kernel(Tables T, SwArgs a) {
 #undef RRTMG_SW_PUT
 #undef RRTMG_SW_PUTI
   fld[static_cast<size_t>(f) * fstride] = __int_as_float(cloud_water ? 1 : 0);
-  float4 *rec = reinterpret_cast<float4 *>(sw_layrecs(a) + (static_cast<size_t>(u) * n + l) * kSwRec);
-  rec[kSwRecJp / 4] = make_float4(__int_as_float(L.jp), 0.0f, 0.0f, 0.0f);
-}
-
-// sw_optics_kernel: one band per block.  Blocks of (layer, chunk slot) pairs
-// are taken kSwOpticsGroup at a time through all 14 bands, so that a group's
-// layer fields (about 8 MB) are read from L2 by the later bands; each block
-// runs one band's code only.
-// Resident blocks per SM the register allocation must allow: 6 (80
-// registers); at 8 (64 registers, with spills) the 425 x 425 x 50 step took
-// 118 ms instead of 103.
-constexpr int kSwOpticsGroup = 512;
-constexpr int kSwOpticsMinBlocks = 6;
-constexpr int kSwSweepMinBlocks = 4;
-__global__ void __launch_bounds__(128, kSwOpticsMinBlocks) sw_optics_kernel(Tables T, SwArgs a, int nblk) {
-  const int group = blockIdx.x / (kSwOpticsGroup * kSwBands);
-  const int g0 = group * kSwOpticsGroup;
-  const int gsize = nblk - g0 < kSwOpticsGroup ? nblk - g0 : kSwOpticsGroup;
-  const int within = blockIdx.x - group * kSwOpticsGroup * kSwBands;
-  const int band = within / gsize;
-  const int blk = g0 + (within - band * gsize);
-  const int n = a.nk + 1;
-  const long long idx = static_cast<long long>(blk) * blockDim.x + threadIdx.x;
-  const int l = static_cast<int>(idx / a.chunk_count);
-  const int u = static_cast<int>(idx - static_cast<long long>(l) * a.chunk_count);
-  if (l >= n || a.chunk_first + u >= *a.nday) return;
-  const float *fld = sw_layfields(a) + static_cast<size_t>(l) * a.chunk_capacity + u;
-  const size_t fstride = static_cast<size_t>(n) * a.chunk_capacity;
-  SLayer L;
-  int f = 0;
-#define RRTMG_SW_GET(name) L.name = fld[static_cast<size_t>(f++) * fstride];
-#define RRTMG_SW_GETI(name) L.name = __float_as_int(fld[static_cast<size_t>(f++) * fstride]);
-  RRTMG_SW_LAYER_FLOATS(RRTMG_SW_GET)
-  RRTMG_SW_LAYER_INTS(RRTMG_SW_GETI)
-#undef RRTMG_SW_GET
-#undef RRTMG_SW_GETI
-  const bool cloud_water = __float_as_int(fld[static_cast<size_t>(f) * fstride]) != 0;
-  const int iceflg = sw_colrecs(a)[u].C.iceflg;
-  float *rec = sw_layrecs(a) + (static_cast<size_t>(u) * n + l) * kSwRec;
-  float spec[2 * kSwBands];
-#define RRTMG_SW_OPT(B)                                                                                    \
-  {                                                                                                        \
-    sw_band_record<B>(T, L, cloud_water, iceflg, reinterpret_cast<float4 *>(rec), spec);                   \
-    *reinterpret_cast<float2 *>(rec + kSwRecSpec + 2 * (B)) = make_float2(spec[2 * (B)], spec[2 * (B) + 1]); \
-  }
-  switch (band) {
-    case 0: RRTMG_SW_OPT(0); break;
-    case 1: RRTMG_SW_OPT(1); break;
-    case 2: RRTMG_SW_OPT(2); break;
-    case 3: RRTMG_SW_OPT(3); break;
-    case 4: RRTMG_SW_OPT(4); break;
-    case 5: RRTMG_SW_OPT(5); break;
-    case 6: RRTMG_SW_OPT(6); break;
-    case 7: RRTMG_SW_OPT(7); break;
-    case 8: RRTMG_SW_OPT(8); break;
-    case 9: RRTMG_SW_OPT(9); break;
-    case 10: RRTMG_SW_OPT(10); break;
-    case 11: RRTMG_SW_OPT(11); break;
-    case 12: RRTMG_SW_OPT(12); break;
-    default: RRTMG_SW_OPT(13); break;
-  }
-#undef RRTMG_SW_OPT
 }
 
 #define RRTMG_SW_BAND_SWITCH(band, CALL) \
@@ -1112,23 +1062,53 @@ __global__ void __launch_bounds__(128, kSwOpticsMinBlocks) sw_optics_kernel(Tabl
     default: CALL(13); break;            \
   }
 
+// sw_optics_kernel: one band per block.  Blocks of (layer, chunk slot) pairs
+// are taken kSwOpticsGroup at a time through all 14 bands, so that a group's
+// layer fields are read from L2 by the later bands and its records, which the
+// bands fill piece by piece, leave L2 whole; each block runs one band's code
+// only.  SW optics of 425 x 425 x 50 (day list, set-up and source included):
+// 6.85 ms with groups of 128 and 5 blocks per SM (96 registers), 7.0 ms at 6
+// blocks (80 registers), 9.4 ms with groups of 512; 14.2 ms with the g-points
+// unrolled over unpadded tables and stores of a lane per record.
+constexpr int kSwOpticsGroup = 128;
+constexpr int kSwOpticsMinBlocks = 5;
+constexpr int kSwSweepMinBlocks = 4;
+__global__ void __launch_bounds__(128, kSwOpticsMinBlocks) sw_optics_kernel(Tables T, SwArgs a, int nblk) {
+  const int group = blockIdx.x / (kSwOpticsGroup * kSwBands);
+  const int g0 = group * kSwOpticsGroup;
+  const int gsize = nblk - g0 < kSwOpticsGroup ? nblk - g0 : kSwOpticsGroup;
+  const int within = blockIdx.x - group * kSwOpticsGroup * kSwBands;
+  const int band = within / gsize;
+  const int blk = g0 + (within - band * gsize);
+  const int n = a.nk + 1;
+  const long long idx = static_cast<long long>(blk) * blockDim.x + threadIdx.x;
+  const int l = static_cast<int>(idx / a.chunk_count);
+  const int u = static_cast<int>(idx - static_cast<long long>(l) * a.chunk_count);
+  const bool live = l < n && a.chunk_first + u < *a.nday;
+  if (!__any_sync(0xffffffffu, live)) return;  // whole warps
+  __shared__ float4 stages[4][kSwStage];
+  float4 *stage = stages[threadIdx.x >> 5];
+  const float *fld = sw_layfields(a) + static_cast<size_t>(l) * a.chunk_capacity + u;
+  const size_t fstride = static_cast<size_t>(n) * a.chunk_capacity;
+  const int record = live ? u * n + l : -1;
+#define RRTMG_SW_OPT(B) sw_band_record<B>(T, a, fld, fstride, record, stage)
+  RRTMG_SW_BAND_SWITCH(band, RRTMG_SW_OPT)
+#undef RRTMG_SW_OPT
+}
+
 __global__ void __launch_bounds__(128) sw_source_kernel(Tables T, SwArgs a) {
   const int u = blockIdx.x * blockDim.x + threadIdx.x;
   if (u >= a.chunk_count || a.chunk_first + u >= *a.nday) return;
   const int n = a.nk + 1;
   SwColRec &R = sw_colrecs(a)[u];
-  const float *recs = sw_layrecs(a) + static_cast<size_t>(u) * n * kSwRec;
   const int band = blockIdx.y;
-  auto jp = [&](int l) { return __float_as_int(recs[static_cast<size_t>(l) * kSwRec + kSwRecJp]); };
-  auto spec = [&](int ls, int &js0, float &fs) {
-    const float *q = recs + static_cast<size_t>(ls) * kSwRec + kSwRecSpec + 2 * band;
-    js0 = __float_as_int(q[0]);
-    fs = q[1];
-  };
+  const float *fld = sw_layfields(a) + u;
+  auto field = [&](int f, int l) { return fld[(static_cast<size_t>(f) * n + l) * a.chunk_capacity]; };
+  auto jp = [&](int l) { return __float_as_int(field(kSwField_jp, l)); };
 #define RRTMG_SW_SRC(B)                                 \
   {                                                     \
     constexpr int gofs_ = kGofs[B];                     \
-    sw_source<B>(T, R.C, jp, spec, R.sflux + gofs_);    \
+    sw_source<B>(T, R.C, jp, field, R.sflux + gofs_);   \
   }
   RRTMG_SW_BAND_SWITCH(band, RRTMG_SW_SRC)
 #undef RRTMG_SW_SRC
