@@ -21,8 +21,8 @@ LIB = HERE / "librrtmg_b200.so"
 SOURCES = ("rrtmg_capi.cu", "rrtmg_mcica.cu", "rrtmg_lw.cu", "rrtmg_lw_fused.cu", "rrtmg_sw.cu", "surrogate_gemm.cu",
            "surrogate_ops.cu", "surrogate_capi.cu", "surrogate_mlp.cu", "rrtmg_prologue.cu",
            "rrtmg_tendency.cu", "rrtmg_tables.cu", "rrtmg_status.cu", "rrtmg_ffi.cu")
-HEADERS = ("rrtmg_device.cuh", "rrtmg_lw_common.cuh", "rrtmg_lw_gas.cuh", "rrtmg_kernels.h", "surrogate_kernels.h",
-           "umma_common.cuh", "kiss_jump_host.h", "xla_ffi_abi.h")
+HEADERS = ("rrtmg_device.cuh", "rrtmg_divide.cuh", "rrtmg_lw_common.cuh", "rrtmg_lw_gas.cuh", "rrtmg_kernels.h",
+           "surrogate_kernels.h", "umma_common.cuh", "kiss_jump_host.h", "xla_ffi_abi.h")
 ARCH = ["-gencode", "arch=compute_100a,code=sm_100a"]
 NVCC_FLAGS = ["-O3", "-lineinfo", "-std=c++17", "--expt-relaxed-constexpr", "-fmad=false",
               "-prec-div=true", "-prec-sqrt=true", "-ftz=false",

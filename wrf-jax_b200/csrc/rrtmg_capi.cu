@@ -386,6 +386,15 @@ bool fill_tables(rrtmg_ctx *ctx, std::string &err) {
   T.fdlice3 = dev_ptr<float>(ctx, "sw.fdlice3");
   T.sw_pade_exp = dev_ptr<float>(ctx, "sw.pade_exp_tbl", &n);
   T.sw_ntbl = n - 1;
+  if (const float *ex = host_ptr<float>(ctx, "sw.pade_exp_tbl")) {
+    const size_t base = (ctx->padded.size() + 63) / 64 * 64;
+    ctx->padded.resize(base + 2 * static_cast<size_t>(n));
+    for (int i = 0; i < n; ++i) {
+      ctx->padded[base + 2 * i] = ex[i];
+      ctx->padded[base + 2 * i + 1] = 1.0f / ex[i];
+    }
+    ctx->padded_refs.emplace_back(reinterpret_cast<const float **>(&T.sw_pade), base);
+  }
   const float *sbp = host_ptr<float>(ctx, "sw.pade_bpade");
   T.sw_bpade = sbp ? sbp[0] : 0.0f;
   T.retab = dev_ptr<float>(ctx, "retab");

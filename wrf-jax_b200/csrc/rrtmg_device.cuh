@@ -74,6 +74,7 @@ struct Tables {
   const float *sw_preflog, *sw_tref;
   const float *extliq1, *ssaliq1, *asyliq1, *extice3, *ssaice3, *asyice3, *fdlice3;
   const float *sw_pade_exp;
+  const float2 *sw_pade;  // (exp, 1 / exp) of each position
   float sw_bpade;
   int sw_ntbl;
   // shared

@@ -19,6 +19,7 @@
 #include <atomic>
 
 #include "rrtmg_device.cuh"
+#include "rrtmg_divide.cuh"
 #include "rrtmg_kernels.h"
 
 namespace rrtmg {
@@ -537,12 +538,6 @@ __device__ __forceinline__ float zero_over(float x) {
   return __int_as_float(__float_as_int(x) & static_cast<int>(0x80000000u));
 }
 
-// The four components of x and y have the same bit patterns.
-__device__ __forceinline__ bool same_bits(float4 x, float4 y) {
-  return ((__float_as_uint(x.x) ^ __float_as_uint(y.x)) | (__float_as_uint(x.y) ^ __float_as_uint(y.y)) |
-          (__float_as_uint(x.z) ^ __float_as_uint(y.z)) | (__float_as_uint(x.w) ^ __float_as_uint(y.w))) == 0u;
-}
-
 // FP64 mode: the Pade lookup of exp(-v) (sw:2722-2760) with binary64
 // arithmetic; the table is the same binary32 data.
 __device__ __forceinline__ double exp_lookup64(const Tables &T, double v) {
@@ -702,6 +697,229 @@ __device__ __forceinline__ RT4 reftra(const Tables &T, float zg, float mu, float
   r.refd = g2 * (1.0f - zemm) * zdend;
   r.trad = zrk2 * zem1 * zdend;
   return r;
+}
+
+// ---------------------------------------------------------------------------
+// Layer optics of one g-point for the sweep: delta-Eddington results and the
+// direct beam's transmittances with and without delta scaling.
+// ---------------------------------------------------------------------------
+struct SwOptics {
+  RT4 rt;
+  float dbt, dbt_nd;
+};
+
+// The clear-sky layer's inputs that the cloudy one builds on.
+struct SwClear {
+  float ztau, ztauc, zomcc, zgcc;
+};
+
+// Clear sky, any operands: gas + Rayleigh, no aerosol (sw:6923-6927).  Divisions
+// whose divisor is exactly 1 are skipped: their quotient is the dividend.
+template <bool kFp64>
+__device__ __forceinline__ SwOptics sw_clear_any(const Tables &T, float tg, float tr, float mu, SwClear &c) {
+  SwOptics o;
+  c.ztau = (tr + tg) + 0.0f;
+  const float zom0 = tr + 0.0f * 1.0f;
+  const float zgr = zero_over(zom0);  // 0 * 1 * 0 / zom
+  const float zom = zom0 / c.ztau;
+  const float v_nd = c.ztau / mu;
+  o.dbt_nd = exp_lookup(T, v_nd);
+  const float zf = zgr * zgr;
+  const float zwf = zom * zf;
+  const float d_w = 1.0f - zwf;
+  c.ztauc = d_w * c.ztau;
+  c.zomcc = div_or_same(zom - zwf, d_w);
+  c.zgcc = div_or_same(zgr - zf, 1.0f - zf);
+  // ztauc is ztau exactly when d_w == 1
+  const float v_c = d_w == 1.0f ? v_nd : c.ztauc / mu;
+  o.dbt = d_w == 1.0f ? o.dbt_nd : exp_lookup(T, v_c);
+  o.rt = reftra<kFp64>(T, c.zgcc, mu, c.ztauc, c.zomcc, v_c, o.dbt);
+  return o;
+}
+
+// A cloudy g-point layer, any operands (sw:6935-7010): cld = the band's cloud
+// (tau, ssa, asm, unscaled tau).  The reference's mix clear * c + cloud * o has
+// clear = 0, cloud = 1 here.
+template <bool kFp64>
+__device__ __forceinline__ SwOptics sw_cloudy_any(const Tables &T, const SwClear &c, const SwOptics &oc, float4 cld,
+                                                  float mu) {
+  const float clear = 0.0f, cloud = 1.0f;
+  const float tcld = cld.x, wcld = cld.y, gcld = cld.z, taor = cld.w;
+  const float dbtmo_nd = exp_lookup(T, (c.ztau + taor) / mu);
+  const float ztauo = c.ztauc + tcld;
+  float zomco = c.ztauc * c.zomcc + tcld * wcld;
+  const float zgco = (tcld * wcld * gcld + c.ztauc * c.zomcc * c.zgcc) / zomco;
+  zomco = zomco / ztauo;
+  const float v_o = ztauo / mu;
+  const float dbtmo = exp_lookup(T, v_o);
+  const RT4 o = reftra<kFp64>(T, zgco, mu, ztauo, zomco, v_o, dbtmo);
+  SwOptics t;
+  t.dbt_nd = clear * oc.dbt_nd + cloud * dbtmo_nd;
+  t.rt.ref = clear * oc.rt.ref + cloud * o.ref;
+  t.rt.refd = clear * oc.rt.refd + cloud * o.refd;
+  t.rt.tra = clear * oc.rt.tra + cloud * o.tra;
+  t.rt.trad = clear * oc.rt.trad + cloud * o.trad;
+  t.dbt = clear * oc.dbt + cloud * dbtmo;
+  return t;
+}
+
+// ---------------------------------------------------------------------------
+// The same layers with their operands checked once: every division is then
+// within the ranges of rrtmg_divide.cuh, quotients by mu and by equal divisors
+// share a reciprocal, and the reciprocals of table exponentials come from the
+// table.  `ok` turns false where an operand is outside (the caller then takes
+// the *_any form); inside, the results are the same bits.  (Where a zero
+// differs only in its sign it stays a zero in every flux.)
+// ---------------------------------------------------------------------------
+constexpr float kSafeLow = 0x1p-90f, kSafeHigh = 0x1p60f;
+
+struct SwExp {
+  float e, r;  // exp(-v) by the table or the series, and its reciprocal
+};
+
+__device__ __forceinline__ SwExp exp_pair(const Tables &T, float v) {
+  SwExp x;
+  if (v <= 0.06f) {
+    x.e = (1.0f - v) + (0.5f * v) * v;
+    x.r = recip_in_range(x.e);
+  } else {
+    const float tblind = quotient_in_range(v, T.sw_bpade + v);
+    const int it = clampi(static_cast<int>(static_cast<float>(T.sw_ntbl) * tblind + 0.5f), 0, T.sw_ntbl);
+    const float2 p = __ldg(T.sw_pade + it);
+    x.e = p.x;
+    x.r = p.y;
+  }
+  return x;
+}
+
+__device__ __forceinline__ bool safe_size(float a) { return fabsf(a) >= kSafeLow && fabsf(a) <= kSafeHigh; }
+
+// reftra's general and conservative branches.  kIso: zg = 0 (no cloud), where
+// g3 = g4 = 1/2 and za1, za2 are one value.  zw in (0, 1], zto1 in
+// [kSafeLow, kSafeHigh].
+template <bool kIso>
+__device__ __forceinline__ RT4 reftra_safe(const Tables &T, float zg, float mu, float zto1, float zw, float zto1_mu,
+                                           SwExp ex2, bool conservative, bool &ok) {
+  RT4 r;
+  const float eps = 1.0e-8f;
+  const float zg3 = 3.0f * zg;
+  const float g1 = kIso ? (8.0f - zw * 5.0f) * 0.25f : (8.0f - zw * (5.0f + zg3)) * 0.25f;
+  const float g2 = kIso ? 3.0f * zw * 0.25f : 3.0f * (zw * (1.0f - zg)) * 0.25f;
+  const float g3 = kIso ? 0.5f : (2.0f - zg3 * mu) * 0.25f;
+  const float g4 = kIso ? 0.5f : 1.0f - g3;
+  if (zto1_mu > 500.0f) ex2 = exp_pair(T, 500.0f);
+  if (conservative) {
+    const float za = g1 * mu;
+    const float za1 = za - g3;
+    const float zgt = g1 * zto1;
+    const float num = zgt - za1 * (1.0f - ex2.e), den = 1.0f + zgt, y = recip_in_range(den);
+    ok = ok && safe_size(num);
+    r.ref = quotient_by(num, den, y);
+    r.tra = 1.0f - r.ref;
+    r.refd = quotient_by(zgt, den, y);
+    r.trad = 1.0f - r.refd;
+    if (ex2.e == 1.0f) { r.ref = 0.0f; r.tra = 1.0f; r.refd = 0.0f; r.trad = 1.0f; }
+    return r;
+  }
+  const float za1 = g1 * g4 + g2 * g3;
+  const float za2 = kIso ? za1 : g1 * g3 + g2 * g4;
+  const float rad = g1 * g1 - g2 * g2;
+  const float zrk = sqrtf(rad > 0.0f ? rad : 0.0f);
+  const float zrp = zrk * mu;
+  const float zrp1 = 1.0f + zrp, zrm1 = 1.0f - zrp, zrk2 = 2.0f * zrk;
+  const float zrpp = 1.0f - zrp * zrp;
+  const float zrkg = zrk + g1;
+  const float s3 = zrk * g3, s4 = zrk * g4;
+  const float zr1 = zrm1 * (za2 + s3);
+  const float zr2 = zrp1 * (za2 - s3);
+  const float zr3 = zrk2 * (g3 - za2 * mu);
+  const float zr4 = zrpp * zrkg;
+  const float zr5 = zrpp * (zrk - g1);
+  const float zt1 = zrp1 * (za1 + s4);
+  const float zt2 = zrm1 * (za1 - s4);
+  const float zt3 = zrk2 * (g4 + za1 * mu);
+  const float zbeta = quotient_in_range(g1 - zrk, zrkg);
+  float ze1 = zrk * zto1;
+  if (ze1 > 500.0f) ze1 = 500.0f;
+  const SwExp ex1 = exp_pair(T, ze1);
+  const float zden = zr4 * ex1.r + zr5 * ex1.e;
+  if ((zden >= -eps) && (zden <= eps)) {
+    r.ref = eps;
+    r.tra = ex2.e;
+  } else {
+    const float y = recip_in_range(zden);
+    const float nr = zw * (zr1 * ex1.r - zr2 * ex1.e - zr3 * ex2.e);
+    const float nt = ex2.e * zw * (zt1 * ex1.r - zt2 * ex1.e - zt3 * ex2.r);
+    const float least = fabsf(zden) * 0x1p-95f;  // of a numerator, for a quotient in range
+    ok = ok && fabsf(zden) <= 0x1p90f && fabsf(nr) <= 0x1p90f && fabsf(nt) <= 0x1p90f &&
+         fabsf(nr) >= fmaxf(least, kSafeLow) && fabsf(nt) >= fmaxf(least, kSafeLow);
+    r.ref = quotient_by(nr, zden, y);
+    r.tra = ex2.e - quotient_by(nt, zden, y);
+  }
+  const float zemm = ex1.e * ex1.e;
+  const float dd = (1.0f - zbeta * zemm) * zrkg;
+  ok = ok && safe_size(dd);
+  const float zdend = recip_in_range(dd);
+  r.refd = g2 * (1.0f - zemm) * zdend;
+  r.trad = zrk2 * ex1.e * zdend;
+  return r;
+}
+
+// y_mu = recip_in_range(mu)
+__device__ __forceinline__ SwOptics sw_clear_safe(const Tables &T, float tg, float tr, float mu, float y_mu, SwClear &c,
+                                                  bool &ok) {
+  SwOptics o;
+  c.ztau = (tr + tg) + 0.0f;
+  const float zom = quotient_in_range(tr, c.ztau);
+  ok = tr >= kSafeLow && c.ztau <= kSafeHigh && zom >= 0x1p-30f && zom <= 1.0f && mu >= 0x1p-34f && mu <= 2.0f;
+  // zg = 0: no delta scaling (sw:6923-6927 gives zf = 0), scaled = unscaled
+  c.ztauc = c.ztau;
+  c.zomcc = zom;
+  c.zgcc = 0.0f;
+  const float v = quotient_by(c.ztau, mu, y_mu);
+  const SwExp ex2 = exp_pair(T, v);
+  o.dbt = ex2.e;
+  o.dbt_nd = ex2.e;
+  o.rt = reftra_safe<true>(T, 0.0f, mu, c.ztau, zom, v, ex2, zom >= 0.9999995f, ok);
+  return o;
+}
+
+__device__ __forceinline__ SwOptics sw_cloudy_safe(const Tables &T, const SwClear &c, float4 cld, float mu, float y_mu,
+                                                   bool &ok) {
+  SwOptics t;
+  const float tcld = cld.x, wcld = cld.y, gcld = cld.z, taor = cld.w;
+  t.dbt_nd = exp_pair(T, quotient_by(c.ztau + taor, mu, y_mu)).e;
+  const float ztauo = c.ztauc + tcld;
+  const float scat = c.ztauc * c.zomcc + tcld * wcld;
+  const float scatg = tcld * wcld * gcld + 0.0f;  // the clear sky's share has zgcc = 0
+  const float zg = quotient_in_range(scatg, scat);
+  const float zw = quotient_in_range(scat, ztauo);
+  ok = ok && tcld >= 0.0f && taor >= 0.0f && taor <= kSafeHigh && ztauo <= kSafeHigh && scat >= kSafeLow &&
+       scatg >= kSafeLow && zg <= 0.99f && zw >= 0x1p-30f && zw <= 1.0f;
+  // whether zw / (1 - (1 - zw) (zg / (1 - zg))^2) reaches 0.9999995: far below
+  // it by an approximate divisor, else by the reference's own quotients
+  float sr_approx = __fdividef(zg, 1.0f - zg);
+  const float den_approx = 1.0f - (1.0f - zw) * sr_approx * sr_approx;
+  bool conservative = false;
+  if (!(den_approx > 0.05f && zw < 0.99f * den_approx)) {
+    const float sr = div_or_same(zg, 1.0f - zg);
+    const float denom = 1.0f - (1.0f - zw) * sr * sr;
+    conservative = (denom != 0.0f ? div_or_same(zw, denom) : 0.0f) >= 0.9999995f;
+  }
+  const float v = quotient_by(ztauo, mu, y_mu);
+  const SwExp ex2 = exp_pair(T, v);
+  t.dbt = ex2.e;
+  t.rt = reftra_safe<false>(T, zg, mu, ztauo, zw, v, ex2, conservative, ok);
+  return t;
+}
+
+// The *_any forms out of line, for the rare layers with operands out of range.
+__device__ __noinline__ SwOptics sw_clear_slow(const Tables &T, float tg, float tr, float mu, SwClear &c) {
+  return sw_clear_any<false>(T, tg, tr, mu, c);
+}
+__device__ __noinline__ SwOptics sw_cloudy_slow(const Tables &T, const SwClear &c, const SwOptics &oc, float4 cld,
+                                                float mu) {
+  return sw_cloudy_any<false>(T, c, oc, cld, mu);
 }
 
 // Solar source of band B (the per-band rules of sw:4430-4450): the source
@@ -1170,21 +1388,65 @@ __device__ __forceinline__ void sweep_flush(SweepShared &S, int round, int count
   S.sums[c][type0 + q][level0 + dir * j] = acc;
 }
 
+// 1 / d of the adding method's denominators 1 - r r', in (0, 1] but for
+// roundings and meaningless inputs.
+__device__ __forceinline__ float sw_recip(float d) { return safe_size(d) ? recip_in_range(d) : 1.0f / d; }
+
+// Upward recurrence of vrtqdr (sw:3655-3680) across the layer of slot s.
+__device__ __forceinline__ void sw_up(const SwLevel &s, float &rup, float &rupd) {
+  const float z = sw_recip(1.0f - rupd * s.rt.y);
+  const float nrup = s.rt.x + s.rt.w * ((s.rt.z - s.dn.x) * rupd + s.dn.x * rup) * z;
+  rupd = s.rt.y + s.rt.w * s.rt.w * rupd * z;
+  rup = nrup;
+}
+
+// Level fluxes (sw:3703-3720); tdbt = dn.y, tdn = dn.z, rdnd = dn.w.
+__device__ __forceinline__ void sw_fluxes(const SwLevel &s, float rup, float rupd, float &fu, float &fd) {
+  const float z = sw_recip(1.0f - s.dn.w * rupd);
+  fu = (s.dn.y * rup + (s.dn.z - s.dn.y) * rupd) * z;
+  fd = s.dn.y + (s.dn.z - s.dn.y + s.dn.y * rup * s.dn.w) * z;
+}
+
+// Downward recurrence of vrtqdr (sw:3681-3702): the path's values at level
+// r + 1 from those at level r and layer r's optics.
+struct SwCarry {
+  float tdbt, tdn, rdnd;
+};
+
+__device__ __forceinline__ SwCarry sw_down(const SwCarry &c, const SwOptics &o, bool top) {
+  SwCarry n;
+  n.tdbt = c.tdbt * o.dbt;
+  if (top) {
+    n.tdn = o.rt.tra;
+    n.rdnd = o.rt.refd;
+  } else {
+    const float zreflect = sw_recip(1.0f - o.rt.refd * c.rdnd);
+    n.tdn = c.tdbt * o.rt.tra + o.rt.trad * ((c.tdn - c.tdbt) + c.tdbt * o.rt.ref * c.rdnd) * zreflect;
+    n.rdnd = o.rt.refd + o.rt.trad * o.rt.trad * c.rdnd * zreflect;
+  }
+  return n;
+}
+
 // Block = kSweepCols consecutive slots of the chunk; thread = (slot, g-point).
 // A slot past the day count repeats the block's first slot so that every
 // thread takes the same barriers; its results are not written.
 //
 // Work per g-point layer follows spcvmc (sw:6887-7041) statement by statement;
-// three kinds of operation are shared or skipped where the result is known
-// bit for bit: the quotient tau / mu and its Pade lookup, computed once for
-// the direct beam and reftra's exponent; divisions by a divisor that is
-// exactly 1; and, in a g-point layer without cloud, the cloudy
-// reflectance/transmittance inputs, whose only consumer is a reftra call the
-// reference skips (lrt = false).  The total-sky stack slot of such a layer is
-// not stored: the bottom-up pass re-forms it from the clear-sky slot with the
-// reference's mixing expression.
+// operations are shared or skipped where the result is known bit for bit: the
+// quotient tau / mu and its Pade lookup, computed once for the direct beam and
+// reftra's exponent; divisions by a divisor that is exactly 1; in a g-point
+// layer without cloud, the cloudy reflectance/transmittance, whose weight is
+// zero; and above a g-point's highest cloud the whole total-sky path, which
+// equals the clear-sky one.  Outside the FP64 mode the divisions themselves
+// are those of rrtmg_divide.cuh.
+// Bound by instruction issue, then by the stack's traffic.  Sweep of a
+// 425 x 425 x 50 call: 25.7 ms with IEEE divisions throughout and the total-sky
+// path followed from the top; 21.8 ms now (80 registers at 3 blocks per SM:
+// 24.9).  The tables are a __grid_constant__: the out-of-line forms take their
+// address, and a per-thread copy of them cost 14 ms.
 template <bool kFp64>
-__global__ void __launch_bounds__(kSweepThreads, kSwSweepMinBlocks) sw_sweep_kernel(Tables T, SwArgs a) {
+__global__ void __launch_bounds__(kSweepThreads, kSwSweepMinBlocks) sw_sweep_kernel(const __grid_constant__ Tables T,
+                                                                                        const SwArgs a) {
   extern __shared__ __align__(16) unsigned char smem_raw[];
   SweepShared &S = *reinterpret_cast<SweepShared *>(smem_raw);
   const int nday = *a.nday;
@@ -1201,12 +1463,17 @@ __global__ void __launch_bounds__(kSweepThreads, kSwSweepMinBlocks) sw_sweep_ker
   const float sflux_g = R.sflux[G];
   const int n = C.nlay;
   const float mu = C.mu;
+  const float y_mu = recip_in_range(mu);
   const int clear_only = a.icld == 0;
   int band = kSwBands - 1;
   while (G < kSwGofsDev[band]) --band;
   const int P = kPadOfsDev[band] + (G - kSwGofsDev[band]);  // record position of the g-point
-  const float *recs = sw_layrecs(a) + static_cast<size_t>(u) * n * kSwRec;
-  const float *crec = recs + kSwRecCloud + 4 * band;
+  // the block's layer records, addressed from one base by 32-bit byte offsets
+  const char *const base =
+      reinterpret_cast<const char *>(sw_layrecs(a) + static_cast<size_t>(u0) * n * kSwRec);
+  constexpr uint32_t kStep = kSwRec * sizeof(float);
+  const uint32_t column = static_cast<uint32_t>((u - u0) * n) * kStep;
+  const uint32_t off_tau = column + 4u * P, off_cld = column + 4u * (kSwRecCloud + 4 * band);
   const uint32_t *maskbase = a.mask + col + static_cast<size_t>(G >> 5) * a.ncol;
   const size_t mstride = static_cast<size_t>(kSwMaskWords) * a.ncol;
   const uint32_t bit = 1u << (G & 31);
@@ -1215,9 +1482,9 @@ __global__ void __launch_bounds__(kSweepThreads, kSwSweepMinBlocks) sw_sweep_ker
   SwLevel stc[kMaxLev], stt[kMaxLev];
   // per stack slot r, bit r & 31 of word r >> 5 (gathered in registers, 32
   // slots at a time, then kept in shared memory): the g-point layer is cloudy
-  // (its total-sky reftra results are stored), and the slot's total-sky
-  // values equal the clear-sky ones bit for bit (no total-sky slot is stored;
-  // the bottom-up pass reuses the clear-sky slot and reads no mask word)
+  // (its total-sky reftra results are stored), and the slot's total-sky values
+  // are the clear-sky ones (no cloud in this g-point so far: no total-sky slot
+  // is stored; the bottom-up pass reuses the clear-sky slot)
   uint32_t cloudy_bits = 0, same_word = 0;
 
   // ---- top-down pass: layer optics, direct beam, downward adding (sw:6887-7041)
@@ -1230,132 +1497,67 @@ __global__ void __launch_bounds__(kSweepThreads, kSwSweepMinBlocks) sw_sweep_ker
   ring0[0] = tdbt_nd * zincflx;
   ring0[kTypeStep] = tdbtc_nd * zincflx;
   int filled = 1, level0 = 0, round = 0;
-  // carry of the downward recurrence: level r values of each path
-  float c_tdbt = 1.0f, c_tdn = 1.0f, c_rdnd = 0.0f;
-  float t_tdbt = 1.0f, t_tdn = 1.0f, t_rdnd = 0.0f;
+  // the downward recurrence's values at level r; the total-sky ones count from
+  // the g-point's first cloud on (differ)
+  SwCarry cc{1.0f, 1.0f, 0.0f}, ct = cc;
+  bool differ = false;
   // layer values are loaded one layer ahead
-  const float *rl = recs + static_cast<size_t>(n - 1) * kSwRec;
-  float nx_tg = rl[P], nx_tr = rl[kSwRecTaur + P];
-  float4 nx_cld = *reinterpret_cast<const float4 *>(crec + static_cast<size_t>(n - 1) * kSwRec);
-  uint32_t nx_word = maskbase[static_cast<size_t>(n - 1) * mstride];
+  float nx_tg, nx_tr;
+  float4 nx_cld;
+  uint32_t nx_word;
+  auto load = [&](int l) {
+    const uint32_t step = static_cast<uint32_t>(l) * kStep;
+    nx_tg = *reinterpret_cast<const float *>(base + off_tau + step);
+    nx_tr = *reinterpret_cast<const float *>(base + off_tau + step + 4 * kSwRecTaur);
+    nx_cld = *reinterpret_cast<const float4 *>(base + off_cld + step);
+    nx_word = maskbase[static_cast<size_t>(l) * mstride];
+  };
+  load(n - 1);
   for (int r = 0; r < n; ++r) {
     const int l = n - 1 - r;
-    const uint32_t word = nx_word;
+    const bool cldb = !clear_only && (nx_word & bit) != 0u;
     const float tr = nx_tr, tg = nx_tg;
     const float4 cld = nx_cld;
-    if (l > 0) {
-      const float *q = recs + static_cast<size_t>(l - 1) * kSwRec;
-      nx_tg = q[P];
-      nx_tr = q[kSwRecTaur + P];
-      nx_cld = *reinterpret_cast<const float4 *>(crec + static_cast<size_t>(l - 1) * kSwRec);
-      nx_word = maskbase[static_cast<size_t>(l - 1) * mstride];
-    }
-    const bool cldb = !clear_only && (word & bit) != 0u;
-    const float cloud = cldb ? 1.0f : 0.0f;
-    const float clear = 1.0f - cloud;
-    // clear sky: gas + Rayleigh, no aerosol (sw:6923-6927)
-    const float ztau = (tr + tg) + 0.0f;
-    const float zom0 = tr + 0.0f * 1.0f;
-    const float zgr = zero_over(zom0);  // 0 * 1 * 0 / zom
-    const float zom = zom0 / ztau;
-    const float v_nd = ztau / mu;
-    const float dbtc_nd = exp_lookup(T, v_nd);
-    tdbtc_nd = tdbtc_nd * dbtc_nd;
-    const float zf = zgr * zgr;
-    const float zwf = zom * zf;
-    const float d_w = 1.0f - zwf;
-    const float ztauc = d_w * ztau;
-    const float zomcc = div_or_same(zom - zwf, d_w);
-    const float zgcc = div_or_same(zgr - zf, 1.0f - zf);
-    // ztauc is ztau exactly when d_w == 1
-    const float v_c = d_w == 1.0f ? v_nd : ztauc / mu;
-    const float dbtc = d_w == 1.0f ? dbtc_nd : exp_lookup(T, v_c);
-    const RT4 c = reftra<kFp64>(T, zgcc, mu, ztauc, zomcc, v_c, dbtc);
-    const float4 c_rt = make_float4(c.ref, c.refd, c.tra, c.trad);
-    stc[r].rt = c_rt;
-    stc[r].dn = make_float4(dbtc, c_tdbt, c_tdn, c_rdnd);
-    // the total-sky carry equals the clear-sky one bit for bit (first half of
-    // the test whether this slot's total-sky values need storing)
-    const bool carry_same =
-        same_bits(make_float4(0.0f, t_tdbt, t_tdn, t_rdnd), make_float4(0.0f, c_tdbt, c_tdn, c_rdnd));
-    // downward recurrence of vrtqdr (sw:3681-3702) for level r + 1
-    {
-      const float tdbt_next = c_tdbt * dbtc;
-      float tdn_next, rdnd_next;
-      if (r == 0) {
-        tdn_next = c.tra;
-        rdnd_next = c.refd;
-      } else {
-        const float zreflect = 1.0f / (1.0f - c.refd * c_rdnd);
-        tdn_next = c_tdbt * c.tra + c.trad * ((c_tdn - c_tdbt) + c_tdbt * c.ref * c_rdnd) * zreflect;
-        rdnd_next = c.refd + c.trad * c.trad * c_rdnd * zreflect;
-      }
-      c_tdbt = tdbt_next;
-      c_tdn = tdn_next;
-      c_rdnd = rdnd_next;
-    }
-    if (!clear_only) {
-      float ref, refd, tra, trad, dbt;
-      if (cldb) {
-        const float tcld = cld.x, wcld = cld.y, gcld = cld.z, taor = cld.w;
-        const float tauorig = ztau + taor;
-        const float dbtmo_nd = exp_lookup(T, tauorig / mu);
-        const float dbt_nd = clear * dbtc_nd + cloud * dbtmo_nd;
-        tdbt_nd = tdbt_nd * dbt_nd;
-        const float ztauo = ztauc + tcld;
-        float zomco = ztauc * zomcc + tcld * wcld;
-        const float zgco = (tcld * wcld * gcld + ztauc * zomcc * zgcc) / zomco;
-        zomco = zomco / ztauo;
-        const float v_o = ztauo / mu;
-        const float dbtmo = exp_lookup(T, v_o);
-        const RT4 o = reftra<kFp64>(T, zgco, mu, ztauo, zomco, v_o, dbtmo);
-        ref = clear * c.ref + cloud * o.ref;
-        refd = clear * c.refd + cloud * o.refd;
-        tra = clear * c.tra + cloud * o.tra;
-        trad = clear * c.trad + cloud * o.trad;
-        dbt = clear * dbtc + cloud * dbtmo;
-        stt[r].rt = make_float4(ref, refd, tra, trad);
-        cloudy_bits |= 1u << (r & 31);
-      } else {
-        // no cloud in this g-point layer: taor = tcld = 0, so tauorig and
-        // ztauo are ztau and ztauc plus zero, and the cloudy reftra is the
-        // reference's lrt = false constant set (0, 0, 1, 1)
-        const float tauorig = ztau + 0.0f;
-        const float dbtmo_nd = __float_as_uint(tauorig) == __float_as_uint(ztau) ? dbtc_nd
-                                                                                 : exp_lookup(T, tauorig / mu);
-        const float dbt_nd = clear * dbtc_nd + cloud * dbtmo_nd;
-        tdbt_nd = tdbt_nd * dbt_nd;
-        const float ztauo = ztauc + 0.0f;
-        const float dbtmo = __float_as_uint(ztauo) == __float_as_uint(ztauc) ? dbtc : exp_lookup(T, ztauo / mu);
-        ref = clear * c.ref + cloud * 0.0f;
-        refd = clear * c.refd + cloud * 0.0f;
-        tra = clear * c.tra + cloud * 1.0f;
-        trad = clear * c.trad + cloud * 1.0f;
-        dbt = clear * dbtc + cloud * dbtmo;
-      }
-      const float4 t_dn = make_float4(dbt, t_tdbt, t_tdn, t_rdnd);
-      if (!cldb && carry_same && __float_as_uint(dbt) == __float_as_uint(dbtc) &&
-          same_bits(make_float4(ref, refd, tra, trad), c_rt)) {
-        same_word |= 1u << (r & 31);
-      } else {
-        stt[r].dn = t_dn;
-      }
-      const float tdbt_next = t_tdbt * dbt;
-      float tdn_next, rdnd_next;
-      if (r == 0) {
-        tdn_next = tra;
-        rdnd_next = refd;
-      } else {
-        const float zreflect = 1.0f / (1.0f - refd * t_rdnd);
-        tdn_next = t_tdbt * tra + trad * ((t_tdn - t_tdbt) + t_tdbt * ref * t_rdnd) * zreflect;
-        rdnd_next = refd + trad * trad * t_rdnd * zreflect;
-      }
-      t_tdbt = tdbt_next;
-      t_tdn = tdn_next;
-      t_rdnd = rdnd_next;
+    if (l > 0) load(l - 1);
+    SwClear c;
+    SwOptics oc;
+    if constexpr (kFp64) {
+      oc = sw_clear_any<true>(T, tg, tr, mu, c);
     } else {
+      bool ok;
+      oc = sw_clear_safe(T, tg, tr, mu, y_mu, c, ok);
+      if (!ok) oc = sw_clear_slow(T, tg, tr, mu, c);
+    }
+    stc[r].rt = make_float4(oc.rt.ref, oc.rt.refd, oc.rt.tra, oc.rt.trad);
+    stc[r].dn = make_float4(oc.dbt, cc.tdbt, cc.tdn, cc.rdnd);
+    if (cldb && !differ) {
+      differ = true;
+      ct = cc;
       tdbt_nd = tdbtc_nd;
     }
+    if (differ) {
+      SwOptics ot;
+      if (cldb) {
+        if constexpr (kFp64) {
+          ot = sw_cloudy_any<true>(T, c, oc, cld, mu);
+        } else {
+          bool ok = c.zgcc == 0.0f && safe_size(c.ztau);
+          ot = sw_cloudy_safe(T, c, cld, mu, y_mu, ok);
+          if (!ok) ot = sw_cloudy_slow(T, c, oc, cld, mu);
+        }
+        stt[r].rt = make_float4(ot.rt.ref, ot.rt.refd, ot.rt.tra, ot.rt.trad);
+        cloudy_bits |= 1u << (r & 31);
+      } else {
+        ot = oc;  // the reference's mix clear * c + cloud * (0, 0, 1, 1) with clear = 1, cloud = 0
+      }
+      stt[r].dn = make_float4(ot.dbt, ct.tdbt, ct.tdn, ct.rdnd);
+      tdbt_nd = tdbt_nd * ot.dbt_nd;
+      ct = sw_down(ct, ot, r == 0);
+    } else {
+      same_word |= 1u << (r & 31);
+    }
+    tdbtc_nd = tdbtc_nd * oc.dbt_nd;
+    cc = sw_down(cc, oc, r == 0);
     if ((r & 31) == 31 || r == n - 1) {
       S.slotbits[0][r >> 5][threadIdx.x] = cloudy_bits;
       S.slotbits[1][r >> 5][threadIdx.x] = same_word;
@@ -1364,7 +1566,7 @@ __global__ void __launch_bounds__(kSweepThreads, kSwSweepMinBlocks) sw_sweep_ker
     }
     {
       float *q = ring0 + (round & 1) * kBufStep + filled * (2 * kTypeStep);
-      q[0] = tdbt_nd * zincflx;
+      q[0] = (differ ? tdbt_nd : tdbtc_nd) * zincflx;
       q[kTypeStep] = tdbtc_nd * zincflx;
     }
     if (++filled == kDownLevels || r == n - 1) {
@@ -1374,6 +1576,7 @@ __global__ void __launch_bounds__(kSweepThreads, kSwSweepMinBlocks) sw_sweep_ker
       filled = 0;
     }
   }
+  if (!differ) ct = cc;
 
   // ---- bottom-up pass: upward adding and level fluxes (vrtqdr, sw:3655-3720)
   // surface albedos of this g-point's band: direct (albp) and diffuse (albd);
@@ -1389,11 +1592,11 @@ __global__ void __launch_bounds__(kSweepThreads, kSwSweepMinBlocks) sw_sweep_ker
   float rupt = albp, rupdt = albd;
   level0 = n;
   // surface level n: albedo reflection, no transmission; the recurrence's level-n values
-  SwLevel c = {make_float4(albp, albd, 0.0f, 0.0f), make_float4(0.0f, c_tdbt, c_tdn, c_rdnd)};
-  SwLevel t = {make_float4(albp, albd, 0.0f, 0.0f), make_float4(0.0f, t_tdbt, t_tdn, t_rdnd)};
+  SwLevel c = {make_float4(albp, albd, 0.0f, 0.0f), make_float4(0.0f, cc.tdbt, cc.tdn, cc.rdnd)};
+  SwLevel t = {make_float4(albp, albd, 0.0f, 0.0f), make_float4(0.0f, ct.tdbt, ct.tdn, ct.rdnd)};
   if (clear_only) t = c;
   // stack slot j (layer n - 1 - j) of both paths; a layer without cloud in
-  // this g-point has the total-sky mix clear * c + cloud * (0, 0, 1, 1)
+  // this g-point has the clear-sky layer's optics in both
   auto load_slot = [&](int j, SwLevel &lc, SwLevel &lt) {
     lc = stc[j];
     if (clear_only || ((S.slotbits[1][j >> 5][threadIdx.x] >> (j & 31)) & 1u) != 0u) {
@@ -1401,40 +1604,22 @@ __global__ void __launch_bounds__(kSweepThreads, kSwSweepMinBlocks) sw_sweep_ker
       return;
     }
     lt.dn = stt[j].dn;
-    if (((S.slotbits[0][j >> 5][threadIdx.x] >> (j & 31)) & 1u) != 0u) {
-      lt.rt = stt[j].rt;
-    } else {
-      const float clear = 1.0f, cloud = 0.0f;
-      lt.rt = make_float4(clear * lc.rt.x + cloud * 0.0f, clear * lc.rt.y + cloud * 0.0f,
-                          clear * lc.rt.z + cloud * 1.0f, clear * lc.rt.w + cloud * 1.0f);
-    }
+    lt.rt = ((S.slotbits[0][j >> 5][threadIdx.x] >> (j & 31)) & 1u) != 0u ? stt[j].rt : lc.rt;
   };
   for (int k = n; k >= 0; --k) {
     SwLevel nc = c, nt = t;
     if (k > 0) load_slot(k - 1, nc, nt);
     if (k < n) {
-      const float zrc = 1.0f / (1.0f - rupdc * c.rt.y);
-      const float nrupc = c.rt.x + c.rt.w * ((c.rt.z - c.dn.x) * rupdc + c.dn.x * rupc) * zrc;
-      const float nrupdc = c.rt.y + c.rt.w * c.rt.w * rupdc * zrc;
-      rupc = nrupc;
-      rupdc = nrupdc;
-      if (!clear_only) {
-        const float zrt = 1.0f / (1.0f - rupdt * t.rt.y);
-        const float nrupt = t.rt.x + t.rt.w * ((t.rt.z - t.dn.x) * rupdt + t.dn.x * rupt) * zrt;
-        const float nrupdt = t.rt.y + t.rt.w * t.rt.w * rupdt * zrt;
-        rupt = nrupt;
-        rupdt = nrupdt;
-      }
+      sw_up(c, rupc, rupdc);
+      if (!clear_only) sw_up(t, rupt, rupdt);
     }
-    // level fluxes; tdbt = dn.y, tdn = dn.z, rdnd = dn.w
-    const float zrefc = 1.0f / (1.0f - c.dn.w * rupdc);
-    const float fuc = (c.dn.y * rupc + (c.dn.z - c.dn.y) * rupdc) * zrefc;
-    const float fdc = c.dn.y + (c.dn.z - c.dn.y + c.dn.y * rupc * c.dn.w) * zrefc;
-    float fut = fuc, fdt = fdc;
+    float fuc, fdc, fut, fdt;
+    sw_fluxes(c, rupc, rupdc, fuc, fdc);
     if (!clear_only) {
-      const float zreft = 1.0f / (1.0f - t.dn.w * rupdt);
-      fut = (t.dn.y * rupt + (t.dn.z - t.dn.y) * rupdt) * zreft;
-      fdt = t.dn.y + (t.dn.z - t.dn.y + t.dn.y * rupt * t.dn.w) * zreft;
+      sw_fluxes(t, rupt, rupdt, fut, fdt);
+    } else {
+      fut = fuc;
+      fdt = fdc;
     }
     {
       float *q = ring0 + (round & 1) * kBufStep + filled * (4 * kTypeStep);
