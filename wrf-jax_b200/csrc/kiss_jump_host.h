@@ -13,6 +13,7 @@
 #pragma once
 
 #include <cstdint>
+#include <cstring>
 
 namespace rrtmg {
 
@@ -101,6 +102,15 @@ inline void kiss_jumps(uint64_t skip, int nlay, int nsub, KissJump *out) {
     J.steps = static_cast<uint32_t>(k);
     out[g] = J;
     cur = compose(stride, cur);
+  }
+}
+
+// Words of the jumps with the subcolumns fastest, as the kernel reads them.
+inline void transpose_jumps(const KissJump *jumps, int nsub, uint32_t *words) {
+  for (int g = 0; g < nsub; ++g) {
+    uint32_t w[kJumpWords];
+    std::memcpy(w, &jumps[g], sizeof(w));
+    for (int i = 0; i < kJumpWords; ++i) words[static_cast<size_t>(i) * nsub + g] = w[i];
   }
 }
 

@@ -46,7 +46,7 @@ struct rrtmg_ctx {
   std::mutex mutex;
   std::string last_error;
   // KISS jump tables keyed by (nlay, nsub, skip); never freed before destroy
-  std::map<std::tuple<int, int, int>, KissJump *> jumps;
+  std::map<std::tuple<int, int, int>, uint32_t *> jumps;
   // stream-ordered per-call scratch; keeps its memory between calls
   cudaMemPool_t pool = nullptr;
   // launch schedule (rrtmg_set_schedule)
@@ -353,9 +353,10 @@ bool fill_tables(rrtmg_ctx *ctx, std::string &err) {
   T.lw_preflog = dev_ptr<float>(ctx, "lw.preflog");
   T.lw_tref = dev_ptr<float>(ctx, "lw.tref");
   T.chi_mls = dev_ptr<float>(ctx, "lw.chi_mls");
-  T.totplnk = dev_ptr<float>(ctx, "lw.totplnk");
-  T.absice3 = dev_ptr<float>(ctx, "lw.absice3");
-  T.absliq1 = dev_ptr<float>(ctx, "lw.absliq1");
+  // rows of 16 bands, aligned for 16-byte loads
+  const bool have_lw_rows = (add_padded(ctx, "lw.totplnk", kLwBands, kLwBands, &T.totplnk) > 0) &
+                            (add_padded(ctx, "lw.absice3", kLwBands, kLwBands, &T.absice3) > 0) &
+                            (add_padded(ctx, "lw.absliq1", kLwBands, kLwBands, &T.absliq1) > 0);
   int n = 0;
   T.lw_pade_tau = dev_ptr<float>(ctx, "lw.pade_tau_tbl", &n);
   T.lw_ntbl = n - 1;
@@ -406,7 +407,7 @@ bool fill_tables(rrtmg_ctx *ctx, std::string &err) {
   const double *lp = host_ptr<double>(ctx, "glibc.logf_ln2_poly");
   T.expf_tab = dev_ptr<unsigned long long>(ctx, "glibc.expf_tab");
   const double *ep = host_ptr<double>(ctx, "glibc.expf_invln2n_poly");
-  if (!T.lw_preflog || !T.chi_mls || !T.totplnk || !T.absice3 || !T.absliq1 || !T.lw_pade_tau ||
+  if (!T.lw_preflog || !T.chi_mls || !have_lw_rows || !T.lw_pade_tau ||
       !T.sw_preflog || !T.extliq1 || !T.extice3 || !T.sw_pade_exp || !T.retab || !T.pprof || !T.tprof ||
       !T.logf_tab || !lp || !T.expf_tab || !ep || !host_ptr<float>(ctx, "o3sum")) {
     err = "table blob is missing required tables";
@@ -435,7 +436,7 @@ bool fill_tables(rrtmg_ctx *ctx, std::string &err) {
   return true;
 }
 
-rrtmg_status get_jumps(rrtmg_ctx *ctx, int nlay, int nsub, int skip, const KissJump **out) {
+rrtmg_status get_jumps(rrtmg_ctx *ctx, int nlay, int nsub, int skip, const uint32_t **out) {
   std::lock_guard<std::mutex> lk(ctx->mutex);
   auto key = std::make_tuple(nlay, nsub, skip);
   auto it = ctx->jumps.find(key);
@@ -446,13 +447,15 @@ rrtmg_status get_jumps(rrtmg_ctx *ctx, int nlay, int nsub, int skip, const KissJ
   // offsets skip + g * nlay
   std::vector<KissJump> host(nsub);
   kiss_jumps(static_cast<uint64_t>(skip), nlay, nsub, host.data());
-  KissJump *dev = nullptr;
+  std::vector<uint32_t> words(static_cast<size_t>(kJumpWords) * nsub);
+  transpose_jumps(host.data(), nsub, words.data());
+  uint32_t *dev = nullptr;
   cudaError_t e = cudaMalloc(&dev, sizeof(KissJump) * nsub);
   if (e != cudaSuccess) {
     ctx->last_error = std::string("cudaMalloc(jump table): ") + cudaGetErrorString(e);
     return RRTMG_CUDA;
   }
-  e = cudaMemcpy(dev, host.data(), sizeof(KissJump) * nsub, cudaMemcpyHostToDevice);
+  e = cudaMemcpy(dev, words.data(), sizeof(KissJump) * nsub, cudaMemcpyHostToDevice);
   if (e != cudaSuccess) {
     cudaFree(dev);
     ctx->last_error = std::string("cudaMemcpy(jump table): ") + cudaGetErrorString(e);
@@ -730,7 +733,7 @@ static rrtmg_status lwrad_impl(rrtmg_ctx *ctx, const rrtmg_config *cfg, const rr
   cudaError_t e = guard.status();
   if (e != cudaSuccess) return cuda_fail(ctx, e, "cudaSetDevice");
   const int ncol = cfg->nx * cfg->ny;
-  const KissJump *jumps = nullptr;
+  const uint32_t *jumps = nullptr;
   st = get_jumps(ctx, nlay, kLwGpts, 150, &jumps);
   if (st != RRTMG_OK) return st;
   uint32_t *mask = nullptr;
@@ -839,7 +842,7 @@ static rrtmg_status swrad_impl(rrtmg_ctx *ctx, const rrtmg_config *cfg, const rr
   cudaError_t e = guard.status();
   if (e != cudaSuccess) return cuda_fail(ctx, e, "cudaSetDevice");
   const int ncol = cfg->nx * cfg->ny;
-  const KissJump *jumps = nullptr;
+  const uint32_t *jumps = nullptr;
   st = get_jumps(ctx, nlay, kSwGpts, 1, &jumps);
   if (st != RRTMG_OK) return st;
   uint32_t *mask = nullptr;
@@ -862,6 +865,7 @@ static rrtmg_status swrad_impl(rrtmg_ctx *ctx, const rrtmg_config *cfg, const rr
   m.enabled = icld >= 1;
   m.live = live;
   m.p3d = in->p3d; m.cldfra = in->cldfra3d; m.jumps = jumps; m.mask = mask;
+  m.coszr = in->coszr;
   e = launch_mcica(m, stream);
   timing_mark(ctx, 1, tslot, stream);
   if (e != cudaSuccess) {
@@ -986,7 +990,7 @@ size_t rrtmg_lw_workspace_bytes(rrtmg_ctx *ctx, const rrtmg_config *cfg) {
   if (check_config(ctx, cfg) != RRTMG_OK) return 0;
   const int nlay = rrtmg_lw_nlayers(cfg->p_top, cfg->nk);
   if (nlay > kMaxLay || nlay - cfg->nk > kMaxBuf || nlay < cfg->nk) return 0;
-  const KissJump *jumps = nullptr;  // built here, ahead of the first call
+  const uint32_t *jumps = nullptr;  // built here, ahead of the first call
   {
     DeviceGuard guard(ctx->device);
     if (guard.status() != cudaSuccess || get_jumps(ctx, nlay, kLwGpts, 150, &jumps) != RRTMG_OK) return 0;
@@ -996,7 +1000,7 @@ size_t rrtmg_lw_workspace_bytes(rrtmg_ctx *ctx, const rrtmg_config *cfg) {
 
 size_t rrtmg_sw_workspace_bytes(rrtmg_ctx *ctx, const rrtmg_config *cfg) {
   if (check_config(ctx, cfg) != RRTMG_OK || cfg->nk + 1 > kMaxLay) return 0;
-  const KissJump *jumps = nullptr;
+  const uint32_t *jumps = nullptr;
   {
     DeviceGuard guard(ctx->device);
     if (guard.status() != cudaSuccess || get_jumps(ctx, cfg->nk + 1, kSwGpts, 1, &jumps) != RRTMG_OK) return 0;
@@ -1041,12 +1045,12 @@ constexpr int kStaticMaxDevices = 64;
 constexpr int kStaticMinLay = 4;  // nlay >= nk >= 4
 
 __device__ __align__(256) uint32_t g_static_mask[kStaticMaskWords];
-__device__ __align__(256) KissJump g_static_jumps[kMaxLay + 1][kLwGpts];
+__device__ __align__(256) uint32_t g_static_jumps[kMaxLay + 1][kJumpWords * kLwGpts];
 
 struct StaticScratch {
   bool ready = false;
   uint32_t *mask = nullptr;
-  KissJump *jumps = nullptr;  // slot nlay at jumps + nlay * kLwGpts
+  uint32_t *jumps = nullptr;  // slot nlay at jumps + nlay * kJumpWords * kLwGpts
 };
 
 std::mutex g_static_mutex;
@@ -1060,11 +1064,15 @@ cudaError_t static_scratch_setup(StaticScratch &s) {
   s.mask = static_cast<uint32_t *>(p);
   e = cudaGetSymbolAddress(&p, g_static_jumps);
   if (e != cudaSuccess) return e;
-  s.jumps = static_cast<KissJump *>(p);
-  std::vector<KissJump> host(static_cast<size_t>(kMaxLay + 1) * kLwGpts, KissJump{});
-  for (int nlay = kStaticMinLay; nlay <= kMaxLay; ++nlay)
-    kiss_jumps(150ull, nlay, kLwGpts, host.data() + static_cast<size_t>(nlay) * kLwGpts);
-  e = cudaMemcpy(s.jumps, host.data(), host.size() * sizeof(KissJump), cudaMemcpyHostToDevice);
+  s.jumps = static_cast<uint32_t *>(p);
+  constexpr size_t slot = static_cast<size_t>(kJumpWords) * kLwGpts;
+  std::vector<uint32_t> host((kMaxLay + 1) * slot, 0u);
+  std::vector<KissJump> one(kLwGpts);
+  for (int nlay = kStaticMinLay; nlay <= kMaxLay; ++nlay) {
+    kiss_jumps(150ull, nlay, kLwGpts, one.data());
+    transpose_jumps(one.data(), kLwGpts, host.data() + nlay * slot);
+  }
+  e = cudaMemcpy(s.jumps, host.data(), host.size() * sizeof(uint32_t), cudaMemcpyHostToDevice);
   if (e != cudaSuccess) return e;
   s.ready = true;
   return cudaSuccess;
@@ -1108,7 +1116,7 @@ extern "C" rrtmg_status rrtmg_lwrad_static_scratch(rrtmg_ctx *ctx, const rrtmg_c
   if (e != cudaSuccess) return cuda_fail(ctx, e, "cudaSetDevice");
 
   uint32_t *mask = nullptr;
-  KissJump *jumps = nullptr;
+  uint32_t *jumps = nullptr;
   {
     std::lock_guard<std::mutex> lk(g_static_mutex);
     StaticScratch &s = g_static_scratch[ctx->device];
@@ -1117,7 +1125,7 @@ extern "C" rrtmg_status rrtmg_lwrad_static_scratch(rrtmg_ctx *ctx, const rrtmg_c
       if (e != cudaSuccess) return cuda_fail(ctx, e, "static McICA scratch set-up");
     }
     mask = s.mask;
-    jumps = s.jumps + static_cast<size_t>(nlay) * kLwGpts;
+    jumps = s.jumps + static_cast<size_t>(nlay) * kJumpWords * kLwGpts;
   }
 
   McicaArgs m{};

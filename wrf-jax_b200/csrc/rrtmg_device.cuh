@@ -199,7 +199,7 @@ __device__ __forceinline__ float glibc_expf(const Tables &T, float x) {
 // KISS generator step (module_ra_rrtmg_common.py:976-997).
 struct Kiss {
   uint32_t s1, s2, s3, s4;
-  __device__ __forceinline__ float next() {
+  __device__ __forceinline__ uint32_t step() {
     s1 = 69069u * s1 + 1327217885u;
     uint32_t x = s2;
     x ^= x << 13;
@@ -208,8 +208,10 @@ struct Kiss {
     s2 = x;
     s3 = 18000u * (s3 & 65535u) + (s3 >> 16);
     s4 = 30903u * (s4 & 65535u) + (s4 >> 16);
-    const uint32_t kiss = s1 + s2 + (s3 << 16) + s4;
-    const float k = static_cast<float>(static_cast<int32_t>(kiss));
+    return s1 + s2 + (s3 << 16) + s4;
+  }
+  __device__ __forceinline__ float next() {
+    const float k = static_cast<float>(static_cast<int32_t>(step()));
     return k * 2.328306e-10f + 0.5f;
   }
 };
@@ -225,28 +227,41 @@ struct KissJump {
   uint32_t pad;
 };
 
-__device__ __forceinline__ uint32_t mwc_step(uint32_t v, uint32_t a) { return a * (v & 65535u) + (v >> 16); }
+constexpr int kJumpWords = sizeof(KissJump) / sizeof(uint32_t);
 
-__device__ __forceinline__ uint32_t mwc_jump(uint32_t v, uint32_t a, uint32_t pw, uint32_t k) {
+// The multiply-with-carry jump of generator A: twice * pw mod A * 2^16 - 1.  The
+// remainder by Barrett's method (CRYPTO '86): the quotient's estimate from the
+// modulus's reciprocal scaled by 2^64 is at most one too small.
+template <uint32_t A>
+__device__ __forceinline__ uint32_t mwc_jump(uint32_t v, uint32_t pw, uint32_t k) {
+  constexpr uint64_t m = static_cast<uint64_t>(A) * 65536ull - 1ull, inverse = ~0ull / m;
+  auto step = [](uint32_t x) { return A * (x & 65535u) + (x >> 16); };
   if (k == 0) return v;
-  const uint32_t once = mwc_step(v, a);
+  const uint32_t once = step(v);
   if (k == 1) return once;
-  const uint32_t twice = mwc_step(once, a);
-  const uint64_t m = static_cast<uint64_t>(a) * 65536ull - 1ull;
+  const uint32_t twice = step(once);
   if (twice == static_cast<uint32_t>(m)) return twice;
-  return static_cast<uint32_t>((static_cast<uint64_t>(twice) * pw) % m);
+  const uint64_t x = static_cast<uint64_t>(twice) * pw;
+  uint64_t r = x - __umul64hi(x, inverse) * m;
+  if (r >= m) r -= m;
+  return static_cast<uint32_t>(r);
 }
 
-__device__ __forceinline__ Kiss kiss_jump(Kiss s, const KissJump &J) {
+// Jump of subcolumn g by the transposed table `words`: word w of KissJump for
+// every subcolumn at words + w * nsub, so that a warp's loads are contiguous.
+__device__ __forceinline__ Kiss kiss_jump(Kiss s, const uint32_t *words, int nsub, int g) {
+  const uint32_t *J = words + g;
+  auto word = [&](int w) { return __ldg(J + w * nsub); };
   Kiss o;
-  o.s1 = J.lcg_mul * s.s1 + J.lcg_add;
+  o.s1 = word(0) * s.s1 + word(1);
   uint32_t acc = 0;
 #pragma unroll
   for (int b = 0; b < 32; ++b)
-    if ((s.s2 >> b) & 1u) acc ^= J.xs[b];
+    if ((s.s2 >> b) & 1u) acc ^= word(2 + b);
   o.s2 = acc;
-  o.s3 = mwc_jump(s.s3, 18000u, J.mwc3_pow, J.steps);
-  o.s4 = mwc_jump(s.s4, 30903u, J.mwc4_pow, J.steps);
+  const uint32_t k = word(36);
+  o.s3 = mwc_jump<18000u>(s.s3, word(34), k);
+  o.s4 = mwc_jump<30903u>(s.s4, word(35), k);
   return o;
 }
 

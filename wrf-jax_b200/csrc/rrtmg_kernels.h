@@ -16,9 +16,10 @@ __device__ __forceinline__ bool dead_column(const int *live, int col) { return l
 struct McicaArgs {
   int ncol, ny, nk, nlay, nsub, words, enabled;
   const float *p3d, *cldfra;
-  const KissJump *jumps;  // one per subcolumn
+  const uint32_t *jumps;  // KissJump words of every subcolumn, transposed (kiss_jump)
   uint32_t *mask;         // (nlay, words, ncol)
   const int *live;        // null, or a device count of leading columns to process
+  const float *coszr;     // null, or the columns whose value is not positive are skipped
 };
 
 // Per-column inputs shared by LW and SW (WRF layout, device pointers).
