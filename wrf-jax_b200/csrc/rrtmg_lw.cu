@@ -158,57 +158,92 @@ __global__ void __launch_bounds__(128) lw_colprep_kernel(Tables T, LwArgs a) {
 constexpr int kLwLayerMinBlocks = 6;
 constexpr int kLwGasMinBlocks = 5;
 constexpr int kLwSweepMinBlocks = 4;
+
+// A warp's 32 layer records written Q 16-byte pieces at a time: `row` is the
+// lane's row of the stage (rows of kRow pieces, an odd number, so that no banks
+// conflict), its first Q pieces go to `at` floats into the lane's record.
+// record: the lane's layer record, or -1 where it has none.
+template <int Q, int kRow>
+__device__ __forceinline__ void store_records(float *recs, int record, const float4 *stage, int at) {
+  const int lane = threadIdx.x & 31;
+  __syncwarp();
+#pragma unroll
+  for (int i = 0; i < Q; ++i) {
+    const int e = i * 32 + lane, r = e / Q, q = e - r * Q;
+    const int rec = __shfl_sync(0xffffffffu, record, r);
+    if (rec >= 0) reinterpret_cast<float4 *>(recs + static_cast<size_t>(rec) * kLwRec + at)[q] = stage[r * kRow + q];
+  }
+  __syncwarp();
+}
+
 __global__ void __launch_bounds__(128, kLwLayerMinBlocks) lw_layer_kernel(Tables T, LwArgs a) {
+  constexpr int kRow = 7;
+  __shared__ float4 stages[4][32 * kRow];
   const long long idx = static_cast<long long>(blockIdx.x) * blockDim.x + threadIdx.x;
   const int l = static_cast<int>(idx / a.chunk_count);
   const int lc = static_cast<int>(idx - static_cast<long long>(l) * a.chunk_count);
-  if (l >= a.nlay) return;
   const int col = a.chunk_first + lc;
-  if (dead_column(a.live, col)) return;
-  const Col &C = col_records(a)[lc].C;
-  const Layer L = make_layer(T, a, C, l);
-  float *gas = gas_fields(a) + static_cast<size_t>(l) * a.chunk_capacity + lc;
-  const size_t fstride = static_cast<size_t>(a.nlay) * a.chunk_capacity;
-  int f = 0;
+  const bool live = l < a.nlay && !dead_column(a.live, col);
+  if (!__any_sync(0xffffffffu, live)) return;  // whole warps
+  float4 *stage = stages[threadIdx.x >> 5];
+  float4 *row = stage + (threadIdx.x & 31) * kRow;
+  float *recs = layer_records(a);
+  const int record = live ? lc * a.nlay + l : -1;
+  const ColRec &R = col_records(a)[live ? lc : 0];
+  Layer L{};
+  uint32_t mask[kLwMaskWords] = {0};
+  bool cloudy = false;
+  if (live) {
+    L = make_layer(T, a, R.C, l);
+    float *gas = gas_fields(a) + static_cast<size_t>(l) * a.chunk_capacity + lc;
+    const size_t fstride = static_cast<size_t>(a.nlay) * a.chunk_capacity;
+    int f = 0;
 #define RRTMG_LW_PUT(name) gas[static_cast<size_t>(f++) * fstride] = L.name;
 #define RRTMG_LW_PUTI(name) gas[static_cast<size_t>(f++) * fstride] = __int_as_float(L.name);
-  RRTMG_LW_GAS_FLOATS(RRTMG_LW_PUT)
-  RRTMG_LW_GAS_INTS(RRTMG_LW_PUTI)
+    RRTMG_LW_GAS_FLOATS(RRTMG_LW_PUT)
+    RRTMG_LW_GAS_INTS(RRTMG_LW_PUTI)
 #undef RRTMG_LW_PUT
 #undef RRTMG_LW_PUTI
-  uint32_t mask[kLwMaskWords];
-  const bool cloudy = load_mask(a, l, col, mask);
-  float4 *rec = reinterpret_cast<float4 *>(layer_records(a) + (static_cast<size_t>(lc) * a.nlay + l) * kLwRec);
-  const int iceflag = C.iceflg;
-  const float *secdiff = col_records(a)[lc].secdiff;
-#pragma unroll 1
-  for (int b4 = 0; b4 < kLwBands; b4 += 4) {
-    float efcl[4];
+    cloudy = load_mask(a, l, col, mask);
+  }
+  // four bands at a time: Planck terms and the cloud's optical depth and
+  // absorptance along the diffusivity angle (lw:5562-5565).  The latter are the
+  // same for all g-points of a band, so the binary64 exponential is evaluated
+  // here, once per band and not once per g-point and direction.  Four bands per
+  // table load and staged stores: 64 x 64 x 44 87 -> 63 us, LW optics of
+  // 425 x 425 x 50 14.2 -> 13.2 ms.
+  const int iceflag = a.iceflg;
+  float4 efcl[kLwBands / 4];
 #pragma unroll
-    for (int e = 0; e < 4; ++e) {
-      const int b = b4 + e;
-      const float blay = planck(T, L.indlay, L.tlayfrac, b);
-      const float dplankup = planck(T, L.indlev1, L.tlev1frac, b) - blay;
-      const float dplankdn = planck(T, L.indlev0, L.tlev0frac, b) - blay;
-      // a cloudy g-point's optical depth and absorptance (lw:5562-5565): the
-      // same for all g-points of the band, so its binary64 exponential is
-      // evaluated here, once per band and not once per g-point and direction
-      float odcld = 0.0f;
-      efcl[e] = 0.0f;
+  for (int b4 = 0; b4 < kLwBands / 4; ++b4) {
+    efcl[b4] = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+    if (live) {
+      const float4 blay = planck4(T, L.indlay, L.tlayfrac, b4);
+      const float4 up = planck4(T, L.indlev1, L.tlev1frac, b4), dn = planck4(T, L.indlev0, L.tlev0frac, b4);
+      float4 od = efcl[b4];
       if (cloudy) {
         bool active = false;
-        const float tauc = cloud_tau(T, L, b, iceflag, active);
-        odcld = secdiff[b] * (active ? tauc : 0.0f);
-        efcl[e] = (1.0f - glibc_expf(T, -odcld)) * 1.0f;
+        const float4 tauc = cloud_tau4(T, L, b4, iceflag, active);
+        const float *sd = R.secdiff + 4 * b4;
+        const float4 t = active ? tauc : od;
+        od = make_float4(sd[0] * t.x, sd[1] * t.y, sd[2] * t.z, sd[3] * t.w);
+        auto absorptance = [&](float x) { return (1.0f - glibc_expf(T, -x)) * 1.0f; };
+        efcl[b4] = make_float4(absorptance(od.x), absorptance(od.y), absorptance(od.z), absorptance(od.w));
       }
-      rec[kLwRecBand / 4 + b] = make_float4(blay, dplankup, dplankdn, odcld);
+      row[0] = make_float4(blay.x, up.x - blay.x, dn.x - blay.x, od.x);
+      row[1] = make_float4(blay.y, up.y - blay.y, dn.y - blay.y, od.y);
+      row[2] = make_float4(blay.z, up.z - blay.z, dn.z - blay.z, od.z);
+      row[3] = make_float4(blay.w, up.w - blay.w, dn.w - blay.w, od.w);
     }
-    rec[kLwRecEfcl / 4 + b4 / 4] = make_float4(efcl[0], efcl[1], efcl[2], efcl[3]);
+    store_records<4, kRow>(recs, record, stage, kLwRecBand + 16 * b4);
   }
-  static_assert(kLwMaskWords == 5, "mask words of a record");
-  rec[kLwRecMask / 4] = make_float4(__uint_as_float(mask[0]), __uint_as_float(mask[1]), __uint_as_float(mask[2]),
-                                    __uint_as_float(mask[3]));
-  rec[kLwRecMask / 4 + 1] = make_float4(__uint_as_float(mask[4]), 0.0f, 0.0f, 0.0f);
+  static_assert(kLwMaskWords == 5 && kLwRecMask == kLwRecEfcl + kLwBands, "absorptances, then mask words");
+#pragma unroll
+  for (int b4 = 0; b4 < kLwBands / 4; ++b4) row[b4] = efcl[b4];
+  row[4] = make_float4(__uint_as_float(mask[0]), __uint_as_float(mask[1]), __uint_as_float(mask[2]),
+                       __uint_as_float(mask[3]));
+  row[5] = make_float4(__uint_as_float(mask[4]), 0.0f, 0.0f, 0.0f);
+  store_records<6, kRow>(recs, record, stage, kLwRecEfcl);
 }
 
 // 16-byte pieces of a warp's stage: optical depths, then fractions, of 32 rows of up to 5

@@ -361,6 +361,37 @@ __device__ __forceinline__ float cloud_tau(const Tables &T, const Layer &L, int 
   return (ciwp * abscoice + clwp * abscoliq) + cswp * abscosno;
 }
 
+// cloud_tau and planck of bands 4 b4 .. 4 b4 + 3 (table rows of 16 bands).
+__device__ __forceinline__ float4 cloud_tau4(const Tables &T, const Layer &L, int b4, int iceflag, bool &active) {
+  const float4 zero = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+  const float ciwp = L.ciwp, clwp = L.clwp, cswp = L.cswp;
+  const float cwp = (ciwp + clwp) + cswp;
+  active = cwp >= 1.0e-20f;
+  // rows `index - 1` and `index` of a size with spacing 3, as cldprmc does
+  auto ice = [&](float size) {
+    const float factor = (size - 2.0f) / 3.0f;
+    int index = static_cast<int>(factor);
+    if (index == 46) index = 45;
+    return interp4(row4<16>(T.absice3, jrow(index - 1, 46), b4), row4<16>(T.absice3, jrow(index, 46), b4),
+                   factor - static_cast<float>(index));
+  };
+  const float4 abscoice = (ciwp + cswp) == 0.0f ? zero : ice(L.rei);
+  const float4 abscosno = iceflag == 5 && cswp > 0.0f ? ice(L.res) : zero;
+  float4 abscoliq = zero;
+  if (clwp != 0.0f) {
+    int il = static_cast<int>(L.rel - 1.5f);
+    if (il == 0) il = 1;
+    if (il == 58) il = 57;
+    const float fl = (L.rel - 1.5f) - static_cast<float>(il);
+    abscoliq = interp4(row4<16>(T.absliq1, jrow(il - 1, 58), b4), row4<16>(T.absliq1, jrow(il, 58), b4), fl);
+  }
+  return add4(add4(mul4(ciwp, abscoice), mul4(clwp, abscoliq)), mul4(cswp, abscosno));
+}
+
+__device__ __forceinline__ float4 planck4(const Tables &T, int ind, float frac, int b4) {
+  return interp4(row4<16>(T.totplnk, ind - 1, b4), row4<16>(T.totplnk, ind, b4), frac);
+}
+
 __device__ __forceinline__ int pade_index(const Tables &T, float od) {
   const float tblind = od / (T.lw_bpade + od);
   const float pos = static_cast<float>(T.lw_ntbl) * tblind + 0.5f;
