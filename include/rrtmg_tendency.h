@@ -44,6 +44,14 @@ rrtmg_status rrtmg_radiation_tendency(const rrtmg_tendency_bounds *bounds, const
                                       const float *mut, int couple, float *rthraten, float *rt_tendf,
                                       void *stream);
 
+/* The fused chain with the updated tendency in another array: rt_tendf becomes
+ * rt_tendf_in plus the coupled heating over the a2a region and rt_tendf_in
+ * elsewhere.  Both are required and must not overlap; rthraten may be NULL. */
+rrtmg_status rrtmg_radiation_tendency_into(const rrtmg_tendency_bounds *bounds, const float *rthratenlw,
+                                           const float *rthratensw, const float *c1, const float *c2,
+                                           const float *mut, int couple, float *rthraten, const float *rt_tendf_in,
+                                           float *rt_tendf, void *stream);
+
 /* phy_ra_ten alone (module_physics_addtendc.py:542): rt_tendf += rthraten over
  * the a2a region, in place. */
 rrtmg_status rrtmg_phy_ra_ten(const rrtmg_tendency_bounds *bounds, float *rt_tendf, const float *rthraten,

@@ -70,12 +70,13 @@ def radiation_tendency(rthratenlw, rthratensw, c1, c2, mut, rt_tendf, config_fla
                    or tuple(d["mut"].shape) != (shape[0], shape[2])):
         raise ValueError("c1/c2 must have kme-kms+1 values and mut (ime-ims+1, jme-jms+1)")
     r = torch.empty(shape, dtype=torch.float32, device=d["lw"].device)
-    t = d["t"].clone()
+    t = torch.empty_like(d["t"])
     s = stream if stream is not None else torch.cuda.current_stream().cuda_stream
     lib = _capi.load()
-    _check(lib.rrtmg_radiation_tendency(ctypes.byref(tb), d["lw"].data_ptr(), d["sw"].data_ptr(),
-                                        d["c1"].data_ptr(), d["c2"].data_ptr(), d["mut"].data_ptr(), int(couple),
-                                        r.data_ptr(), t.data_ptr(), ctypes.c_void_p(s)), "rrtmg_radiation_tendency")
+    _check(lib.rrtmg_radiation_tendency_into(ctypes.byref(tb), d["lw"].data_ptr(), d["sw"].data_ptr(),
+                                             d["c1"].data_ptr(), d["c2"].data_ptr(), d["mut"].data_ptr(), int(couple),
+                                             r.data_ptr(), d["t"].data_ptr(), t.data_ptr(), ctypes.c_void_p(s)),
+           "rrtmg_radiation_tendency")
     if host:
         torch.cuda.current_stream().synchronize()
         return r.cpu().numpy(), t.cpu().numpy()
