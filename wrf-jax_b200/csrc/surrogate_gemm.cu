@@ -3,18 +3,22 @@
 //
 //   C[M x N] = A[M x K] * B[N x K]^T      (A, B row-major BF16, FP32 accumulate)
 //
-// One CTA of 128 threads owns a 128 x BN output tile (BN = 256 when N allows,
-// else 128).  Its accumulator lives in tensor memory (128 lanes x BN FP32
+// One CTA of 256 threads owns a 128 x BN output tile (BN = 128, or 256 on
+// request).  Its accumulator lives in tensor memory (128 lanes x BN FP32
 // columns).  K advances in blocks of 64: all threads copy the A and B blocks
-// into shared memory (cp.async, 3-4 stages in flight) in the 128-byte swizzled
+// into shared memory (cp.async, three stages) in the 128-byte swizzled
 // K-major layout, and one thread issues four tcgen05.mma (K = 16 each)
 // whose completion is committed to the stage's mbarrier before the stage is
-// refilled.  The epilogue reads the accumulator back with tcgen05.ld (warp w
-// owns lanes 32w..32w+31, i.e. tile rows) and applies one of:
+// refilled.  With BN = 128 two CTAs share an SM, one's epilogue under the
+// other's loads and MMAs.  The epilogue reads the accumulator back with
+// tcgen05.ld (warp w owns tile rows 32 (w mod 4) .. and column half w / 4), 32
+// columns at a time, and passes them through a shared stage of the warp's own
+// so that every global access is a run of whole sectors along a row:
 //   kEpiF32    C (+ bias) as FP32, one slab per K split (split-K partials)
 //   kEpiGelu   Z = acc + bias (FP32), H = GELU(Z) as BF16 row-major and
 //              transposed (the transposed copy feeds the weight gradient)
 //   kEpiDgelu  dZ = acc * GELU'(aux) as BF16 row-major and transposed
+// Bound by the epilogue's traffic at the surrogate's shapes (K = 512).
 //
 // Shared-memory layout of an operand block (R rows x 64 K, BF16): the
 // canonical K-major SWIZZLE_128B layout, row r at r * 128 bytes with its eight
@@ -23,6 +27,8 @@
 #include <cuda_bf16.h>
 #include <cuda_runtime.h>
 #include <stdint.h>
+
+#include <atomic>
 
 #include "surrogate_kernels.h"
 #include "umma_common.cuh"
@@ -38,11 +44,11 @@ using umma::smem_u32;
 using umma::swz;
 
 constexpr int kBM = 128, kBK = 64;
-constexpr int kThreads = 128;
+constexpr int kThreads = 256;
 
 template <int BN>
 struct Tile {
-  static constexpr int kStages = BN == 256 ? 3 : 4;
+  static constexpr int kStages = 3;
   static constexpr int kBytesA = kBM * kBK * 2;
   static constexpr int kBytesB = BN * kBK * 2;
   static constexpr int kStageBytes = kBytesA + kBytesB;
@@ -51,30 +57,44 @@ struct Tile {
   static constexpr uint32_t kIdesc = umma::idesc_bf16(kBM, BN);
 };
 
+// A warp's stage of the epilogue, over the pipeline's shared memory: 32 rows x
+// 32 FP32 values, and the BF16 results by rows and by columns.  Row pitches are
+// odd numbers of 16 bytes, so that neither side of the transposition conflicts.
+constexpr int kEpiCols = 32;
+struct EpiStage {
+  float z[32][36];
+  __nv_bfloat16 h[32][40];
+  __nv_bfloat16 ht[kEpiCols][40];
+};
+static_assert(sizeof(EpiStage) * (kThreads / 32) <= 3 * Tile<128>::kStageBytes, "stages of the epilogue");
+
 __device__ unsigned g_gemm_error;
 
 __device__ __forceinline__ void cp_async16(void *smem, const void *gmem) {
   asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(smem_u32(smem)), "l"(gmem) : "memory");
 }
 
-// Tile (m-tile = blockIdx.y, n-tile = blockIdx.x, K split = blockIdx.z): the
-// n-tiles of one m-tile are neighbouring CTAs, so they share the A rows in L2.
+// One tile: m-tile `my`, n-tile `nx`, K split `z` of problem g (its K blocks
+// are dealt to the splits as evenly as they go).  The n-tiles of one m-tile are
+// neighbouring CTAs, so they share the A rows in L2.
 // K blocks stream through kStages shared-memory stages: the copies of block
 // kb + kStages - 1 are in flight while the tensor cores work on block kb.
 template <int BN>
-__global__ void __launch_bounds__(kThreads, 1) umma_gemm_kernel(GemmArgs g) {
+__device__ __forceinline__ void gemm_tile(const GemmArgs &g, int nx, int my, int z) {
   using TL = Tile<BN>;
   constexpr int S = TL::kStages;
   extern __shared__ __align__(1024) uint8_t smem[];
   __shared__ __align__(8) uint64_t mbar[S];
   __shared__ uint32_t tmem_sh;
   __shared__ int fail_sh;
+  __shared__ __align__(16) float bias_sh[BN];
 
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
-  const int n0 = blockIdx.x * BN, m0 = blockIdx.y * kBM;
-  const int kper = g.K / g.ksplit;
-  const int kbeg = blockIdx.z * kper;
-  const int nkb = kper / kBK;
+  const int n0 = nx * BN, m0 = my * kBM;
+  const int blocks = g.K / kBK;
+  const int kb0 = static_cast<int>(static_cast<long long>(blocks) * z / g.ksplit);
+  const int kbeg = kb0 * kBK;
+  const int nkb = static_cast<int>(static_cast<long long>(blocks) * (z + 1) / g.ksplit) - kb0;
 
   if (warp == 0) {
     asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(&tmem_sh)),
@@ -87,6 +107,7 @@ __global__ void __launch_bounds__(kThreads, 1) umma_gemm_kernel(GemmArgs g) {
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     fail_sh = 0;
   }
+  for (int j = tid; j < BN; j += kThreads) bias_sh[j] = g.bias && z == 0 ? g.bias[n0 + j] : 0.0f;
   asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
   __syncthreads();
   asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
@@ -181,65 +202,96 @@ __global__ void __launch_bounds__(kThreads, 1) umma_gemm_kernel(GemmArgs g) {
   if (failed) {
     if (tid == 0) atomicOr(&g_gemm_error, 1u);
   } else {
-    const int row = m0 + warp * 32 + lane;
+    // rows r0 .. r0 + 31 of the output, columns n0 + c .. of the warp's half
+    const int r0 = m0 + (warp & 3) * 32;
+    const uint32_t trow = tmem + (static_cast<uint32_t>((warp & 3) * 32) << 16);
+    EpiStage &st = reinterpret_cast<EpiStage *>(tiles)[warp];
+    const int zr = lane >> 3, zc = (lane & 7) * 4;  // a row's 32 FP32 values: 8 lanes
+    const int hr = lane >> 2, hc = (lane & 3) * 8;  // 32 BF16 values: 4 lanes
+    const bool ht_rows = (g.ldht % 8) == 0 && (reinterpret_cast<uintptr_t>(g.Ht) & 15u) == 0;
+    auto put_rows = [&](float *dst, size_t ld) {  // the FP32 stage to rows of dst
+      __syncwarp();
+#pragma unroll
+      for (int i = 0; i < 8; ++i)
+        *reinterpret_cast<float4 *>(dst + static_cast<size_t>(r0 + 4 * i + zr) * ld + zc) =
+            *reinterpret_cast<const float4 *>(&st.z[4 * i + zr][zc]);
+    };
 #pragma unroll 1
-    for (int c = 0; c < BN; c += 16) {
-      uint32_t v[16];
-      asm volatile(
-          "tcgen05.ld.sync.aligned.32x32b.x16.b32 {%0, %1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, "
-          "%14, %15}, [%16];"
-          : "=r"(v[0]), "=r"(v[1]), "=r"(v[2]), "=r"(v[3]), "=r"(v[4]), "=r"(v[5]), "=r"(v[6]), "=r"(v[7]),
-            "=r"(v[8]), "=r"(v[9]), "=r"(v[10]), "=r"(v[11]), "=r"(v[12]), "=r"(v[13]), "=r"(v[14]), "=r"(v[15])
-          : "r"(tmem + (static_cast<uint32_t>(warp * 32) << 16) + static_cast<uint32_t>(c)));
-      asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
-      // each thread holds 16 consecutive columns of its row: row-major outputs
-      // are written as 16-byte vectors, transposed ones as 2-byte elements
-      // that are contiguous across the warp's 32 rows
-      float acc[16];
-#pragma unroll
-      for (int j = 0; j < 16; ++j) acc[j] = __uint_as_float(v[j]);
+    for (int c = (warp >> 2) * (BN / 2); c < (warp >> 2) * (BN / 2) + BN / 2; c += kEpiCols) {
       const int nc = n0 + c;
-      if (g.epi == kEpiF32) {
-        if (g.bias && blockIdx.z == 0) {
+      __syncwarp();  // the stage's previous readers are done
+      if (g.epi == kEpiDgelu) {
 #pragma unroll
-          for (int j = 0; j < 16; ++j) acc[j] += g.bias[nc + j];
-        }
-        float4 *dst = reinterpret_cast<float4 *>(g.C + static_cast<size_t>(blockIdx.z) * g.split_stride +
-                                                 static_cast<size_t>(row) * g.ldc + nc);
+        for (int i = 0; i < 8; ++i)
+          *reinterpret_cast<float4 *>(&st.z[4 * i + zr][zc]) = *reinterpret_cast<const float4 *>(
+              g.aux + static_cast<size_t>(r0 + 4 * i + zr) * g.ldaux + nc + zc);
+        __syncwarp();
+      }
 #pragma unroll
-        for (int q = 0; q < 4; ++q) dst[q] = make_float4(acc[4 * q], acc[4 * q + 1], acc[4 * q + 2], acc[4 * q + 3]);
-      } else {
+      for (int half = 0; half < 2; ++half) {
+        uint32_t v[16];
+        umma::tmem_ld16(trow + static_cast<uint32_t>(c + 16 * half), v);
+        umma::tmem_ld_wait();
+        float acc[16];
+#pragma unroll
+        for (int j = 0; j < 16; ++j) acc[j] = __uint_as_float(v[j]);
+        float4 *zs = reinterpret_cast<float4 *>(&st.z[lane][16 * half]);
         __align__(16) __nv_bfloat16 h[16];
-        if (g.epi == kEpiGelu) {
-#pragma unroll
-          for (int j = 0; j < 16; ++j) acc[j] += g.bias ? g.bias[nc + j] : 0.0f;
-          if (g.Z) {
-            float4 *dz = reinterpret_cast<float4 *>(g.Z + static_cast<size_t>(row) * g.ldz + nc);
-#pragma unroll
-            for (int q = 0; q < 4; ++q) dz[q] = make_float4(acc[4 * q], acc[4 * q + 1], acc[4 * q + 2], acc[4 * q + 3]);
-          }
-#pragma unroll
-          for (int j = 0; j < 16; ++j) h[j] = __float2bfloat16_rn(gelu(acc[j]));
-        } else {  // kEpiDgelu
-          const float4 *za = reinterpret_cast<const float4 *>(g.aux + static_cast<size_t>(row) * g.ldaux + nc);
+        if (g.epi == kEpiDgelu) {
 #pragma unroll
           for (int q = 0; q < 4; ++q) {
-            const float4 z = za[q];
-            h[4 * q + 0] = __float2bfloat16_rn(acc[4 * q + 0] * gelu_grad(z.x));
-            h[4 * q + 1] = __float2bfloat16_rn(acc[4 * q + 1] * gelu_grad(z.y));
-            h[4 * q + 2] = __float2bfloat16_rn(acc[4 * q + 2] * gelu_grad(z.z));
-            h[4 * q + 3] = __float2bfloat16_rn(acc[4 * q + 3] * gelu_grad(z.w));
+            const float4 zz = zs[q];
+            h[4 * q + 0] = __float2bfloat16_rn(acc[4 * q + 0] * gelu_grad(zz.x));
+            h[4 * q + 1] = __float2bfloat16_rn(acc[4 * q + 1] * gelu_grad(zz.y));
+            h[4 * q + 2] = __float2bfloat16_rn(acc[4 * q + 2] * gelu_grad(zz.z));
+            h[4 * q + 3] = __float2bfloat16_rn(acc[4 * q + 3] * gelu_grad(zz.w));
           }
+        } else {
+          // (a split's partial sums take no bias: bias_sh is zero there)
+          const float4 *b4 = reinterpret_cast<const float4 *>(bias_sh + c + 16 * half);
+#pragma unroll
+          for (int q = 0; q < 4; ++q) {
+            const float4 b = b4[q];
+            if (g.bias) {
+              acc[4 * q] += b.x;
+              acc[4 * q + 1] += b.y;
+              acc[4 * q + 2] += b.z;
+              acc[4 * q + 3] += b.w;
+            }
+            zs[q] = make_float4(acc[4 * q], acc[4 * q + 1], acc[4 * q + 2], acc[4 * q + 3]);
+          }
+          if (g.epi == kEpiF32) continue;
+#pragma unroll
+          for (int j = 0; j < 16; ++j) h[j] = __float2bfloat16_rn(gelu(acc[j]));
         }
-        if (g.H) {
-          uint4 *dh = reinterpret_cast<uint4 *>(g.H + static_cast<size_t>(row) * g.ldh + nc);
-          dh[0] = *reinterpret_cast<const uint4 *>(&h[0]);
-          dh[1] = *reinterpret_cast<const uint4 *>(&h[8]);
-        }
+        uint4 *hs = reinterpret_cast<uint4 *>(&st.h[lane][16 * half]);
+        hs[0] = *reinterpret_cast<const uint4 *>(&h[0]);
+        hs[1] = *reinterpret_cast<const uint4 *>(&h[8]);
         if (g.Ht) {
 #pragma unroll
-          for (int j = 0; j < 16; ++j) g.Ht[static_cast<size_t>(nc + j) * g.ldht + row] = h[j];
+          for (int j = 0; j < 16; ++j) st.ht[16 * half + j][lane] = h[j];
         }
+      }
+      if (g.epi == kEpiF32) {
+        put_rows(g.C + static_cast<size_t>(z) * g.split_stride + nc, g.ldc);
+        continue;
+      }
+      if (g.epi == kEpiGelu && g.Z) put_rows(g.Z + nc, g.ldz);
+      __syncwarp();
+      if (g.H) {
+#pragma unroll
+        for (int i = 0; i < 4; ++i)
+          *reinterpret_cast<uint4 *>(g.H + static_cast<size_t>(r0 + 8 * i + hr) * g.ldh + nc + hc) =
+              *reinterpret_cast<const uint4 *>(&st.h[8 * i + hr][hc]);
+      }
+      if (g.Ht && ht_rows) {
+#pragma unroll
+        for (int i = 0; i < 4; ++i)
+          *reinterpret_cast<uint4 *>(g.Ht + static_cast<size_t>(nc + 8 * i + hr) * g.ldht + r0 + hc) =
+              *reinterpret_cast<const uint4 *>(&st.ht[8 * i + hr][hc]);
+      } else if (g.Ht) {
+        for (int j = 0; j < kEpiCols; ++j)
+          g.Ht[static_cast<size_t>(nc + j) * g.ldht + r0 + lane] = st.ht[j][lane];
       }
     }
   }
@@ -252,14 +304,27 @@ __global__ void __launch_bounds__(kThreads, 1) umma_gemm_kernel(GemmArgs g) {
 }
 
 template <int BN>
+__global__ void __launch_bounds__(kThreads, BN == 128 ? 2 : 1) umma_gemm_kernel(const __grid_constant__ GemmArgs g) {
+  gemm_tile<BN>(g, blockIdx.x, blockIdx.y, blockIdx.z);
+}
+
+// Opts a kernel in to its shared memory, once per device (a bit of `done` each).
+template <class Kernel>
+cudaError_t raise_smem(Kernel kernel, int bytes, std::atomic<unsigned long long> &done) {
+  int dev = 0;
+  cudaError_t e = cudaGetDevice(&dev);
+  if (e != cudaSuccess) return e;
+  if (dev < 64 && ((done.load() >> dev) & 1ull)) return cudaSuccess;
+  e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes);
+  if (e == cudaSuccess && dev < 64) done.fetch_or(1ull << dev);
+  return e;
+}
+
+template <int BN>
 cudaError_t launch_tile(const GemmArgs &g, cudaStream_t stream) {
-  static bool configured = false;
-  if (!configured) {
-    cudaError_t e = cudaFuncSetAttribute(umma_gemm_kernel<BN>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                         Tile<BN>::kSmemBytes);
-    if (e != cudaSuccess) return e;
-    configured = true;
-  }
+  static std::atomic<unsigned long long> configured{0};
+  cudaError_t e = raise_smem(umma_gemm_kernel<BN>, Tile<BN>::kSmemBytes, configured);
+  if (e != cudaSuccess) return e;
   dim3 grid(g.N / BN, g.M / kBM, g.ksplit);
   umma_gemm_kernel<BN><<<grid, kThreads, Tile<BN>::kSmemBytes, stream>>>(g);
   return cudaGetLastError();
@@ -268,12 +333,13 @@ cudaError_t launch_tile(const GemmArgs &g, cudaStream_t stream) {
 }  // namespace
 
 namespace {
-int g_tile_choice = 0;  // 0 automatic, else 128 or 256
+// 0 automatic (128: two CTAs per SM), else 128 or 256
+int g_tile_choice = 0;
 }  // namespace
 
 void set_gemm_tile(int bn) { g_tile_choice = bn; }
 
-bool gemm_wide(int n) { return n % 256 == 0 && g_tile_choice != 128; }
+bool gemm_wide(int n) { return n % 256 == 0 && g_tile_choice == 256; }
 
 int gemm_stages(int n) { return gemm_wide(n) ? Tile<256>::kStages : Tile<128>::kStages; }
 
