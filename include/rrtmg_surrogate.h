@@ -121,6 +121,34 @@ typedef struct {
 } rrtmg_sur_adam_args;
 rrtmg_status rrtmg_sur_adam(const rrtmg_sur_adam_args *args, void *stream);
 
+/* One training step of the four-layer network (512 -> 512 -> 512 -> 512 -> 128)
+ * in one call: batch gather, forward pass, loss gradient (the batch's weighted
+ * squared error is added to loss[0]), backward pass, split-K weight gradients
+ * of all layers in one launch, bias gradients, and Adam on every weight and
+ * bias.  Layer i has rows[i] outputs and 512 inputs; gradients are left in gw /
+ * gb, the BF16 copies wb (row-major) and wbt (transposed) are rewritten.  batch
+ * is a multiple of 128.  The buffers are the caller's: Xb, H, dZ [batch][512]
+ * and dY [batch][128] BF16, their transposes Xbt, Ht, dZt [512][batch] and dYt
+ * [128][batch], Z [batch][512], Tb and Y [batch][128] FP32, and part of
+ * rrtmg_sur_train_part_floats(batch) floats; all 16-byte aligned. */
+typedef struct {
+    const void *X; int ldx;              /* normalized inputs (BF16), 512 columns */
+    const float *T; int ldt;             /* normalized targets, 128 columns */
+    const int *idx; int batch;           /* rows of the batch */
+    const float *weights;                /* loss weight of each output */
+    float loss_scale;
+    float lr, beta1, beta2, eps, bc1, bc2, weight_decay;
+    float *w[4], *mw[4], *vw[4], *gw[4], *b[4], *mb[4], *vb[4], *gb[4];
+    void *wb[4], *wbt[4];
+    void *Xb, *Xbt; float *Tb;
+    float *Z[3]; void *H[3], *Ht[3];
+    float *Y; void *dY, *dYt;
+    void *dZ[3], *dZt[3];
+    float *part, *loss;
+} rrtmg_sur_train_args;
+size_t rrtmg_sur_train_part_floats(int batch);
+rrtmg_status rrtmg_sur_train_step(const rrtmg_sur_train_args *args, void *stream);
+
 /* Network outputs Y[ncol][ldy] (normalized) to WRF fields: rthratenlw/sw
  * (nx, nk, ny) = hr / 86400 / pi3d (a multiplication by 1/86400 and a fast
  * division), glw, lwupb, swdnb, swupb (nx, ny); SW is

@@ -94,6 +94,15 @@ class SurAdamArgs(ctypes.Structure):
                 ("wb", _F), ("ldwb", _I), ("wbt", _F), ("ldwbt", _I)]
 
 
+class SurTrainArgs(ctypes.Structure):
+    _fields_ = [("X", _F), ("ldx", _I), ("T", _F), ("ldt", _I), ("idx", _F), ("batch", _I), ("weights", _F),
+                ("loss_scale", _FL), ("lr", _FL), ("beta1", _FL), ("beta2", _FL), ("eps", _FL), ("bc1", _FL),
+                ("bc2", _FL), ("weight_decay", _FL)] + \
+        [(n, _F * 4) for n in ("w", "mw", "vw", "gw", "b", "mb", "vb", "gb", "wb", "wbt")] + \
+        [("Xb", _F), ("Xbt", _F), ("Tb", _F), ("Z", _F * 3), ("H", _F * 3), ("Ht", _F * 3), ("Y", _F), ("dY", _F),
+         ("dYt", _F), ("dZ", _F * 3), ("dZt", _F * 3), ("part", _F), ("loss", _F)]
+
+
 class SurDecodeArgs(ctypes.Structure):
     _fields_ = [("ncol", _I), ("nk", _I), ("ny", _I), ("Y", _F), ("ldy", _I), ("out_mean", _F), ("out_std", _F),
                 ("coszr", _F), ("pi3d", _F), ("p8w", _F), ("energy_tol", _FL)] + \
@@ -154,7 +163,8 @@ FFI_EXPORTS = ("rrtmg_ffi_lwrad", "rrtmg_ffi_swrad", "rrtmg_ffi_set_table_blob",
 SURROGATE_EXPORTS = ("rrtmg_gemm_bf16", "rrtmg_gemm_error", "rrtmg_gemm_set_tile", "rrtmg_gemm_set_wait_ns",
                      "rrtmg_gemm_test_withhold_commit", "rrtmg_sur_features", "rrtmg_sur_targets",
                      "rrtmg_sur_column_stats", "rrtmg_sur_normalize", "rrtmg_sur_gather", "rrtmg_sur_loss_grad",
-                     "rrtmg_sur_row_sum", "rrtmg_sur_reduce_splits", "rrtmg_sur_adam", "rrtmg_sur_decode",
+                     "rrtmg_sur_row_sum", "rrtmg_sur_reduce_splits", "rrtmg_sur_adam", "rrtmg_sur_train_step",
+                     "rrtmg_sur_train_part_floats", "rrtmg_sur_decode",
                      "rrtmg_sur_compact", "rrtmg_sur_move_columns", "rrtmg_sur_timestamp",
                      "rrtmg_sur_pack_weights", "rrtmg_sur_mlp", "rrtmg_sur_move_fields")
 PROLOGUE_EXPORTS = ("rrtmg_radconst", "rrtmg_prologue_scalars_from_calendar", "rrtmg_set_ozone_climatology",
@@ -221,6 +231,7 @@ def load(path: str | os.PathLike | None = None) -> ctypes.CDLL:
         "rrtmg_sur_row_sum": [P, I, I, I, P, V],
         "rrtmg_sur_reduce_splits": [P, I, SZ, P, V],
         "rrtmg_sur_adam": [ctypes.POINTER(SurAdamArgs), V],
+        "rrtmg_sur_train_step": [ctypes.POINTER(SurTrainArgs), V],
         "rrtmg_sur_decode": [ctypes.POINTER(SurDecodeArgs), V],
         "rrtmg_sur_compact": [P, I, P, P, V],
         "rrtmg_sur_move_columns": [P, P, I, I, I, P, P, I, I, I, V],
@@ -251,6 +262,8 @@ def load(path: str | os.PathLike | None = None) -> ctypes.CDLL:
         fn = getattr(lib, name)
         fn.restype = ctypes.c_int
         fn.argtypes = argtypes
+    lib.rrtmg_sur_train_part_floats.restype = SZ
+    lib.rrtmg_sur_train_part_floats.argtypes = [I]
     lib.rrtmg_lw_nlayers.restype = ctypes.c_int
     lib.rrtmg_lw_nlayers.argtypes = [ctypes.c_double, ctypes.c_int]
     lib.rrtmg_last_error.restype = ctypes.c_char_p

@@ -162,6 +162,139 @@ extern "C" rrtmg_status rrtmg_sur_adam(const rrtmg_sur_adam_args *a, void *strea
   return cuda_status(launch_sur_adam(*a, as_stream(stream)));
 }
 
+// ---------------------------------------------------------------------------
+// training step
+// ---------------------------------------------------------------------------
+namespace {
+
+constexpr int kTrainLayers = 4, kTrainWidth = 512, kTrainOut = 128;
+
+int train_rows(int layer) { return layer == 3 ? kTrainOut : kTrainWidth; }
+
+// K splits of the weight gradients: 26 tiles of 128 x 256 in all, so 5 splits
+// give each SM one tile, but a split keeps at least four 64-row blocks so that
+// its pipeline fills.
+int train_splits(int batch) {
+  const int blocks = batch / 64;
+  return blocks / 4 < 1 ? 1 : (blocks / 4 > 5 ? 5 : blocks / 4);
+}
+
+}  // namespace
+
+extern "C" size_t rrtmg_sur_train_part_floats(int batch) {
+  if (batch <= 0 || batch % 128) return 0;
+  return static_cast<size_t>(train_splits(batch)) * kTrainWidth * (3 * kTrainWidth + kTrainOut);
+}
+
+extern "C" rrtmg_status rrtmg_sur_train_step(const rrtmg_sur_train_args *a, void *stream) {
+  if (!a || a->batch <= 0 || a->batch % 128 || a->ldx != kTrainWidth || a->ldt != kTrainOut) return RRTMG_BAD_ARG;
+  const void *need[] = {a->Xb, a->Xbt, a->Tb, a->Y, a->dY, a->dYt, a->part};
+  for (const void *p : need)
+    if (!p || !aligned16(p)) return RRTMG_BAD_ARG;
+  if (!a->X || !a->T || !a->idx || !a->weights || !a->loss) return RRTMG_BAD_ARG;
+  for (int i = 0; i < kTrainLayers; ++i) {
+    const void *per[] = {a->w[i], a->mw[i], a->vw[i], a->gw[i], a->wb[i], a->wbt[i]};
+    for (const void *p : per)
+      if (!p || !aligned16(p)) return RRTMG_BAD_ARG;
+    if (!a->b[i] || !a->mb[i] || !a->vb[i] || !a->gb[i]) return RRTMG_BAD_ARG;
+  }
+  for (int i = 0; i < 3; ++i) {
+    const void *per[] = {a->Z[i], a->H[i], a->Ht[i], a->dZ[i], a->dZt[i]};
+    for (const void *p : per)
+      if (!p || !aligned16(p)) return RRTMG_BAD_ARG;
+  }
+  cudaStream_t s = as_stream(stream);
+  const int B = a->batch;
+  auto bf = [](const void *p) { return static_cast<const __nv_bfloat16 *>(p); };
+  auto bfo = [](void *p) { return static_cast<__nv_bfloat16 *>(p); };
+  cudaError_t e = launch_sur_gather(bf(a->X), a->ldx, a->T, a->ldt, a->idx, B, bfo(a->Xb), bfo(a->Xbt), B, a->Tb, s);
+  auto gemm = [&](const void *A, int lda, const void *W, int ldb, int M, int N, int K) {
+    GemmArgs g{};
+    g.A = bf(A);
+    g.lda = lda;
+    g.B = bf(W);
+    g.ldb = ldb;
+    g.M = M;
+    g.N = N;
+    g.K = K;
+    g.ksplit = 1;
+    g.wait_ns = g_wait_ns.load();
+    return g;
+  };
+  // forward
+  const void *in = a->Xb;
+  for (int i = 0; i < 3 && e == cudaSuccess; ++i) {
+    GemmArgs g = gemm(in, kTrainWidth, a->wb[i], kTrainWidth, B, kTrainWidth, kTrainWidth);
+    g.epi = kEpiGelu;
+    g.bias = a->b[i];
+    g.Z = a->Z[i];
+    g.ldz = kTrainWidth;
+    g.H = bfo(a->H[i]);
+    g.ldh = kTrainWidth;
+    g.Ht = bfo(a->Ht[i]);
+    g.ldht = B;
+    e = launch_umma_gemm(g, s);
+    in = a->H[i];
+  }
+  if (e == cudaSuccess) {
+    GemmArgs g = gemm(in, kTrainWidth, a->wb[3], kTrainWidth, B, kTrainOut, kTrainWidth);
+    g.epi = kEpiF32;
+    g.bias = a->b[3];
+    g.C = a->Y;
+    g.ldc = kTrainOut;
+    e = launch_umma_gemm(g, s);
+  }
+  if (e == cudaSuccess)
+    e = launch_sur_loss_grad(a->Y, a->Tb, a->weights, B, kTrainOut, a->loss_scale, bfo(a->dY), bfo(a->dYt), B, a->loss,
+                             s);
+  // backward: d(pre-activation) of layers 2, 1, 0
+  for (int i = 3; i > 0 && e == cudaSuccess; --i) {
+    GemmArgs g = gemm(i == 3 ? a->dY : a->dZ[i], train_rows(i), a->wbt[i], train_rows(i), B, kTrainWidth, train_rows(i));
+    g.epi = kEpiDgelu;
+    g.aux = a->Z[i - 1];
+    g.ldaux = kTrainWidth;
+    g.H = bfo(a->dZ[i - 1]);
+    g.ldh = kTrainWidth;
+    g.Ht = bfo(a->dZt[i - 1]);
+    g.ldht = B;
+    e = launch_umma_gemm(g, s);
+  }
+  if (e != cudaSuccess) return cuda_status(e);
+  // weight gradients d(pre-activation)^T x inputs^T, then the update
+  const int splits = train_splits(B);
+  GemmArgs group[kTrainLayers];
+  SurUpdateArgs u{};
+  u.layers = kTrainLayers;
+  u.splits = splits;
+  u.batch = B;
+  u.lr = a->lr; u.beta1 = a->beta1; u.beta2 = a->beta2; u.eps = a->eps;
+  u.bc1 = a->bc1; u.bc2 = a->bc2; u.weight_decay = a->weight_decay;
+  float *part = a->part;
+  for (int i = 0; i < kTrainLayers; ++i) {
+    const int rows = train_rows(i);
+    const size_t slab = static_cast<size_t>(rows) * kTrainWidth;
+    GemmArgs g = gemm(i == 3 ? a->dYt : a->dZt[i], B, i == 0 ? a->Xbt : a->Ht[i - 1], B, rows, kTrainWidth, B);
+    g.epi = kEpiF32;
+    g.ksplit = splits;
+    g.C = part;
+    g.ldc = kTrainWidth;
+    g.split_stride = slab;
+    group[i] = g;
+    u.rows[i] = rows;
+    u.cols[i] = kTrainWidth;
+    u.gt[i] = g.A;
+    u.part[i] = part;
+    u.w[i] = a->w[i]; u.mw[i] = a->mw[i]; u.vw[i] = a->vw[i]; u.gw[i] = a->gw[i];
+    u.b[i] = a->b[i]; u.mb[i] = a->mb[i]; u.vb[i] = a->vb[i]; u.gb[i] = a->gb[i];
+    u.wb[i] = bfo(a->wb[i]);
+    u.wbt[i] = bfo(a->wbt[i]);
+    part += splits * slab;
+  }
+  e = launch_umma_gemm_group(group, kTrainLayers, s);
+  if (e == cudaSuccess) e = launch_sur_update(u, s);
+  return cuda_status(e);
+}
+
 extern "C" rrtmg_status rrtmg_sur_decode(const rrtmg_sur_decode_args *a, void *stream) {
   if (!a || a->ncol < 0 || a->nk <= 0 || a->ny <= 0 || !a->Y || a->ldy < 2 * a->nk + 6 || 2 * a->nk + 6 > 128 ||
       !a->out_mean ||

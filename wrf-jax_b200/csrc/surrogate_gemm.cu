@@ -308,6 +308,21 @@ __global__ void __launch_bounds__(kThreads, BN == 128 ? 2 : 1) umma_gemm_kernel(
   gemm_tile<BN>(g, blockIdx.x, blockIdx.y, blockIdx.z);
 }
 
+// Several problems in one launch (their K split and tile shape are common): the
+// weight gradients of a training step, each too small to fill the GPU alone.
+struct GemmGroup {
+  GemmArgs g[kGemmGroup];
+  int first[kGemmGroup + 1];  // first tile of each problem
+};
+
+__global__ void __launch_bounds__(kThreads, 1) umma_gemm_group_kernel(const __grid_constant__ GemmGroup p) {
+  int q = 0;
+  while (q + 1 < kGemmGroup && static_cast<int>(blockIdx.x) >= p.first[q + 1]) ++q;
+  const GemmArgs &g = p.g[q];
+  const int tile = blockIdx.x - p.first[q], nt = g.N / 256;
+  gemm_tile<256>(g, tile % nt, tile / nt, blockIdx.y);
+}
+
 // Opts a kernel in to its shared memory, once per device (a bit of `done` each).
 template <class Kernel>
 cudaError_t raise_smem(Kernel kernel, int bytes, std::atomic<unsigned long long> &done) {
@@ -345,6 +360,24 @@ int gemm_stages(int n) { return gemm_wide(n) ? Tile<256>::kStages : Tile<128>::k
 
 cudaError_t launch_umma_gemm(const GemmArgs &g, cudaStream_t stream) {
   return gemm_wide(g.N) ? launch_tile<256>(g, stream) : launch_tile<128>(g, stream);
+}
+
+cudaError_t launch_umma_gemm_group(const GemmArgs *g, int count, cudaStream_t stream) {
+  static std::atomic<unsigned long long> configured{0};
+  cudaError_t e = raise_smem(umma_gemm_group_kernel, Tile<256>::kSmemBytes, configured);
+  if (e != cudaSuccess) return e;
+  GemmGroup p{};
+  int tiles = 0;
+  for (int q = 0; q < kGemmGroup; ++q) {
+    p.first[q] = tiles;
+    if (q < count) {
+      p.g[q] = g[q];
+      tiles += (g[q].M / kBM) * (g[q].N / 256);
+    }
+  }
+  p.first[kGemmGroup] = tiles;
+  umma_gemm_group_kernel<<<dim3(tiles, g[0].ksplit), kThreads, Tile<256>::kSmemBytes, stream>>>(p);
+  return cudaGetLastError();
 }
 
 cudaError_t gemm_error_flag(unsigned *out, bool reset) {

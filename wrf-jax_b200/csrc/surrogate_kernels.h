@@ -55,6 +55,10 @@ struct GemmArgs {
 };
 
 cudaError_t launch_umma_gemm(const GemmArgs &g, cudaStream_t stream);
+// Up to kGemmGroup problems of 128 x 256 tiles (N a multiple of 256) and one
+// common K split in one launch.
+constexpr int kGemmGroup = 4;
+cudaError_t launch_umma_gemm_group(const GemmArgs *g, int count, cudaStream_t stream);
 // pipeline stages of the GEMM tile an N selects (the test hook's K bound)
 int gemm_stages(int n);
 
@@ -76,6 +80,18 @@ cudaError_t launch_sur_loss_grad(const float *Y, const float *T, const float *w,
 cudaError_t launch_sur_row_sum(const __nv_bfloat16 *Gt, int ld, int rows, int B, float *db, cudaStream_t s);
 cudaError_t launch_sur_reduce_splits(const float *P, int splits, size_t n, float *G, cudaStream_t s);
 cudaError_t launch_sur_adam(const SurAdamArgs &a, cudaStream_t s);
+// Last two launches of a training step: bias gradients with their Adam step,
+// and the split sums, Adam step and BF16 copies of all weights.
+struct SurUpdateArgs {
+  int layers, splits, batch;
+  int rows[4], cols[4];
+  const __nv_bfloat16 *gt[4];  // d(pre-activation)^T [rows][batch]
+  const float *part[4];        // splits slabs of rows x cols
+  float *w[4], *mw[4], *vw[4], *gw[4], *b[4], *mb[4], *vb[4], *gb[4];
+  __nv_bfloat16 *wb[4], *wbt[4];
+  float lr, beta1, beta2, eps, bc1, bc2, weight_decay;
+};
+cudaError_t launch_sur_update(const SurUpdateArgs &a, cudaStream_t s);
 cudaError_t launch_sur_decode(const SurDecodeArgs &a, cudaStream_t s);
 cudaError_t launch_sur_compact(const unsigned *flags, int ncol, int *list, int *count, cudaStream_t s);
 cudaError_t launch_sur_move_columns(const int *list, const int *count, int max_n, int nz, int ny, const float *src,

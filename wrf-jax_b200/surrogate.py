@@ -243,10 +243,7 @@ class SurrogateModel:
             gw=[torch.empty_like(w) for w in self.w], gb=[torch.empty_like(b) for b in self.b],
             loss=e(1),
         )
-        self._ksplit = max(1, min(16, B // 1024))
-        while B % (64 * self._ksplit):
-            self._ksplit //= 2
-        buf["part"] = e(self._ksplit * HIDDEN * max(K_IN, HIDDEN))
+        buf["part"] = e(max(1, _capi.load().rrtmg_sur_train_part_floats(B)))
         self._buf, self._buf_batch = buf, B
         return buf
 
@@ -284,40 +281,22 @@ class SurrogateModel:
         lib = _capi.load()
         B = idx.shape[0]
         b = self._buffers(B)
-        s = _stream()
-        _check(lib.rrtmg_sur_gather(X.data_ptr(), K_IN, Tn.data_ptr(), N_OUT, idx.data_ptr(), B, b["Xb"].data_ptr(),
-                                    b["Xbt"].data_ptr(), B, b["Tb"].data_ptr(), s), "gather")
-        self.forward(b["Xb"], Z=b["Z"], H=b["H"], Ht=b["Ht"], Y=b["Y"])
-        _check(lib.rrtmg_sur_loss_grad(b["Y"].data_ptr(), b["Tb"].data_ptr(), weights.data_ptr(), B, N_OUT,
-                                       1.0 / (B * N_TARGETS), b["dY"].data_ptr(), b["dYt"].data_ptr(), B,
-                                       b["loss"].data_ptr(), s), "loss gradient")
-        ks = self._ksplit
-        # layer 4 (linear), then the three GELU layers, last to first
-        grads_in = (b["dYt"], b["dZt"][2], b["dZt"][1], b["dZt"][0])   # d(pre-activation)^T per layer 3..0
-        acts_t = (b["Ht"][2], b["Ht"][1], b["Ht"][0], b["Xbt"])          # layer inputs^T
-        for layer, gt, at in zip((3, 2, 1, 0), grads_in, acts_t):
-            out_f, in_f = LAYER_SHAPES[layer]
-            part = b["part"][:ks * out_f * in_f].view(ks, out_f, in_f)
-            gemm_bf16(gt, at, epilogue=_capi.EPI_F32, C=part, ksplit=ks)
-            _check(lib.rrtmg_sur_reduce_splits(part.data_ptr(), ks, out_f * in_f, b["gw"][layer].data_ptr(), s),
-                   "reduce splits")
-            _check(lib.rrtmg_sur_row_sum(gt.data_ptr(), B, out_f, B, b["gb"][layer].data_ptr(), s), "bias gradient")
-            if layer > 0:
-                g_rows = b["dY"] if layer == 3 else b["dZ"][layer]
-                gemm_bf16(g_rows, self.wbt[layer], epilogue=_capi.EPI_DGELU, aux=b["Z"][layer - 1],
-                          H=b["dZ"][layer - 1], Ht=b["dZt"][layer - 1])
-        self.step += 1
-        bc1, bc2 = 1.0 - beta1 ** self.step, 1.0 - beta2 ** self.step
-        for i, (out_f, in_f) in enumerate(LAYER_SHAPES):
-            a = _capi.SurAdamArgs(rows=out_f, cols=in_f, w=self.w[i].data_ptr(), m=self.mw[i].data_ptr(),
-                                  v=self.vw[i].data_ptr(), grad=b["gw"][i].data_ptr(), lr=lr, beta1=beta1,
-                                  beta2=beta2, eps=eps, bc1=bc1, bc2=bc2, weight_decay=weight_decay,
-                                  wb=self.wb[i].data_ptr(), ldwb=in_f, wbt=self.wbt[i].data_ptr(), ldwbt=out_f)
-            _check(lib.rrtmg_sur_adam(ctypes.byref(a), s), "adam (weights)")
-            a = _capi.SurAdamArgs(rows=1, cols=out_f, w=self.b[i].data_ptr(), m=self.mb[i].data_ptr(),
-                                  v=self.vb[i].data_ptr(), grad=b["gb"][i].data_ptr(), lr=lr, beta1=beta1,
-                                  beta2=beta2, eps=eps, bc1=bc1, bc2=bc2, weight_decay=0.0)
-            _check(lib.rrtmg_sur_adam(ctypes.byref(a), s), "adam (biases)")
+        step = self.step + 1
+        a = _capi.SurTrainArgs(
+            X=X.data_ptr(), ldx=K_IN, T=Tn.data_ptr(), ldt=N_OUT, idx=idx.data_ptr(), batch=B,
+            weights=weights.data_ptr(), loss_scale=1.0 / (B * N_TARGETS), lr=lr, beta1=beta1, beta2=beta2, eps=eps,
+            bc1=1.0 - beta1 ** step, bc2=1.0 - beta2 ** step, weight_decay=weight_decay,
+            Xb=b["Xb"].data_ptr(), Xbt=b["Xbt"].data_ptr(), Tb=b["Tb"].data_ptr(), Y=b["Y"].data_ptr(),
+            dY=b["dY"].data_ptr(), dYt=b["dYt"].data_ptr(), part=b["part"].data_ptr(), loss=b["loss"].data_ptr())
+        for name, tensors in (("w", self.w), ("mw", self.mw), ("vw", self.vw), ("gw", b["gw"]), ("b", self.b),
+                              ("mb", self.mb), ("vb", self.vb), ("gb", b["gb"]), ("wb", self.wb), ("wbt", self.wbt),
+                              ("Z", b["Z"]), ("H", b["H"]), ("Ht", b["Ht"]), ("dZ", b["dZ"]), ("dZt", b["dZt"])):
+            field = getattr(a, name)
+            for i, t in enumerate(tensors):
+                field[i] = t.data_ptr()
+        if lib.rrtmg_sur_train_step(ctypes.byref(a), _stream()) != 0:
+            raise ValueError(f"rrtmg_sur_train_step rejected the arguments (batch {B}; a multiple of 128 is needed)")
+        self.step = step
 
     # -- persistence ----------------------------------------------------------
     def state(self) -> dict:
