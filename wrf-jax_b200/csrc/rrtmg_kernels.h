@@ -80,6 +80,14 @@ struct SwArgs {
 // default day-list slots per chunk of the SW sweep schedule (its records take
 // about 64 KB per slot at nk = 50)
 constexpr int kSwChunkColumns = 32768;
+// Chunks of up to kSmallColumns columns may hold few enough live (LW) or day
+// (SW) columns for the small-chunk sweeps (transfer terms of all layers first,
+// then the recurrences alone): up to kLwSmallColumns / kSwSmallColumns, which
+// the kernels of both forms find on the device.
+constexpr int kSmallColumns = 2048;
+constexpr int kSwSmallColumns = 320, kLwSmallColumns = 384;
+// blocks of their transfer-term kernels: 16 per SM
+constexpr int kSmallBlocks = 148 * 16;
 // no longer used by the SW path (every domain runs the sweep schedule); kept
 // as the default of the schedule field that used to select it
 constexpr int kSwSplitMaxColumns = 4096;

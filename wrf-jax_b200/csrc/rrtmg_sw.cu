@@ -16,8 +16,6 @@
 // transmittance, direct beam, downward adding recurrence) and a bottom-up pass
 // (upward adding recurrence, level fluxes) that accumulates the spectral sums
 // in g-point order.
-#include <atomic>
-
 #include "rrtmg_device.cuh"
 #include "rrtmg_divide.cuh"
 #include "rrtmg_kernels.h"
@@ -1388,6 +1386,53 @@ __device__ __forceinline__ void sweep_flush(SweepShared &S, int round, int count
   S.sums[c][type0 + q][level0 + dir * j] = acc;
 }
 
+// A layer's optics: the checked form, or the general one where that says so
+// and in the FP64 mode.
+template <bool kFp64>
+__device__ __forceinline__ SwOptics sw_clear(const Tables &T, float tg, float tr, float mu, float y_mu, SwClear &c) {
+  if constexpr (kFp64) {
+    return sw_clear_any<true>(T, tg, tr, mu, c);
+  } else {
+    bool ok;
+    SwOptics o = sw_clear_safe(T, tg, tr, mu, y_mu, c, ok);
+    if (!ok) o = sw_clear_slow(T, tg, tr, mu, c);
+    return o;
+  }
+}
+
+template <bool kFp64>
+__device__ __forceinline__ SwOptics sw_cloudy(const Tables &T, const SwClear &c, const SwOptics &oc, float4 cld,
+                                              float mu, float y_mu) {
+  if constexpr (kFp64) {
+    return sw_cloudy_any<true>(T, c, oc, cld, mu);
+  } else {
+    bool ok = c.zgcc == 0.0f && safe_size(c.ztau);
+    SwOptics o = sw_cloudy_safe(T, c, cld, mu, y_mu, ok);
+    if (!ok) o = sw_cloudy_slow(T, c, oc, cld, mu);
+    return o;
+  }
+}
+
+// Surface albedos of a g-point's band, direct (albp) and diffuse (albd), from
+// the Noah-MP fields where these are given, for columns with xland < 1.5
+// (sw:2519-2530): visible in bands 25-28, near infrared in 16-24 and 29
+// (sw:2120-2127).
+__device__ __forceinline__ void sw_albedos(const SwArgs &a, int col, int band, float &albp, float &albd) {
+  if (!a.in.alswvisdir || !(ld(a.in.xland + col) < 1.5f)) return;
+  const bool vis = band >= 9 && band <= 12;
+  albp = ld((vis ? a.in.alswvisdir : a.in.alswnirdir) + col);
+  albd = ld((vis ? a.in.alswvisdif : a.in.alswnirdif) + col);
+}
+
+// Day slots of the launched chunk, and whether the small-chunk sweep takes them.
+__device__ __forceinline__ int sw_chunk_slots(const SwArgs &a) {
+  const int left = *a.nday - a.chunk_first;
+  return left < a.chunk_count ? left : a.chunk_count;
+}
+__device__ __forceinline__ bool sw_small(const SwArgs &a, int slots) {
+  return a.chunk_capacity <= kSmallColumns && slots <= kSwSmallColumns;
+}
+
 // 1 / d of the adding method's denominators 1 - r r', in (0, 1] but for
 // roundings and meaningless inputs.
 __device__ __forceinline__ float sw_recip(float d) { return safe_size(d) ? recip_in_range(d) : 1.0f / d; }
@@ -1451,7 +1496,7 @@ __global__ void __launch_bounds__(kSweepThreads, kSwSweepMinBlocks) sw_sweep_ker
   SweepShared &S = *reinterpret_cast<SweepShared *>(smem_raw);
   const int nday = *a.nday;
   const int u0 = blockIdx.x * kSweepCols;
-  if (u0 >= a.chunk_count || a.chunk_first + u0 >= nday) return;  // whole block
+  if (u0 >= a.chunk_count || a.chunk_first + u0 >= nday || sw_small(a, sw_chunk_slots(a))) return;  // whole block
   const int cslot = threadIdx.x / kSwGpts;
   const int G = threadIdx.x - cslot * kSwGpts;
   const int u_own = u0 + cslot;
@@ -1520,14 +1565,7 @@ __global__ void __launch_bounds__(kSweepThreads, kSwSweepMinBlocks) sw_sweep_ker
     const float4 cld = nx_cld;
     if (l > 0) load(l - 1);
     SwClear c;
-    SwOptics oc;
-    if constexpr (kFp64) {
-      oc = sw_clear_any<true>(T, tg, tr, mu, c);
-    } else {
-      bool ok;
-      oc = sw_clear_safe(T, tg, tr, mu, y_mu, c, ok);
-      if (!ok) oc = sw_clear_slow(T, tg, tr, mu, c);
-    }
+    const SwOptics oc = sw_clear<kFp64>(T, tg, tr, mu, y_mu, c);
     stc[r].rt = make_float4(oc.rt.ref, oc.rt.refd, oc.rt.tra, oc.rt.trad);
     stc[r].dn = make_float4(oc.dbt, cc.tdbt, cc.tdn, cc.rdnd);
     if (cldb && !differ) {
@@ -1538,13 +1576,7 @@ __global__ void __launch_bounds__(kSweepThreads, kSwSweepMinBlocks) sw_sweep_ker
     if (differ) {
       SwOptics ot;
       if (cldb) {
-        if constexpr (kFp64) {
-          ot = sw_cloudy_any<true>(T, c, oc, cld, mu);
-        } else {
-          bool ok = c.zgcc == 0.0f && safe_size(c.ztau);
-          ot = sw_cloudy_safe(T, c, cld, mu, y_mu, ok);
-          if (!ok) ot = sw_cloudy_slow(T, c, oc, cld, mu);
-        }
+        ot = sw_cloudy<kFp64>(T, c, oc, cld, mu, y_mu);
         stt[r].rt = make_float4(ot.rt.ref, ot.rt.refd, ot.rt.tra, ot.rt.trad);
         cloudy_bits |= 1u << (r & 31);
       } else {
@@ -1579,15 +1611,8 @@ __global__ void __launch_bounds__(kSweepThreads, kSwSweepMinBlocks) sw_sweep_ker
   if (!differ) ct = cc;
 
   // ---- bottom-up pass: upward adding and level fluxes (vrtqdr, sw:3655-3720)
-  // surface albedos of this g-point's band: direct (albp) and diffuse (albd);
-  // the Noah-MP fields, when given, for columns with xland < 1.5 (sw:2519-2530):
-  // visible in bands 25-28, near infrared in 16-24 and 29 (sw:2120-2127)
   float albp = C.albedo, albd = C.albedo;
-  if (a.in.alswvisdir && ld(a.in.xland + col) < 1.5f) {
-    const bool vis = band >= 9 && band <= 12;
-    albp = ld((vis ? a.in.alswvisdir : a.in.alswnirdir) + col);
-    albd = ld((vis ? a.in.alswvisdif : a.in.alswnirdif) + col);
-  }
+  sw_albedos(a, col, band, albp, albd);
   float rupc = albp, rupdc = albd;
   float rupt = albp, rupdt = albd;
   level0 = n;
@@ -1650,6 +1675,226 @@ __global__ void __launch_bounds__(kSweepThreads, kSwSweepMinBlocks) sw_sweep_ker
   if (G == 0 && live) sw_column_outputs(a, C, col, &S.sums[cslot][0][0], kMaxLev);
 }
 
+// ---------------------------------------------------------------------------
+// The sweep of small chunks.  With few columns the kernel above is a serial
+// chain: each level's optics, some 400 dependent operations, wait for the level
+// before although only the adding recurrences depend on it.  Here the optics of
+// all layers are evaluated first, a thread per (slot, layer, g-point), into
+// optics records, and the sweep then runs the recurrences alone, its loads four
+// levels ahead.  The operations are the same functions, so the results are the
+// same bits.  Sweep of 11 day columns of 50 layers 132 -> 64 us, of 180 day
+// columns 181 -> 95 us, of 360 194 -> 181 us; of 720 296 us against 214, as the
+// optics records (274 KB per slot) then pass through memory: hence
+// kSwSmallColumns.
+// ---------------------------------------------------------------------------
+
+// Optics record of a (slot, layer): clear-sky (ref, refd, tra, trad) and (dbt,
+// dbt_nd) of every g-point, then the total sky's where the g-point is cloudy.
+constexpr int kSwOptClearDbt = 4 * kSwGpts, kSwOptTotal = 6 * kSwGpts, kSwOptTotalDbt = 10 * kSwGpts;
+constexpr int kSwOpt = 12 * kSwGpts;
+static_assert(kSwOpt % 8 == 0 && kSwOptClearDbt % 4 == 0 && kSwOptTotal % 4 == 0, "optics records");
+
+__host__ __device__ __forceinline__ size_t sw_base_floats(int nk, int chunk) {
+  const size_t f = (kSwColRecFloats + static_cast<size_t>(kSwRec + kSwLayerFields) * (nk + 1)) * chunk;
+  return (f + 7) / 8 * 8;
+}
+__device__ __forceinline__ float *sw_optrec(const SwArgs &a, int u, int l) {
+  return a.records + sw_base_floats(a.nk, a.chunk_capacity) + (static_cast<size_t>(u) * (a.nk + 1) + l) * kSwOpt;
+}
+
+// One (slot, layer) per item, g-points over the threads; the grid is bounded and
+// walks the items, as the day count is known on the device only.
+template <bool kFp64>
+__global__ void __launch_bounds__(kSwGpts) sw_small_optics_kernel(const __grid_constant__ Tables T, const SwArgs a) {
+  const int G = threadIdx.x, n = a.nk + 1;
+  int band = kSwBands - 1;
+  while (G < kSwGofsDev[band]) --band;
+  const int P = kPadOfsDev[band] + (G - kSwGofsDev[band]);
+  const int slots = sw_chunk_slots(a);
+  if (!sw_small(a, slots)) return;
+  const long long items = static_cast<long long>(slots) * n;
+  for (long long item = blockIdx.x; item < items; item += gridDim.x) {
+    const int u = static_cast<int>(item / n), l = static_cast<int>(item - static_cast<long long>(u) * n);
+    const int col = a.daylist[a.chunk_first + u];
+    const float mu = sw_colrecs(a)[u].C.mu;
+    const float *rec = sw_layrecs(a) + (static_cast<size_t>(u) * n + l) * kSwRec;
+    const float tg = rec[P], tr = rec[kSwRecTaur + P];
+    const float4 cld = *reinterpret_cast<const float4 *>(rec + kSwRecCloud + 4 * band);
+    const uint32_t word = a.mask[(static_cast<size_t>(l) * kSwMaskWords + (G >> 5)) * a.ncol + col];
+    float *out = sw_optrec(a, u, l);
+    auto put = [&](int rt, int dbt, const SwOptics &o) {
+      reinterpret_cast<float4 *>(out + rt)[G] = make_float4(o.rt.ref, o.rt.refd, o.rt.tra, o.rt.trad);
+      reinterpret_cast<float2 *>(out + dbt)[G] = make_float2(o.dbt, o.dbt_nd);
+    };
+    SwClear c;
+    const SwOptics oc = sw_clear<kFp64>(T, tg, tr, mu, recip_in_range(mu), c);
+    put(0, kSwOptClearDbt, oc);
+    if (a.icld != 0 && ((word >> (G & 31)) & 1u) != 0u)
+      put(kSwOptTotal, kSwOptTotalDbt, sw_cloudy<kFp64>(T, c, oc, cld, mu, recip_in_range(mu)));
+  }
+}
+
+constexpr int kAhead = 4;  // levels loaded ahead by the small sweep
+
+__global__ void __launch_bounds__(kSweepThreads, 1) sw_small_sweep_kernel(const SwArgs a) {
+  extern __shared__ __align__(16) unsigned char smem_raw[];
+  SweepShared &S = *reinterpret_cast<SweepShared *>(smem_raw);
+  const int slots = sw_chunk_slots(a);
+  const int u0 = blockIdx.x * kSweepCols;
+  if (u0 >= slots || !sw_small(a, slots)) return;  // whole block
+  const int cslot = threadIdx.x / kSwGpts;
+  const int G = threadIdx.x - cslot * kSwGpts;
+  const bool live = u0 + cslot < slots;
+  const int u = live ? u0 + cslot : u0;
+  const int col = a.daylist[a.chunk_first + u];
+  const SwColRec &R = sw_colrecs(a)[u];
+  const Col C = R.C;
+  const int n = C.nlay;
+  const bool clear_only = a.icld == 0;
+  int band = kSwBands - 1;
+  while (G < kSwGofsDev[band]) --band;
+  const float *opt = sw_optrec(a, u, 0);
+  const uint32_t *mword = a.mask + col + static_cast<size_t>(G >> 5) * a.ncol;
+  const size_t mstride = static_cast<size_t>(kSwMaskWords) * a.ncol;
+  const uint32_t bit = 1u << (G & 31);
+  const float zincflx = ((C.adjflux * R.sflux[G]) * C.mu) * 1.0f;
+  float *const ring0 = &S.ring[0][cslot][G];
+  constexpr int kTypeStep = kSweepCols * kRingStride, kBufStep = kRingRows * kRingStride;
+  constexpr int kDownLevels = kRingRows / (2 * kSweepCols), kUpLevels = kRingRows / (4 * kSweepCols);
+  static_assert(kUpLevels == kAhead && kDownLevels == 2 * kAhead, "levels per round");
+
+  // a layer's optics on both paths (the total sky's where it is cloudy)
+  struct Slot {
+    float4 rt, trt;
+    float2 d, td;
+    bool cloudy;
+  };
+  auto load = [&](int l, Slot &s) {
+    const float *q = opt + static_cast<size_t>(l) * kSwOpt;
+    s.rt = reinterpret_cast<const float4 *>(q)[G];
+    s.d = reinterpret_cast<const float2 *>(q + kSwOptClearDbt)[G];
+    s.cloudy = !clear_only && (mword[static_cast<size_t>(l) * mstride] & bit) != 0u;
+    s.trt = reinterpret_cast<const float4 *>(q + kSwOptTotal)[G];
+    s.td = reinterpret_cast<const float2 *>(q + kSwOptTotalDbt)[G];
+  };
+  auto optics = [](const float4 &rt, const float2 &d) {
+    SwOptics o;
+    o.rt.ref = rt.x; o.rt.refd = rt.y; o.rt.tra = rt.z; o.rt.trad = rt.w;
+    o.dbt = d.x;
+    o.dbt_nd = d.y;
+    return o;
+  };
+
+  // ---- top-down: the recurrences' values at each level go to the stacks
+  SwCarry stc[kMaxLev], stt[kMaxLev];
+  SwCarry cc{1.0f, 1.0f, 0.0f}, ct = cc;
+  float tdbtc_nd = 1.0f, tdbt_nd = 1.0f;
+  ring0[0] = tdbt_nd * zincflx;
+  ring0[kTypeStep] = tdbtc_nd * zincflx;
+  int filled = 1, level0 = 0, round = 0;
+  Slot nx[kAhead];
+#pragma unroll
+  for (int j = 0; j < kAhead; ++j)
+    if (j < n) load(n - 1 - j, nx[j]);
+  for (int r0 = 0; r0 < n; r0 += kAhead) {
+    Slot cur[kAhead];
+#pragma unroll
+    for (int j = 0; j < kAhead; ++j) {
+      cur[j] = nx[j];
+      if (r0 + kAhead + j < n) load(n - 1 - (r0 + kAhead + j), nx[j]);
+    }
+#pragma unroll
+    for (int j = 0; j < kAhead; ++j) {
+      const int r = r0 + j;
+      if (r >= n) break;
+      const SwOptics oc = optics(cur[j].rt, cur[j].d);
+      stc[r] = cc;
+      stt[r] = ct;
+      const SwOptics ot = cur[j].cloudy ? optics(cur[j].trt, cur[j].td) : oc;
+      tdbt_nd = tdbt_nd * ot.dbt_nd;
+      ct = sw_down(ct, ot, r == 0);
+      tdbtc_nd = tdbtc_nd * oc.dbt_nd;
+      cc = sw_down(cc, oc, r == 0);
+      float *q = ring0 + (round & 1) * kBufStep + filled * (2 * kTypeStep);
+      q[0] = tdbt_nd * zincflx;
+      q[kTypeStep] = tdbtc_nd * zincflx;
+      if (++filled == kDownLevels || r == n - 1) {
+        sweep_flush<2>(S, round, filled, 4, level0, 1);
+        ++round;
+        level0 += filled;
+        filled = 0;
+      }
+    }
+  }
+
+  // ---- bottom-up: adding from the surface and the level fluxes
+  float albp = C.albedo, albd = C.albedo;
+  sw_albedos(a, col, band, albp, albd);
+  float rupc = albp, rupdc = albd, rupt = albp, rupdt = albd;
+  level0 = n;
+  auto level = [](const float4 &rt, float dbt, const SwCarry &c) {
+    return SwLevel{rt, make_float4(dbt, c.tdbt, c.tdn, c.rdnd)};
+  };
+  struct Up {
+    Slot s;
+    SwCarry c, t;
+  } up[kAhead];
+  auto load_up = [&](int k, Up &v) {  // level k: the layer below it and the level's stack entries
+    load(n - 1 - k, v.s);
+    v.c = stc[k];
+    v.t = stt[k];
+  };
+#pragma unroll
+  for (int j = 0; j < kAhead; ++j)
+    if (n - 1 - j >= 0) load_up(n - 1 - j, up[j]);
+  const float4 surface = make_float4(albp, albd, 0.0f, 0.0f);
+  auto emit = [&](int k, const SwLevel &c, const SwLevel &t) {
+    float fuc, fdc, fut, fdt;
+    sw_fluxes(c, rupc, rupdc, fuc, fdc);
+    sw_fluxes(t, rupt, rupdt, fut, fdt);
+    float *q = ring0 + (round & 1) * kBufStep + filled * (4 * kTypeStep);
+    q[0] = fut * zincflx;
+    q[kTypeStep] = fdt * zincflx;
+    q[2 * kTypeStep] = fuc * zincflx;
+    q[3 * kTypeStep] = fdc * zincflx;
+    if (++filled == kUpLevels || k == 0) {
+      sweep_flush<4>(S, round, filled, 0, level0, -1);
+      ++round;
+      level0 -= filled;
+      filled = 0;
+    }
+  };
+  filled = 0;
+  emit(n, level(surface, 0.0f, cc), level(surface, 0.0f, ct));
+  for (int k0 = n - 1; k0 >= 0; k0 -= kAhead) {
+    Up cur[kAhead];
+#pragma unroll
+    for (int j = 0; j < kAhead; ++j) {
+      cur[j] = up[j];
+      if (k0 - kAhead - j >= 0) load_up(k0 - kAhead - j, up[j]);
+    }
+#pragma unroll
+    for (int j = 0; j < kAhead; ++j) {
+      const int k = k0 - j;
+      if (k < 0) break;
+      const Slot &s = cur[j].s;
+      const SwLevel c = level(s.rt, s.d.x, cur[j].c);
+      const SwLevel t = s.cloudy ? level(s.trt, s.td.x, cur[j].t) : level(s.rt, s.d.x, cur[j].t);
+      sw_up(c, rupc, rupdc);
+      sw_up(t, rupt, rupdt);
+      emit(k, c, t);
+    }
+  }
+  __syncthreads();  // the last round's sums
+  for (int q = threadIdx.x; q < kSweepCols * kMaxLay; q += kSweepThreads) {
+    const int cs = q / kMaxLay, l = q - cs * kMaxLay;
+    const int uq = u0 + cs;
+    if (l >= a.nk || uq >= slots) continue;
+    sw_layer_output(a, sw_colrecs(a)[uq].C, l, &S.sums[cs][0][0], kMaxLev);
+  }
+  if (G == 0 && live) sw_column_outputs(a, C, col, &S.sums[cslot][0][0], kMaxLev);
+}
+
 }  // namespace
 
 cudaError_t launch_sw_daylist(const SwArgs &a, cudaStream_t stream) {
@@ -1660,7 +1905,10 @@ cudaError_t launch_sw_daylist(const SwArgs &a, cudaStream_t stream) {
 }
 
 size_t sw_record_floats(int nk, int chunk) {
-  return (kSwColRecFloats + static_cast<size_t>(kSwRec + kSwLayerFields) * (nk + 1)) * static_cast<size_t>(chunk);
+  return sw_base_floats(nk, chunk) +
+         (chunk <= kSmallColumns
+              ? static_cast<size_t>(kSwOpt) * (nk + 1) * (chunk < kSwSmallColumns ? chunk : kSwSmallColumns)
+              : size_t(0));
 }
 
 cudaError_t launch_sw_chunk_optics(const Tables &T, const SwArgs &a, cudaStream_t stream) {
@@ -1681,22 +1929,23 @@ cudaError_t launch_sw_chunk_optics(const Tables &T, const SwArgs &a, cudaStream_
   return cudaGetLastError();
 }
 
+static_assert(sizeof(SweepShared) <= 48 * 1024, "more shared memory needs the opt-in");
+
 template <bool kFp64>
 static cudaError_t launch_sweep(const Tables &T, const SwArgs &a, cudaStream_t stream) {
-  if (sizeof(SweepShared) > 48 * 1024) {  // a ring of more levels needs the opt-in
-    static std::atomic<unsigned long long> configured{0};
-    int dev = 0;
-    cudaError_t e = cudaGetDevice(&dev);
+  const int pairs = (a.chunk_count + kSweepCols - 1) / kSweepCols;
+  if (a.chunk_capacity <= kSmallColumns) {
+    const int most = a.chunk_count < kSwSmallColumns ? a.chunk_count : kSwSmallColumns;
+    const long long items = static_cast<long long>(most) * (a.nk + 1);
+    sw_small_optics_kernel<kFp64><<<static_cast<int>(items < kSmallBlocks ? items : kSmallBlocks), kSwGpts, 0,
+                                    stream>>>(T, a);
+    cudaError_t e = cudaGetLastError();
     if (e != cudaSuccess) return e;
-    if (dev < 64 && !((configured.load() >> dev) & 1ull)) {
-      e = cudaFuncSetAttribute(sw_sweep_kernel<kFp64>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                               static_cast<int>(sizeof(SweepShared)));
-      if (e != cudaSuccess) return e;
-      configured.fetch_or(1ull << dev);
-    }
+    sw_small_sweep_kernel<<<(most + kSweepCols - 1) / kSweepCols, kSweepThreads, sizeof(SweepShared), stream>>>(a);
+    e = cudaGetLastError();
+    if (e != cudaSuccess || a.chunk_count <= kSwSmallColumns) return e;
   }
-  sw_sweep_kernel<kFp64><<<(a.chunk_count + kSweepCols - 1) / kSweepCols, kSweepThreads, sizeof(SweepShared),
-                           stream>>>(T, a);
+  sw_sweep_kernel<kFp64><<<pairs, kSweepThreads, sizeof(SweepShared), stream>>>(T, a);
   return cudaGetLastError();
 }
 
