@@ -510,18 +510,17 @@ __device__ __forceinline__ float column_pwvcm(const LwArgs &a, const Col &C, flo
 }
 
 // Band diffusivities from the column water (lw:5520-5539).
+__device__ __forceinline__ float band_secdiff(const Tables &T, const Col &C, int b) {
+  const bool variable = !(b == 0 || b == 3 || b >= 9);
+  if (!variable) return 1.66f;
+  const float e = glibc_expf(T, kA2[b] * C.pwvcm);
+  const float v = kA0[b] + kA1[b] * e;
+  return v < 1.50f ? 1.50f : (v > 1.80f ? 1.80f : v);
+}
+
 __device__ __forceinline__ void column_secdiff(const Tables &T, const Col &C, float *secdiff) {
 #pragma unroll
-  for (int b = 0; b < kLwBands; ++b) {
-    const bool variable = !(b == 0 || b == 3 || b >= 9);
-    if (variable) {
-      const float e = glibc_expf(T, kA2[b] * C.pwvcm);
-      const float v = kA0[b] + kA1[b] * e;
-      secdiff[b] = v < 1.50f ? 1.50f : (v > 1.80f ? 1.80f : v);
-    } else {
-      secdiff[b] = 1.66f;
-    }
-  }
+  for (int b = 0; b < kLwBands; ++b) secdiff[b] = band_secdiff(T, C, b);
 }
 
 }  // namespace

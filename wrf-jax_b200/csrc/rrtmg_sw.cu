@@ -1168,6 +1168,15 @@ __device__ __forceinline__ float *sw_layfields(const SwArgs &a) {
   return sw_layrecs(a) + static_cast<size_t>(kSwRec) * (a.nk + 1) * a.chunk_capacity;
 }
 
+// Day slots of the launched chunk, and whether the small-chunk sweep takes them.
+__device__ __forceinline__ int sw_chunk_slots(const SwArgs &a) {
+  const int left = *a.nday - a.chunk_first;
+  return left < a.chunk_count ? left : a.chunk_count;
+}
+__device__ __forceinline__ bool sw_small(const SwArgs &a, int slots) {
+  return a.chunk_capacity <= kSmallColumns && slots <= kSwSmallColumns;
+}
+
 // A warp per day column; the lanes take the layers of the laytrop count.
 __global__ void __launch_bounds__(128) sw_colprep_kernel(Tables T, SwArgs a) {
   const int lane = threadIdx.x & 31;
@@ -1289,27 +1298,31 @@ __global__ void __launch_bounds__(128) sw_layer_kernel(Tables T, SwArgs a) {
 constexpr int kSwOpticsGroup = 128;
 constexpr int kSwOpticsMinBlocks = 5;
 constexpr int kSwSweepMinBlocks = 4;
-__global__ void __launch_bounds__(128, kSwOpticsMinBlocks) sw_optics_kernel(Tables T, SwArgs a, int nblk) {
-  const int group = blockIdx.x / (kSwOpticsGroup * kSwBands);
-  const int g0 = group * kSwOpticsGroup;
-  const int gsize = nblk - g0 < kSwOpticsGroup ? nblk - g0 : kSwOpticsGroup;
-  const int within = blockIdx.x - group * kSwOpticsGroup * kSwBands;
-  const int band = within / gsize;
-  const int blk = g0 + (within - band * gsize);
-  const int n = a.nk + 1;
-  const long long idx = static_cast<long long>(blk) * blockDim.x + threadIdx.x;
-  const int l = static_cast<int>(idx / a.chunk_count);
-  const int u = static_cast<int>(idx - static_cast<long long>(l) * a.chunk_count);
-  const bool live = l < n && a.chunk_first + u < *a.nday;
-  if (!__any_sync(0xffffffffu, live)) return;  // whole warps
+__global__ void __launch_bounds__(128, kSwOpticsMinBlocks) sw_optics_kernel(Tables T, SwArgs a) {
   __shared__ float4 stages[4][kSwStage];
   float4 *stage = stages[threadIdx.x >> 5];
-  const float *fld = sw_layfields(a) + static_cast<size_t>(l) * a.chunk_capacity + u;
+  const int n = a.nk + 1, slots = sw_chunk_slots(a);
+  const int nblk = static_cast<int>((static_cast<long long>(slots > 0 ? slots : 0) * n + 127) / 128);
   const size_t fstride = static_cast<size_t>(n) * a.chunk_capacity;
-  const int record = live ? u * n + l : -1;
+  for (long long vb = blockIdx.x; vb < static_cast<long long>(nblk) * kSwBands; vb += gridDim.x) {
+    const int group = static_cast<int>(vb / (kSwOpticsGroup * kSwBands));
+    const int g0 = group * kSwOpticsGroup;
+    const int gsize = nblk - g0 < kSwOpticsGroup ? nblk - g0 : kSwOpticsGroup;
+    const int within = static_cast<int>(vb - static_cast<long long>(group) * (kSwOpticsGroup * kSwBands));
+    const int band = within / gsize;
+    const int blk = g0 + (within - band * gsize);
+    const long long idx = static_cast<long long>(blk) * blockDim.x + threadIdx.x;
+    const int l = static_cast<int>(idx / slots);
+    const int u = static_cast<int>(idx - static_cast<long long>(l) * slots);
+    const bool live = l < n;
+    if (!__any_sync(0xffffffffu, live)) continue;  // whole warps
+    const float *fld = sw_layfields(a) + static_cast<size_t>(l) * a.chunk_capacity + u;
+    const int record = live ? u * n + l : -1;
 #define RRTMG_SW_OPT(B) sw_band_record<B>(T, a, fld, fstride, record, stage)
-  RRTMG_SW_BAND_SWITCH(band, RRTMG_SW_OPT)
+    RRTMG_SW_BAND_SWITCH(band, RRTMG_SW_OPT)
 #undef RRTMG_SW_OPT
+    __syncwarp();  // the stage is read out
+  }
 }
 
 __global__ void __launch_bounds__(128) sw_source_kernel(Tables T, SwArgs a) {
@@ -1422,15 +1435,6 @@ __device__ __forceinline__ void sw_albedos(const SwArgs &a, int col, int band, f
   const bool vis = band >= 9 && band <= 12;
   albp = ld((vis ? a.in.alswvisdir : a.in.alswnirdir) + col);
   albd = ld((vis ? a.in.alswvisdif : a.in.alswnirdif) + col);
-}
-
-// Day slots of the launched chunk, and whether the small-chunk sweep takes them.
-__device__ __forceinline__ int sw_chunk_slots(const SwArgs &a) {
-  const int left = *a.nday - a.chunk_first;
-  return left < a.chunk_count ? left : a.chunk_count;
-}
-__device__ __forceinline__ bool sw_small(const SwArgs &a, int slots) {
-  return a.chunk_capacity <= kSmallColumns && slots <= kSwSmallColumns;
 }
 
 // 1 / d of the adding method's denominators 1 - r r', in (0, 1] but for
@@ -1922,7 +1926,10 @@ cudaError_t launch_sw_chunk_optics(const Tables &T, const SwArgs &a, cudaStream_
   sw_layer_kernel<<<static_cast<unsigned>(blocks), threads, 0, stream>>>(T, a);
   e = cudaGetLastError();
   if (e != cudaSuccess) return e;
-  sw_optics_kernel<<<static_cast<unsigned>(blocks * kSwBands), threads, 0, stream>>>(T, a, static_cast<int>(blocks));
+  // small capacities may hold few day slots: a bounded grid walks those there are
+  const long long optics = blocks * kSwBands;
+  const long long most = a.chunk_capacity <= kSmallColumns ? 148ll * kSwOpticsMinBlocks * 2 : optics;
+  sw_optics_kernel<<<static_cast<unsigned>(optics < most ? optics : most), threads, 0, stream>>>(T, a);
   e = cudaGetLastError();
   if (e != cudaSuccess) return e;
   sw_source_kernel<<<dim3((a.chunk_count + threads - 1) / threads, kSwBands), threads, 0, stream>>>(T, a);
