@@ -14,7 +14,15 @@
 namespace rrtmg {
 namespace {
 
-constexpr int kPrologueThreads = 256;
+// Two blocks of 512 per SM: the kernel is bound by its instructions and by the
+// loads it has in flight, and more registers (56) pay more than more threads.
+// 1000 x 50 x 1000, all outputs: 518 us before (five blocks of 256; the slopes
+// divided out in every column), 424 us now; 442 us with 640 threads, 596 us
+// with 768, 610 us with five blocks of 256; inputs loaded two levels ahead 465 us.
+constexpr int kPrologueThreads = 512;
+constexpr int kPrologueBlocks = 2;  // per SM
+// Two blocks' slope rows and queues share an SM's 227 KB.
+constexpr size_t kSlopeRowsMax = 96 * 1024;
 
 // ---------------------------------------------------------------------------
 // sin / cos as the reference's zenith-angle code evaluates them
@@ -158,7 +166,8 @@ __device__ __forceinline__ float cal_cldfra1(float qv, float qc, float qi, float
   float arg = __fdiv_rn(__fmul_rn(-100.0f, qcld), powf(subsat, 0.49f));
   arg = (arg < -6.9f) ? -6.9f : arg;
   const float rpos = (rhum < 1.0e-10f) ? 1.0e-10f : rhum;
-  const float partial = __fmul_rn(powf(rpos, 0.25f), __fsub_rn(1.0f, expf(arg)));
+  // the fourth root as two rounded square roots: within 0.75 units in the last place
+  const float partial = __fmul_rn(__fsqrt_rn(__fsqrt_rn(rpos)), __fsub_rn(1.0f, expf(arg)));
   return (partial < 0.01f) ? 0.0f : partial;
 }
 
@@ -174,32 +183,59 @@ __device__ __forceinline__ int bracket(const float *tab, int n, float v) {
   return i < 0 ? 0 : (i > n - 2 ? n - 2 : i);
 }
 
+// The climatology of a column.  runtime.py:5775-5782: per month lower +
+// (upper - lower) / span * dlat, then the two months weighted; every statement
+// rounded to binary32.  The slopes (upper - lower) / span belong to the table,
+// not to the column: while they fit, a block forms them once as it stages the
+// table, and a level costs one 16-byte load and seven operations.
 struct OzoneColumn {
-  const float *lo0, *hi0, *lo1, *hi1;  // the two months' rows at the bracketing latitudes
+  const float4 *row;  // (lower, slope) of the two months at the lower latitude; null: the plain tables
+  const float *lo0, *lo1;
+  int levsiz;
   float span, dlat, f1, f2;
-  // runtime.py:5775-5782: per month lower + (upper - lower) / span * dlat,
-  // then the two months weighted; every statement rounded to binary32
+  __device__ __forceinline__ float slope(const float *lo, int l) const {
+    return __fdiv_rn(__fsub_rn(lo[levsiz + l], lo[l]), span);
+  }
   __device__ __forceinline__ float at(int l) const {
-    const float a = __fadd_rn(lo0[l], __fmul_rn(__fdiv_rn(__fsub_rn(hi0[l], lo0[l]), span), dlat));
-    const float b = __fadd_rn(lo1[l], __fmul_rn(__fdiv_rn(__fsub_rn(hi1[l], lo1[l]), span), dlat));
+    const float4 v = row ? row[l] : make_float4(lo0[l], slope(lo0, l), lo1[l], slope(lo1, l));
+    const float a = __fadd_rn(v.x, __fmul_rn(v.y, dlat));
+    const float b = __fadd_rn(v.z, __fmul_rn(v.w, dlat));
     return __fadd_rn(__fmul_rn(a, f1), __fmul_rn(b, f2));
   }
 };
 
+size_t slope_rows_bytes(int levsiz, int latsiz) {
+  return sizeof(float4) * static_cast<size_t>(latsiz > 1 ? latsiz - 1 : 0) * levsiz;
+}
+
 template <bool kCld, bool kOz, bool kCz, bool kFlag>
-__global__ void __launch_bounds__(kPrologueThreads, 5)
-prologue_kernel(const PrologueArgs a) {
-  extern __shared__ float smem[];
-  float *s_plev = smem;                       // levsiz
-  float *s_lat = s_plev + a.levsiz;           // latsiz
-  float *s_oz = s_lat + a.latsiz;             // (2, latsiz, levsiz): month_lo, month_hi
+__global__ void __launch_bounds__(kPrologueThreads, kPrologueBlocks)
+prologue_kernel(const PrologueArgs a, bool slopes) {
+  // slopes: (latsiz - 1, levsiz) rows of OzoneColumn; otherwise
+  // (2, latsiz, levsiz): month_lo, month_hi.  Then the levels and latitudes.
+  extern __shared__ float4 smem[];
+  float *s_oz = reinterpret_cast<float *>(smem);
+  const int tab = a.latsiz * a.levsiz;
+  float *s_plev = s_oz + (slopes ? 4 * (tab - a.levsiz) : 2 * tab);
+  float *s_lat = s_plev + a.levsiz;
   if (kOz) {
-    const int tab = a.latsiz * a.levsiz;
     for (int e = threadIdx.x; e < a.levsiz; e += blockDim.x) s_plev[e] = __ldg(a.oz_plev + e);
     for (int e = threadIdx.x; e < a.latsiz; e += blockDim.x) s_lat[e] = __ldg(a.oz_lat + e);
-    for (int e = threadIdx.x; e < tab; e += blockDim.x) {
-      s_oz[e] = __ldg(a.oz_tab + static_cast<size_t>(a.month_lo) * tab + e);
-      s_oz[tab + e] = __ldg(a.oz_tab + static_cast<size_t>(a.month_hi) * tab + e);
+    const float *m0 = a.oz_tab + static_cast<size_t>(a.month_lo) * tab;
+    const float *m1 = a.oz_tab + static_cast<size_t>(a.month_hi) * tab;
+    if (slopes) {
+      for (int e = threadIdx.x; e < tab - a.levsiz; e += blockDim.x) {
+        const int li = e / a.levsiz;
+        const float span = __fsub_rn(__ldg(a.oz_lat + li + 1), __ldg(a.oz_lat + li));
+        const float x = __ldg(m0 + e), y = __ldg(m1 + e);
+        smem[e] = make_float4(x, __fdiv_rn(__fsub_rn(__ldg(m0 + e + a.levsiz), x), span), y,
+                              __fdiv_rn(__fsub_rn(__ldg(m1 + e + a.levsiz), y), span));
+      }
+    } else {
+      for (int e = threadIdx.x; e < tab; e += blockDim.x) {
+        s_oz[e] = __ldg(m0 + e);
+        s_oz[tab + e] = __ldg(m1 + e);
+      }
     }
     __syncthreads();
   }
@@ -259,11 +295,10 @@ prologue_kernel(const PrologueArgs a) {
       const int li = bracket(s_lat, a.latsiz, lat);
       oz.dlat = __fsub_rn(lat, s_lat[li]);
       oz.span = __fsub_rn(s_lat[li + 1], s_lat[li]);
-      const float *m0 = s_oz, *m1 = s_oz + a.latsiz * a.levsiz;
-      oz.lo0 = m0 + li * a.levsiz;
-      oz.hi0 = oz.lo0 + a.levsiz;
-      oz.lo1 = m1 + li * a.levsiz;
-      oz.hi1 = oz.lo1 + a.levsiz;
+      oz.levsiz = a.levsiz;
+      oz.row = slopes ? smem + li * a.levsiz : nullptr;
+      oz.lo0 = s_oz + li * a.levsiz;
+      oz.lo1 = oz.lo0 + tab;
       oz.f1 = a.fact_lo;
       oz.f2 = a.fact_hi;
     }
@@ -272,9 +307,8 @@ prologue_kernel(const PrologueArgs a) {
     const float ptop = kOz ? s_plev[0] : 0.0f;
     const float pbot = kOz ? s_plev[a.levsiz - 1] : 0.0f;
     // pressure bracket, walked from the previous level's (levels go up, so
-    // it mostly stays or steps down), and the climatology at its two ends
-    int kk = kOz ? a.levsiz - 2 : 0, cached = -1;
-    float v_lo = 0.0f, v_hi = 0.0f;
+    // it mostly stays or steps down)
+    int kk = kOz ? a.levsiz - 2 : 0;
     constexpr bool kQ = kCld || kFlag, kP = kCld || kOz;
     float n_qc = 0.0f, n_qi = 0.0f, n_qs = 0.0f, n_t = 0.0f, n_p = 0.0f;
     auto load = [&](size_t e) {
@@ -324,16 +358,8 @@ prologue_kernel(const PrologueArgs a) {
           // largest kk with plev[kk] < p, clamped to [0, levsiz-2]
           while (kk > 0 && !(s_plev[kk] < p)) --kk;
           while (kk < a.levsiz - 2 && s_plev[kk + 1] < p) ++kk;
-          if (kk != cached) {
-            if (kk == cached - 1) {
-              v_hi = v_lo;
-              v_lo = oz.at(kk);
-            } else {
-              v_lo = oz.at(kk);
-              v_hi = oz.at(kk + 1);
-            }
-            cached = kk;
-          }
+          // at both ends anew: keeping them from level to level makes the lanes diverge
+          const float v_lo = oz.at(kk), v_hi = oz.at(kk + 1);
           const float dpu = __fsub_rn(p, s_plev[kk]);
           const float dpl = __fsub_rn(s_plev[kk + 1], p);
           const float num = __fadd_rn(__fmul_rn(v_lo, dpl), __fmul_rn(v_hi, dpu));
@@ -351,13 +377,13 @@ prologue_kernel(const PrologueArgs a) {
 }
 
 template <bool kCld, bool kOz, bool kCz, bool kFlag>
-cudaError_t launch_variant(const PrologueArgs &a, int blocks, size_t smem, cudaStream_t stream) {
+cudaError_t launch_variant(const PrologueArgs &a, int blocks, size_t smem, bool slopes, cudaStream_t stream) {
   auto kern = prologue_kernel<kCld, kOz, kCz, kFlag>;
   if (smem > 48 * 1024) {
     cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(smem));
     if (e != cudaSuccess) return e;
   }
-  kern<<<blocks, kPrologueThreads, smem, stream>>>(a);
+  kern<<<blocks, kPrologueThreads, smem, stream>>>(a, slopes);
   return cudaGetLastError();
 }
 
@@ -375,17 +401,21 @@ cudaError_t launch_prologue(const PrologueArgs &a, cudaStream_t stream) {
   int dev = 0, sms = 148;
   cudaGetDevice(&dev);
   cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-  const size_t smem = oz ? prologue_smem_bytes(a.levsiz, a.latsiz) : 0;
+  const size_t rows = slope_rows_bytes(a.levsiz, a.latsiz);
+  const bool slopes = oz && rows <= kSlopeRowsMax;
+  const size_t smem = !oz ? 0
+                      : slopes ? rows + sizeof(float) * (static_cast<size_t>(a.levsiz) + a.latsiz)
+                               : prologue_smem_bytes(a.levsiz, a.latsiz);
   // the ozone tables are staged once per block: a persistent grid of a few
   // blocks per SM when they are needed, one thread per column otherwise
   const int need = (ncol + kPrologueThreads - 1) / kPrologueThreads;
-  const int blocks = oz ? std::min(need, sms * 5) : need;
+  const int blocks = oz ? std::min(need, sms * kPrologueBlocks) : need;
   const int key = (cld ? 8 : 0) | (oz ? 4 : 0) | (cz ? 2 : 0) | (flag ? 1 : 0);
   switch (key) {
 #define RRTMG_PROLOGUE_CASE(K)                                                              \
   case K:                                                                                   \
     return launch_variant<((K) & 8) != 0, ((K) & 4) != 0, ((K) & 2) != 0, ((K) & 1) != 0>( \
-        a, blocks, smem, stream);
+        a, blocks, smem, slopes, stream);
     RRTMG_PROLOGUE_CASE(1) RRTMG_PROLOGUE_CASE(2) RRTMG_PROLOGUE_CASE(3) RRTMG_PROLOGUE_CASE(4)
     RRTMG_PROLOGUE_CASE(5) RRTMG_PROLOGUE_CASE(6) RRTMG_PROLOGUE_CASE(7) RRTMG_PROLOGUE_CASE(8)
     RRTMG_PROLOGUE_CASE(9) RRTMG_PROLOGUE_CASE(10) RRTMG_PROLOGUE_CASE(11) RRTMG_PROLOGUE_CASE(12)
