@@ -3,13 +3,13 @@
 //
 //   C[M x N] = A[M x K] * B[N x K]^T      (A, B row-major BF16, FP32 accumulate)
 //
-// One CTA of 256 threads owns a 128 x BN output tile (BN = 128, or 256 on
-// request).  Its accumulator lives in tensor memory (128 lanes x BN FP32
+// One CTA of 256 threads owns a 128 x BN output tile (BN = 128; 64 where that
+// leaves SMs idle; 256 on request).  Its accumulator lives in tensor memory (128 lanes x BN FP32
 // columns).  K advances in blocks of 64: all threads copy the A and B blocks
 // into shared memory (cp.async, three stages) in the 128-byte swizzled
 // K-major layout, and one thread issues four tcgen05.mma (K = 16 each)
 // whose completion is committed to the stage's mbarrier before the stage is
-// refilled.  With BN = 128 two CTAs share an SM, one's epilogue under the
+// refilled.  With BN <= 128 two CTAs share an SM, one's epilogue under the
 // other's loads and MMAs.  The epilogue reads the accumulator back with
 // tcgen05.ld (warp w owns tile rows 32 (w mod 4) .. and column half w / 4), 32
 // columns at a time, and passes them through a shared stage of the warp's own
@@ -46,6 +46,9 @@ using umma::swz;
 constexpr int kBM = 128, kBK = 64;
 constexpr int kThreads = 256;
 
+// The epilogue's stages (EpiStage of each warp) lie over the pipeline's.
+constexpr int kEpiBytes = (32 * 36 * 4 + 2 * 32 * 40 * 2) * (kThreads / 32);
+
 template <int BN>
 struct Tile {
   static constexpr int kStages = 3;
@@ -53,7 +56,7 @@ struct Tile {
   static constexpr int kBytesB = BN * kBK * 2;
   static constexpr int kStageBytes = kBytesA + kBytesB;
   // one extra KB so the stages can start on a 1024-byte boundary
-  static constexpr int kSmemBytes = kStages * kStageBytes + 1024;
+  static constexpr int kSmemBytes = (BN == 64 ? kEpiBytes : kStages * kStageBytes) + 1024;
   static constexpr uint32_t kIdesc = umma::idesc_bf16(kBM, BN);
 };
 
@@ -66,7 +69,8 @@ struct EpiStage {
   __nv_bfloat16 h[32][40];
   __nv_bfloat16 ht[kEpiCols][40];
 };
-static_assert(sizeof(EpiStage) * (kThreads / 32) <= 3 * Tile<128>::kStageBytes, "stages of the epilogue");
+static_assert(sizeof(EpiStage) * (kThreads / 32) == kEpiBytes && kEpiBytes <= 3 * Tile<128>::kStageBytes &&
+                  kEpiBytes >= 3 * Tile<64>::kStageBytes, "stages of the epilogue");
 
 __device__ unsigned g_gemm_error;
 
@@ -304,7 +308,7 @@ __device__ __forceinline__ void gemm_tile(const GemmArgs &g, int nx, int my, int
 }
 
 template <int BN>
-__global__ void __launch_bounds__(kThreads, BN == 128 ? 2 : 1) umma_gemm_kernel(const __grid_constant__ GemmArgs g) {
+__global__ void __launch_bounds__(kThreads, BN == 256 ? 1 : 2) umma_gemm_kernel(const __grid_constant__ GemmArgs g) {
   gemm_tile<BN>(g, blockIdx.x, blockIdx.y, blockIdx.z);
 }
 
@@ -348,8 +352,14 @@ cudaError_t launch_tile(const GemmArgs &g, cudaStream_t stream) {
 }  // namespace
 
 namespace {
-// 0 automatic (128: two CTAs per SM), else 128 or 256
+// 0 automatic (64 or 128: two CTAs per SM), else 128 or 256
 int g_tile_choice = 0;
+// Up to this many 128-wide tiles, twice as many 64-wide ones are used: they
+// still find an SM each, and a tile's epilogue, most of its time, is half as
+// long.  Training step of 1,024 columns (32 tiles per layer) 117 us with
+// 128-wide tiles, 104 us with 64; 2,048 (64 tiles) 128 and 111 us; 3,072 (96
+// tiles) 135 and 139 us.
+constexpr long long kNarrowTiles = 74;
 }  // namespace
 
 void set_gemm_tile(int bn) { g_tile_choice = bn; }
@@ -359,7 +369,10 @@ bool gemm_wide(int n) { return n % 256 == 0 && g_tile_choice == 256; }
 int gemm_stages(int n) { return gemm_wide(n) ? Tile<256>::kStages : Tile<128>::kStages; }
 
 cudaError_t launch_umma_gemm(const GemmArgs &g, cudaStream_t stream) {
-  return gemm_wide(g.N) ? launch_tile<256>(g, stream) : launch_tile<128>(g, stream);
+  if (gemm_wide(g.N)) return launch_tile<256>(g, stream);
+  const long long tiles = static_cast<long long>(g.N / 128) * (g.M / kBM) * g.ksplit;
+  if (g_tile_choice == 0 && tiles <= kNarrowTiles) return launch_tile<64>(g, stream);
+  return launch_tile<128>(g, stream);
 }
 
 cudaError_t launch_umma_gemm_group(const GemmArgs *g, int count, cudaStream_t stream) {
