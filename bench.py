@@ -354,8 +354,13 @@ def run_plain(args):
     sw_chunks = -(-ncol // sched.sw_chunk_columns)
     # LW: McICA, then per chunk column set-up, layer set-up, gas optics, sweep;
     # SW: McICA, day list, then per chunk column set-up, layer set-up, band
-    # optics, solar source, sweep
-    gpu_launches = (1 + 4 * lw_chunks) + (2 + 5 * sw_chunks)
+    # optics, solar source, sweep.  Chunks of at most 2,048 columns may take the
+    # small-chunk forms (two kernels for the sweep's one; for SW the number of
+    # day columns decides on the device, so both forms are launched)
+    lw_n, sw_n = min(ncol, sched.lw_chunk_columns), min(ncol, sched.sw_chunk_columns)
+    lw_sweeps = 2 if lw_n <= 384 else 1
+    sw_sweeps = 2 if sw_n <= 320 else 3 if sw_n <= 2048 else 1
+    gpu_launches = (1 + (3 + lw_sweeps) * lw_chunks) + (2 + (4 + sw_sweeps) * sw_chunks)
     nday = int((np.asarray(sw_host["coszr"]) > 0.0).sum())
     # The sweep kernels of the staged schedules and their HBM bytes per unit.
     # sw_sweep_kernel, per day column: per layer each g-point's gas and
@@ -367,13 +372,14 @@ def run_plain(args):
     # layer is cloudy or its total-sky values differ from the clear-sky ones,
     # are data-dependent and not counted: a lower bound on the bytes moved.
     # lw_sweep_kernel, per column: the layer records read in both sweeps
-    # (2 x 140 + 4 x 16 + 1 floats per layer, twice), the mask (5 words per
-    # layer, twice), pi3d and p8w, 2 heating fields and 15 2-D outputs.
+    # (2 x 140 + 5 x 16 + 5 floats per layer, twice), the 140 table positions
+    # the downward sweep leaves there, pi3d and p8w, 2 heating fields and 15
+    # 2-D outputs.
     nlay_lw = ctx.lib.rrtmg_lw_nlayers(float(lw_host["p_top"]), nk)
     unit_bytes = {
         "sw_sweep_kernel": 4 * (nlay_sw * (2 * 112 + 4 * 14) + 2 * 8 * (nlay_sw + 1) * 112 + 4 * nlay_sw
                                 + nk + (nk + 1) + 2 * nk + 16),
-        "lw_sweep_kernel": 4 * (2 * nlay_lw * (2 * 140 + 4 * 16 + 1) + 2 * 5 * nlay_lw + nk + (nk + 1) + 2 * nk + 15),
+        "lw_sweep_kernel": 4 * (nlay_lw * (2 * (2 * 140 + 5 * 16 + 5) + 140) + nk + (nk + 1) + 2 * nk + 15),
     }
     unit_count = {"sw_sweep_kernel": nday, "lw_sweep_kernel": ncol}
     dom = max(("sw_sweep_kernel", "lw_sweep_kernel"), key=lambda k: launch_ms[k])
@@ -428,13 +434,14 @@ def _surrogate_launches(n_fallback: int, fused: bool) -> int:
     kernel (or 4 GEMMs and a decode), compact; then the fallback's batched
     gather and scatter, the LW sweep schedule (McICA, column set-up, layer
     set-up, gas optics, sweep) and the SW sweep schedule (McICA, day list,
-    column set-up, layer set-up, band optics, solar source, sweep), queued
-    with the rejected count left on the device whatever it is; all of the
-    fallback once more on a domain of the exact size when more columns are
-    rejected than its capacity."""
+    column set-up, layer set-up, band optics, solar source, sweep), each with
+    the two kernels of its small-chunk form, queued with the rejected count
+    left on the device whatever it is; all of the fallback once more on a
+    domain of the exact size, without those, when more columns are rejected
+    than its capacity."""
     from wrf_jax_b200 import surrogate as S
     per_solve = 2 + 5 + 7
-    return (3 if fused else 7) + per_solve + (per_solve if n_fallback > S.FALLBACK_CAPACITY else 0)
+    return (3 if fused else 7) + per_solve + 4 + (per_solve if n_fallback > S.FALLBACK_CAPACITY else 0)
 
 
 def run_surrogate(args):

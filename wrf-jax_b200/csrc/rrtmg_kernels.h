@@ -50,7 +50,7 @@ struct LwArgs {
 };
 
 // default columns per chunk of the LW sweep schedule (its scratch takes about
-// 107 KB per column at nk = 50 and a 50 hPa top)
+// 110 KB per column at nk = 50 and a 50 hPa top)
 constexpr int kLwChunkColumns = 16384;
 // no longer used by the LW path (every domain runs the sweep schedule); kept
 // as the default of the schedule field that used to select the split schedule
@@ -78,7 +78,7 @@ struct SwArgs {
 };
 
 // default day-list slots per chunk of the SW sweep schedule (its records take
-// about 64 KB per slot at nk = 50)
+// about 70 KB per slot at nk = 50)
 constexpr int kSwChunkColumns = 32768;
 // Chunks of up to kSmallColumns columns may hold few enough live (LW) or day
 // (SW) columns for the small-chunk sweeps (transfer terms of all layers first,
