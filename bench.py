@@ -354,13 +354,13 @@ def run_plain(args):
     sw_chunks = -(-ncol // sched.sw_chunk_columns)
     # LW: McICA, then per chunk column set-up, layer set-up, gas optics, sweep;
     # SW: McICA, day list, then per chunk column set-up, layer set-up, band
-    # optics, solar source, sweep.  Chunks of at most 2,048 columns may take the
+    # optics and solar source, sweep.  Chunks of at most 2,048 columns may take the
     # small-chunk forms (two kernels for the sweep's one; for SW the number of
     # day columns decides on the device, so both forms are launched)
     lw_n, sw_n = min(ncol, sched.lw_chunk_columns), min(ncol, sched.sw_chunk_columns)
     lw_sweeps = 2 if lw_n <= 384 else 1
     sw_sweeps = 2 if sw_n <= 320 else 3 if sw_n <= 2048 else 1
-    gpu_launches = (1 + (3 + lw_sweeps) * lw_chunks) + (2 + (4 + sw_sweeps) * sw_chunks)
+    gpu_launches = (1 + (3 + lw_sweeps) * lw_chunks) + (2 + (3 + sw_sweeps) * sw_chunks)
     nday = int((np.asarray(sw_host["coszr"]) > 0.0).sum())
     # The sweep kernels of the staged schedules and their HBM bytes per unit.
     # sw_sweep_kernel, per day column: per layer each g-point's gas and
@@ -434,13 +434,13 @@ def _surrogate_launches(n_fallback: int, fused: bool) -> int:
     kernel (or 4 GEMMs and a decode), compact; then the fallback's batched
     gather and scatter, the LW sweep schedule (McICA, column set-up, layer
     set-up, gas optics, sweep) and the SW sweep schedule (McICA, day list,
-    column set-up, layer set-up, band optics, solar source, sweep), each with
+    column set-up, layer set-up, band optics and solar source, sweep), each with
     the two kernels of its small-chunk form, queued with the rejected count
     left on the device whatever it is; all of the fallback once more on a
     domain of the exact size, without those, when more columns are rejected
     than its capacity."""
     from wrf_jax_b200 import surrogate as S
-    per_solve = 2 + 5 + 7
+    per_solve = 2 + 5 + 6
     return (3 if fused else 7) + per_solve + 4 + (per_solve if n_fallback > S.FALLBACK_CAPACITY else 0)
 
 

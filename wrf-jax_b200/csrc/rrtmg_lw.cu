@@ -113,18 +113,23 @@ __device__ __forceinline__ bool load_mask(const LwArgs &a, int l, int col, uint3
 
 // A warp per column: the lanes take the buffer levels of the column set-up
 // and the layers of the column integrals, whose sums are then taken in layer
-// order from shared memory (the operations and order of column_prologue).
-__global__ void __launch_bounds__(128) lw_colprep_kernel(Tables T, LwArgs a) {
+// order from shared memory (the operations and order of column_setup).  Bound
+// by latency: the record is built in shared memory and leaves it in whole
+// lines; in every lane's local memory, stored by one lane, 2,048 slots took 27
+// us and 4,096 columns 44 us (LW optics of 64 x 64 x 44 323 -> 300 us, of
+// 300 x 300 x 50 6.56 -> 6.09 ms).
+__global__ void __launch_bounds__(128) lw_colprep_kernel(const __grid_constant__ Tables T, const LwArgs a) {
   __shared__ float s_cd[4][kMaxLay], s_wk[4][kMaxLay];
-  __shared__ float s_tlev[4][kMaxBuf + 1], s_o3[4][kMaxBuf];
+  __shared__ float s_tlev[4][kMaxBuf + 2], s_o3[4][kMaxBuf + 1];
+  __shared__ Col s_col[4];
   const int w = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int lc = blockIdx.x * 4 + w;
   if (lc >= a.chunk_count || dead_column(a.live, a.chunk_first + lc)) return;  // whole warps
   const int col = a.chunk_first + lc;
-  ColRec r;
-  Col &C = r.C;
+  Col &C = s_col[w];
   column_head(a, col, C);
-  column_setup<true>(T, a, C, lane, s_tlev[w], s_o3[w]);
+  __syncwarp();
+  column_setup_warp(T, a, C, lane, s_tlev[w], s_o3[w]);
   const int nlay = C.nlay;
   int trop_count = 0;
 #pragma unroll 1
@@ -151,9 +156,12 @@ __global__ void __launch_bounds__(128) lw_colprep_kernel(Tables T, LwArgs a) {
   }
   C.laytrop = trop_count;
   C.pwvcm = column_pwvcm(a, C, amttl, wvttl);
+  __syncwarp();
   ColRec &out = reinterpret_cast<ColRec *>(a.scratch)[lc];
   if (lane < kLwBands) out.secdiff[lane] = band_secdiff(T, C, lane);
-  if (lane == 0) out.C = r.C;
+  static_assert(sizeof(Col) % 4 == 0, "words");
+  for (int q = lane; q < static_cast<int>(sizeof(Col) / 4); q += 32)
+    reinterpret_cast<float *>(&out.C)[q] = reinterpret_cast<const float *>(&C)[q];
 }
 
 // thread = (layer, chunk column), columns fastest

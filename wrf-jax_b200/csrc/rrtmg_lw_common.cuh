@@ -86,58 +86,89 @@ __device__ float retab_interp(const Tables &T, float temp, int hi) {
   return ld(T.retab + index - 1) * (1.0f - corr) + ld(T.retab + index) * corr;
 }
 
+// Interface temperature of the standard profile at pressure p, between the last
+// entry not below p (count entries are) and the next.
+__device__ __forceinline__ float profile_between(const Tables &T, int count, float p) {
+  const int idx = clampi(count - 1, 0, T.nprof - 1);
+  const int idx1 = idx + 1 < T.nprof - 1 ? idx + 1 : T.nprof - 1;
+  const float p0 = ld(T.pprof + idx), p1 = ld(T.pprof + idx1);
+  const float t0 = ld(T.tprof + idx), t1 = ld(T.tprof + idx1);
+  const float w = (idx == T.nprof - 1) ? 0.0f : (p - p0) / (p1 - p0);
+  return w * (t1 - t0) + t0;
+}
+
+// Pressures of the levels above the model top.
+__device__ __forceinline__ void column_levels(const LwArgs &a, Col &C) {
+  C.plev_b[0] = pa_to_hpa(in3w(a.in.p8w, C, C.nk));
+  for (int m = 1; m <= C.nbuf; ++m) C.plev_b[m] = C.plev_b[m - 1] - 4.0f;
+  C.plev_b[C.nbuf] = 0.0f;
+}
+
 // Column set-up: buffer layers above the model top (lw:6633-6786).
-// kWarp: called by the 32 lanes of a warp for one column, each lane taking
-// every 32nd buffer level (temperature) and buffer layer (ozone) into the
-// warp's shared arrays s_tlev / s_o3, which every lane then reads back; the
-// values are those of the one-thread form.
-template <bool kWarp = false>
-__device__ void column_setup(const Tables &T, const LwArgs &a, Col &C, int lane = 0, float *s_tlev = nullptr,
-                             float *s_o3 = nullptr) {
-  const int nk = C.nk, nlay = C.nlay, nbuf = C.nbuf;
-  C.plev_b[0] = pa_to_hpa(in3w(a.in.p8w, C, nk));
-  for (int m = 1; m <= nbuf; ++m) C.plev_b[m] = C.plev_b[m - 1] - 4.0f;
-  C.plev_b[nbuf] = 0.0f;
+__device__ void column_setup(const Tables &T, const LwArgs &a, Col &C) {
+  const int nk = C.nk, nbuf = C.nbuf;
+  column_levels(a, C);
   for (int m = 0; m < nbuf; ++m) C.play_b[m] = 0.5f * (C.plev_b[m] + C.plev_b[m + 1]);
   // interface temperatures from the standard profile plus the model-top offset
   auto varint = [&](float p) {
     int count = 0;
     for (int q = 0; q < T.nprof; ++q) count += (ld(T.pprof + q) >= p);
-    const int idx = clampi(count - 1, 0, T.nprof - 1);
-    const int idx1 = idx + 1 < T.nprof - 1 ? idx + 1 : T.nprof - 1;
-    const float p0 = ld(T.pprof + idx), p1 = ld(T.pprof + idx1);
-    const float t0 = ld(T.tprof + idx), t1 = ld(T.tprof + idx1);
-    const float w = (idx == T.nprof - 1) ? 0.0f : (p - p0) / (p1 - p0);
-    return w * (t1 - t0) + t0;
+    return profile_between(T, count, p);
   };
   const float offset = in3w(a.in.t8w, C, nk - 1) - varint(pa_to_hpa(in3w(a.in.p8w, C, nk - 1)));
-  if constexpr (kWarp) {
-    for (int m = lane; m <= nbuf; m += 32) s_tlev[m] = varint(C.plev_b[m]) + offset;
-  } else {
-    for (int m = 0; m <= nbuf; ++m) C.tlev_b[m] = varint(C.plev_b[m]) + offset;
-  }
+  for (int m = 0; m <= nbuf; ++m) C.tlev_b[m] = varint(C.plev_b[m]) + offset;
   // ozone above the model top (lw:6766-6786)
   const float amdo = 0.603461f;
   const float o3base = in3(a.in.o3, C, nk - 1) -
                        o3data_layer(T, pa_to_hpa(in3w(a.in.p8w, C, nk - 1)), C.plev_b[0]) * amdo;
-  auto o3_layer = [&](int m) {
+  for (int m = 0; m < nbuf; ++m) {
     const float mmr = o3data_layer(T, C.plev_b[m], C.plev_b[m + 1]) * amdo;
     float top = o3base + mmr;
     if (top <= 0.0f) top = mmr;
-    return top;
-  };
-  if constexpr (kWarp) {
-    for (int m = lane; m < nbuf; m += 32) s_o3[m] = o3_layer(m);
-    __syncwarp();
-    for (int m = 0; m <= nbuf; ++m) C.tlev_b[m] = s_tlev[m];
-    for (int m = 0; m < nbuf; ++m) C.o3_b[m] = s_o3[m];
-  } else {
-    for (int m = 0; m < nbuf; ++m) C.o3_b[m] = o3_layer(m);
+    C.o3_b[m] = top;
   }
   // tlay[lev-1] = (tlev[lev] + tlev[lev-1]) / 2 for lev = nk .. nlay
   C.tlay_b[0] = 0.5f * (C.tlev_b[0] + in3w(a.in.t8w, C, nk - 1));
   for (int m = 1; m <= nbuf; ++m) C.tlay_b[m] = 0.5f * (C.tlev_b[m] + C.tlev_b[m - 1]);
-  (void)nlay;
+}
+
+// The same by the 32 lanes of a warp for one column, C in shared memory: a
+// lane takes every 32nd level or layer, with the model-top values (the offset's
+// profile temperature, the ozone base) as one more; s_tlev holds kMaxBuf + 2
+// values, s_o3 kMaxBuf + 1.
+__device__ void column_setup_warp(const Tables &T, const LwArgs &a, Col &C, int lane, float *s_tlev, float *s_o3) {
+  const int nk = C.nk, nbuf = C.nbuf;
+  column_levels(a, C);  // every lane, the same values
+  __syncwarp();
+  for (int m = lane; m < nbuf; m += 32) C.play_b[m] = 0.5f * (C.plev_b[m] + C.plev_b[m + 1]);
+  const float top_p = pa_to_hpa(in3w(a.in.p8w, C, nk - 1)), top_t = in3w(a.in.t8w, C, nk - 1);
+  for (int m0 = 0; m0 < nbuf + 2; m0 += 32) {
+    const int m = m0 + lane;
+    const float p = m <= nbuf ? C.plev_b[m] : top_p;
+    int count = 0;
+    for (int q0 = 0; q0 < T.nprof; q0 += 32) {
+      const float v = q0 + lane < T.nprof ? ld(T.pprof + q0 + lane) : 0.0f;
+      const int end = T.nprof - q0 < 32 ? T.nprof - q0 : 32;
+      for (int q = 0; q < end; ++q) count += __shfl_sync(0xffffffffu, v, q) >= p;
+    }
+    if (m < nbuf + 2) s_tlev[m] = profile_between(T, count, p);
+  }
+  const float amdo = 0.603461f;
+  for (int m = lane; m <= nbuf; m += 32)
+    s_o3[m] = (m < nbuf ? o3data_layer(T, C.plev_b[m], C.plev_b[m + 1]) : o3data_layer(T, top_p, C.plev_b[0])) * amdo;
+  __syncwarp();
+  const float offset = top_t - s_tlev[nbuf + 1];
+  const float o3base = in3(a.in.o3, C, nk - 1) - s_o3[nbuf];
+  for (int m = lane; m <= nbuf; m += 32) C.tlev_b[m] = s_tlev[m] + offset;
+  for (int m = lane; m < nbuf; m += 32) {
+    const float mmr = s_o3[m];
+    float top = o3base + mmr;
+    if (top <= 0.0f) top = mmr;
+    C.o3_b[m] = top;
+  }
+  __syncwarp();
+  for (int m = lane; m <= nbuf; m += 32) C.tlay_b[m] = 0.5f * (C.tlev_b[m] + (m == 0 ? top_t : C.tlev_b[m - 1]));
+  __syncwarp();
 }
 
 // Layer coefficients: inatm (lw:953-1035), cloud paths, setcoef (lw:1175-1441).

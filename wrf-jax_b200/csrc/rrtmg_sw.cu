@@ -1130,8 +1130,8 @@ __device__ __forceinline__ void sw_column_outputs(const SwArgs &a, const Col &C,
 //                      layer fields;
 //   sw_optics_kernel   thread = (day slot, layer), block = one band: the
 //                      band's gas and Rayleigh depths of every g-point and its
-//                      cloud optics, into the layer record;
-//   sw_source_kernel   thread = (day slot, band): the band's solar source;
+//                      cloud optics, into the layer record; some blocks take
+//                      the bands' solar sources, thread = (day slot, band);
 //   sw_sweep_kernel    block = kSweepCols day slots x 112 g-points, thread =
 //                      one g-point: the top-down pass (delta-Eddington layers,
 //                      direct beam, downward adding) and the bottom-up pass
@@ -1298,13 +1298,36 @@ __global__ void __launch_bounds__(128) sw_layer_kernel(Tables T, SwArgs a) {
 constexpr int kSwOpticsGroup = 128;
 constexpr int kSwOpticsMinBlocks = 5;
 constexpr int kSwSweepMinBlocks = 4;
-__global__ void __launch_bounds__(128, kSwOpticsMinBlocks) sw_optics_kernel(Tables T, SwArgs a) {
+__global__ void __launch_bounds__(128, kSwOpticsMinBlocks) sw_optics_kernel(Tables T, SwArgs a, int source_blocks) {
+  // The first blocks take the solar sources, thread = (slot, band): they need
+  // the layer fields only, and a launch of their own took 17 to 21 us however
+  // few columns there were (a warp per slot and band instead of a thread: 6 us
+  // less there, but 0.26 ms more for 300 x 300 columns).
+  if (static_cast<int>(blockIdx.x) < source_blocks) {
+    const int n = a.nk + 1, band = blockIdx.x % kSwBands;
+    const int u = static_cast<int>(blockIdx.x / kSwBands) * blockDim.x + threadIdx.x;
+    if (u >= sw_chunk_slots(a)) return;
+    SwColRec &R = sw_colrecs(a)[u];
+    const float *fld = sw_layfields(a) + u;
+    auto field = [&](int f, int l) { return fld[(static_cast<size_t>(f) * n + l) * a.chunk_capacity]; };
+    auto jp = [&](int l) { return __float_as_int(field(kSwField_jp, l)); };
+#define RRTMG_SW_SRC(B)                                 \
+  {                                                     \
+    constexpr int gofs_ = kGofs[B];                     \
+    sw_source<B>(T, R.C, jp, field, R.sflux + gofs_);   \
+  }
+    RRTMG_SW_BAND_SWITCH(band, RRTMG_SW_SRC)
+#undef RRTMG_SW_SRC
+    return;
+  }
   __shared__ float4 stages[4][kSwStage];
   float4 *stage = stages[threadIdx.x >> 5];
   const int n = a.nk + 1, slots = sw_chunk_slots(a);
   const int nblk = static_cast<int>((static_cast<long long>(slots > 0 ? slots : 0) * n + 127) / 128);
   const size_t fstride = static_cast<size_t>(n) * a.chunk_capacity;
-  for (long long vb = blockIdx.x; vb < static_cast<long long>(nblk) * kSwBands; vb += gridDim.x) {
+  const int step = static_cast<int>(gridDim.x) - source_blocks;
+  for (long long vb = static_cast<int>(blockIdx.x) - source_blocks; vb < static_cast<long long>(nblk) * kSwBands;
+       vb += step) {
     const int group = static_cast<int>(vb / (kSwOpticsGroup * kSwBands));
     const int g0 = group * kSwOpticsGroup;
     const int gsize = nblk - g0 < kSwOpticsGroup ? nblk - g0 : kSwOpticsGroup;
@@ -1325,23 +1348,6 @@ __global__ void __launch_bounds__(128, kSwOpticsMinBlocks) sw_optics_kernel(Tabl
   }
 }
 
-__global__ void __launch_bounds__(128) sw_source_kernel(Tables T, SwArgs a) {
-  const int u = blockIdx.x * blockDim.x + threadIdx.x;
-  if (u >= a.chunk_count || a.chunk_first + u >= *a.nday) return;
-  const int n = a.nk + 1;
-  SwColRec &R = sw_colrecs(a)[u];
-  const int band = blockIdx.y;
-  const float *fld = sw_layfields(a) + u;
-  auto field = [&](int f, int l) { return fld[(static_cast<size_t>(f) * n + l) * a.chunk_capacity]; };
-  auto jp = [&](int l) { return __float_as_int(field(kSwField_jp, l)); };
-#define RRTMG_SW_SRC(B)                                 \
-  {                                                     \
-    constexpr int gofs_ = kGofs[B];                     \
-    sw_source<B>(T, R.C, jp, field, R.sflux + gofs_);   \
-  }
-  RRTMG_SW_BAND_SWITCH(band, RRTMG_SW_SRC)
-#undef RRTMG_SW_SRC
-}
 #undef RRTMG_SW_BAND_SWITCH
 
 __constant__ int kSwGofsDev[kSwBands] = {0, 6, 18, 26, 34, 44, 54, 56, 66, 74, 80, 86, 94, 100};
@@ -1929,10 +1935,9 @@ cudaError_t launch_sw_chunk_optics(const Tables &T, const SwArgs &a, cudaStream_
   // small capacities may hold few day slots: a bounded grid walks those there are
   const long long optics = blocks * kSwBands;
   const long long most = a.chunk_capacity <= kSmallColumns ? 148ll * kSwOpticsMinBlocks * 2 : optics;
-  sw_optics_kernel<<<static_cast<unsigned>(optics < most ? optics : most), threads, 0, stream>>>(T, a);
-  e = cudaGetLastError();
-  if (e != cudaSuccess) return e;
-  sw_source_kernel<<<dim3((a.chunk_count + threads - 1) / threads, kSwBands), threads, 0, stream>>>(T, a);
+  const int sources = (a.chunk_count + threads - 1) / threads * kSwBands;
+  sw_optics_kernel<<<static_cast<unsigned>(sources + (optics < most ? optics : most)), threads, 0, stream>>>(T, a,
+                                                                                                        sources);
   return cudaGetLastError();
 }
 
