@@ -230,8 +230,8 @@ typedef struct {
 rrtmg_status rrtmg_sur_move_fields(const int *list, const int *count, int max_n, int ny, const rrtmg_sur_fields *f,
                                    int to_compact, int stride, int offset, void *stream);
 
-/* GEMM tile width: 0 = automatic (256 columns when N allows, else 128), or
- * 128 / 256 (256 needs N % 256 == 0; narrower N falls back to 128).  Process-
+/* GEMM tile width: 0 = automatic (128 columns, 64 where 128 would leave SMs
+ * idle), or 128 / 256 (256 needs N % 256 == 0; narrower N falls back to 128).  Process-
  * wide; set by the ensemble autotuner. */
 rrtmg_status rrtmg_gemm_set_tile(int bn);
 
