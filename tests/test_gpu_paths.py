@@ -85,6 +85,17 @@ def test_small_domains_equal_large_ones(ctx, nx, ny, nk, more, options):
         _assert_copies(small, big, nx, times, call.__name__)
 
 
+# kMaxBuf = 40 layers above the model top; a warp takes 30 of them (and two values of the top) at once
+@pytest.mark.parametrize("p_top", [500.0, 11600.0, 12000.0, 12400.0, 15900.0])
+def test_column_setup_by_warp_equals_by_thread(ctx, torch_cuda, p_top):
+    """rrtmg_lwrad sets a column up with a warp, rrtmg_lwrad_static_scratch with a thread: the same bits."""
+    from test_zz_no_alloc import _assert_same, _device_call
+    from wrf_jax_b200 import _capi, synthetic
+    st = synthetic.make_columns(5, 9, 20, seed=int(p_top), p_top=p_top)
+    env = (ctx, _capi, torch_cuda)
+    _assert_same(_device_call(env, st, "rrtmg_lwrad"), _device_call(env, st, "rrtmg_lwrad_static_scratch"), str(p_top))
+
+
 @pytest.mark.parametrize("levsiz,latsiz", [(59, 64), (2, 2), (96, 65), (97, 65), (120, 90)])
 def test_ozone_table_forms(ctx, torch_cuda, levsiz, latsiz):
     """The slopes formed once per block (up to 96 KB of rows: 96 x 64 levels and
