@@ -17,8 +17,9 @@ namespace {
 // Two blocks of 512 per SM: the kernel is bound by its instructions and by the
 // loads it has in flight, and more registers (56) pay more than more threads.
 // 1000 x 50 x 1000, all outputs: 518 us before (five blocks of 256; the slopes
-// divided out in every column), 424 us now; 442 us with 640 threads, 596 us
-// with 768, 610 us with five blocks of 256; inputs loaded two levels ahead 465 us.
+// divided out in every column), 424 us so and 407 us with 32-bit indices; with
+// 64-bit ones 640 threads took 442 us, 768 596 us, five blocks of 256 610 us,
+// and inputs loaded two levels ahead 465 us.
 constexpr int kPrologueThreads = 512;
 constexpr int kPrologueBlocks = 2;  // per SM
 // Two blocks' slope rows and queues share an SM's 227 KB.
@@ -208,7 +209,9 @@ size_t slope_rows_bytes(int levsiz, int latsiz) {
   return sizeof(float4) * static_cast<size_t>(latsiz > 1 ? latsiz - 1 : 0) * levsiz;
 }
 
-template <bool kCld, bool kOz, bool kCz, bool kFlag>
+// Off: the type of an element's index, 32 bits where a field has fewer than 2^32
+// elements (424 us with 64 bits, 407 us with 32 at 1000 x 50 x 1000).
+template <bool kCld, bool kOz, bool kCz, bool kFlag, class Off>
 __global__ void __launch_bounds__(kPrologueThreads, kPrologueBlocks)
 prologue_kernel(const PrologueArgs a, bool slopes) {
   // slopes: (latsiz - 1, levsiz) rows of OzoneColumn; otherwise
@@ -246,14 +249,17 @@ prologue_kernel(const PrologueArgs a, bool slopes) {
   bool any_condensate = false;
   // Cloudy levels (the only ones whose cloud fraction is not 0 by the final
   // mask) are queued per warp and evaluated 32 at a time with every lane
-  // busy, instead of in place with most lanes idle: up to 63 element indices
-  // per warp (31 left over plus one level's 32).
-  __shared__ unsigned long long s_queue[kPrologueThreads / 32][64];
-  unsigned long long *q = s_queue[threadIdx.x >> 5];
-  int qn = 0;  // warp-uniform
+  // busy, instead of in place with most lanes idle: a ring of up to 63 element
+  // indices per warp (31 left over plus one level's 32).  With the inputs queued
+  // too, instead of read again, qv has to be read everywhere: 409 us at
+  // 1000 x 50 x 1000 with 12% of the levels cloudy, 357 us instead of 334 us
+  // with none.
+  __shared__ Off s_queue[kPrologueThreads / 32][64];
+  Off *q = s_queue[threadIdx.x >> 5];
+  int qn = 0, head = 0;  // warp-uniform
   auto drain = [&](int n) {
     if (lane < n) {
-      const size_t e = q[lane];
+      const Off e = q[(head + lane) & 63];
       a.cldfra[e] = cal_cldfra1(__ldg(a.qv + e), __ldg(a.qc + e), __ldg(a.qi + e), __ldg(a.qs + e),
                                 __ldg(a.t + e), __ldg(a.p + e));
     }
@@ -303,7 +309,7 @@ prologue_kernel(const PrologueArgs a, bool slopes) {
       oz.f2 = a.fact_hi;
     }
     if (!(kCld || kOz || kFlag)) continue;
-    const size_t base = static_cast<size_t>(i) * a.nk * a.ny + j;
+    const Off base = static_cast<Off>(i) * static_cast<Off>(a.nk) * static_cast<Off>(a.ny) + static_cast<Off>(j);
     const float ptop = kOz ? s_plev[0] : 0.0f;
     const float pbot = kOz ? s_plev[a.levsiz - 1] : 0.0f;
     // pressure bracket, walked from the previous level's (levels go up, so
@@ -311,7 +317,7 @@ prologue_kernel(const PrologueArgs a, bool slopes) {
     int kk = kOz ? a.levsiz - 2 : 0;
     constexpr bool kQ = kCld || kFlag, kP = kCld || kOz;
     float n_qc = 0.0f, n_qi = 0.0f, n_qs = 0.0f, n_t = 0.0f, n_p = 0.0f;
-    auto load = [&](size_t e) {
+    auto load = [&](Off e) {
       if (kQ) {
         n_qc = __ldg(a.qc + e);
         n_qi = __ldg(a.qi + e);
@@ -322,7 +328,7 @@ prologue_kernel(const PrologueArgs a, bool slopes) {
     };
     load(base);
     for (int k = 0; k < a.nk; ++k) {
-      const size_t e = base + static_cast<size_t>(k) * a.ny;
+      const Off e = base + static_cast<Off>(k) * static_cast<Off>(a.ny);
       const float qc = n_qc, qi = n_qi, qs = n_qs, t = n_t, p = n_p;
       if (k + 1 < a.nk) load(e + a.ny);
       if (kFlag)
@@ -335,15 +341,14 @@ prologue_kernel(const PrologueArgs a, bool slopes) {
           if (!heavy) a.cldfra[e] = 0.0f;
         }
         const unsigned m = __ballot_sync(0xffffffffu, heavy);
-        if (heavy) q[qn + __popc(m & ((1u << lane) - 1u))] = e;
+        if (heavy) q[(head + qn + __popc(m & ((1u << lane) - 1u))) & 63] = e;
         qn += __popc(m);
         if (qn >= 32) {
           __syncwarp();
           drain(32);
           __syncwarp();
-          if (lane < qn - 32) q[lane] = q[32 + lane];
+          head += 32;
           qn -= 32;
-          __syncwarp();
         }
       }
       if (kOz && live) {
@@ -378,7 +383,8 @@ prologue_kernel(const PrologueArgs a, bool slopes) {
 
 template <bool kCld, bool kOz, bool kCz, bool kFlag>
 cudaError_t launch_variant(const PrologueArgs &a, int blocks, size_t smem, bool slopes, cudaStream_t stream) {
-  auto kern = prologue_kernel<kCld, kOz, kCz, kFlag>;
+  const bool narrow = static_cast<unsigned long long>(a.nx) * a.ny <= 0xffffffffull / a.nk;
+  auto kern = narrow ? prologue_kernel<kCld, kOz, kCz, kFlag, unsigned> : prologue_kernel<kCld, kOz, kCz, kFlag, size_t>;
   if (smem > 48 * 1024) {
     cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(smem));
     if (e != cudaSuccess) return e;
