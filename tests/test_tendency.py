@@ -109,3 +109,40 @@ def test_gpu_matches_oracle_large(pkg, to, jme):
         r, t = tendency.radiation_tendency(lw, sw, c1, c2, mut, t0, flags, **b)
         assert np.array_equal(r.view(np.uint32), want_r.view(np.uint32))
         assert np.array_equal(t.view(np.uint32), want_t.view(np.uint32))
+
+
+# rows of a multiple of four elements, other rows, and arrays that are not 16-byte aligned
+@pytest.mark.gpu
+@pytest.mark.parametrize("south_north,offset", [(1000, 0), (1001, 0), (1000, 1)])
+def test_gpu_in_place_tiles_on_two_streams(pkg, south_north, offset):
+    """Two tiles of one array updated in place at the same time, on two streams:
+    neither call writes outside its own tile, so no update of either is lost.
+    Every pass adds 1 (small whole numbers, exact)."""
+    import torch
+    if not torch.cuda.is_available():
+        pytest.skip("no CUDA device")
+    from wrf_jax_b200 import _capi, tendency
+    lib = _capi.load()
+    nx, nk, ny = 64, 21, south_north
+    n, passes = nx * nk * ny, 200
+    flat = torch.zeros(n + 4, device="cuda")
+    t = flat[offset:offset + n]
+    one = torch.ones(n + 4, device="cuda")[offset:offset + n]
+    assert t.data_ptr() % 16 == 4 * offset
+    dims = dict(ids=1, ide=nx + 1, jds=1, jde=ny + 1, kds=1, kde=nk, ims=1, ime=nx, jms=1, jme=ny, kms=1, kme=nk,
+                kts=1, kte=nk - 1)
+    # rows shared by both tiles, split where no 16-byte boundary lies; the second tile leaves out the last rows
+    tiles = [dict(its=1, ite=nx, jts=3, jte=498), dict(its=2, ite=nx - 3, jts=499, jte=ny - 2)]
+    streams = [torch.cuda.Stream() for _ in tiles]
+    torch.cuda.synchronize()
+    for _ in range(passes):
+        for b, s in zip(tiles, streams):
+            tb = tendency.bounds({}, **dims, **b)
+            assert lib.rrtmg_phy_ra_ten(ctypes.byref(tb), t.data_ptr(), one.data_ptr(),
+                                        ctypes.c_void_p(s.cuda_stream)) == 0
+    torch.cuda.synchronize()
+    want = torch.zeros(nx, nk, ny)
+    for b in tiles:
+        want[b["its"] - 1:b["ite"], :nk - 1, b["jts"] - 1:b["jte"]] += passes
+    assert torch.equal(t.cpu().view(nx, nk, ny), want)
+    assert not flat[:offset].any() and not flat[offset + n:].any()

@@ -33,11 +33,27 @@ struct TendArgs {
 // One element: the coupled heating and the new tendency (runtime.py:7946;
 // module_em.py:597-601: factor = c1 * mut (rounded) + c2 (rounded), field *
 // factor; module_physics_addtendc.py:204: lvar.at[region].add(rvar[region])).
-__device__ __forceinline__ void element(const TendArgs &a, int i, int k, int j, float lw, float sw, float c1, float c2,
+// Whether rt_tendf is to be written there: in place only inside the a2a region,
+// as the elements around it may be another tile's or a halo, which another
+// stream may be updating meanwhile.
+__device__ __forceinline__ bool element(const TendArgs &a, int i, int k, int j, float lw, float sw, float c1, float c2,
                                         float mut, float &r, float &t) {
   r = a.sw ? __fadd_rn(lw, sw) : lw;
   if (a.couple && a.tile.has(i, k, j)) r = __fmul_rn(r, __fadd_rn(__fmul_rn(c1, mut), c2));
-  if (a.a2a.has(i, k, j)) t = __fadd_rn(t, r);
+  const bool inside = a.a2a.has(i, k, j);
+  if (inside) t = __fadd_rn(t, r);
+  return a.rt_tendf && (inside || a.rt_tendf_in != a.rt_tendf);
+}
+
+// Four consecutive elements of rt_tendf, those that `write` has a bit for.
+__device__ __forceinline__ void put4(float *p, const float (&t)[4], unsigned write) {
+  if (write == 15u) {
+    *reinterpret_cast<float4 *>(p) = make_float4(t[0], t[1], t[2], t[3]);
+  } else if (write) {
+#pragma unroll
+    for (int v = 0; v < 4; ++v)
+      if (write >> v & 1u) p[v] = t[v];
+  }
 }
 
 // Arrays that are not 16-byte aligned: one thread per element.
@@ -50,9 +66,9 @@ __global__ void __launch_bounds__(kThreads) tendency_kernel(const TendArgs a) {
     const float c1 = a.couple ? __ldg(a.c1 + k) : 0.0f, c2 = a.couple ? __ldg(a.c2 + k) : 0.0f;
     const float mut = a.couple ? __ldg(a.mut + static_cast<size_t>(i) * a.ny + j) : 0.0f;
     float r, t = a.rt_tendf ? a.rt_tendf_in[e] : 0.0f;
-    element(a, i, k, j, __ldg(a.lw + e), a.sw ? __ldg(a.sw + e) : 0.0f, c1, c2, mut, r, t);
+    const bool write = element(a, i, k, j, __ldg(a.lw + e), a.sw ? __ldg(a.sw + e) : 0.0f, c1, c2, mut, r, t);
     if (a.rthraten) a.rthraten[e] = r;
-    if (a.rt_tendf) a.rt_tendf[e] = t;
+    if (write) a.rt_tendf[e] = t;
   }
 }
 
@@ -75,15 +91,18 @@ __device__ __forceinline__ void tendency4(const TendArgs &a, int row, int j, flo
   }
   const float c1 = couple_row ? __ldg(a.c1 + k) : 0.0f, c2 = couple_row ? __ldg(a.c2 + k) : 0.0f;
   const bool add_row = (i >= a.a2a.i0) & (i < a.a2a.i1) & (k >= a.a2a.k0) & (k < a.a2a.k1);
+  unsigned write = a.rt_tendf && a.rt_tendf_in != a.rt_tendf ? 15u : 0u;  // in place: as element says
 #pragma unroll
   for (int q = 0; q < 4; ++q) {
     if (a.sw) r[q] = __fadd_rn(r[q], s[q]);
     if (couple_row && (j + q >= a.tile.j0) & (j + q < a.tile.j1)) r[q] = __fmul_rn(r[q], __fadd_rn(__fmul_rn(c1, m[q]), c2));
-    if (add_row && (j + q >= a.a2a.j0) & (j + q < a.a2a.j1)) tt[q] = __fadd_rn(tt[q], r[q]);
+    if (add_row && (j + q >= a.a2a.j0) & (j + q < a.a2a.j1)) {
+      tt[q] = __fadd_rn(tt[q], r[q]);
+      if (a.rt_tendf) write |= 1u << q;
+    }
   }
   if (a.rthraten) *reinterpret_cast<float4 *>(a.rthraten + e) = make_float4(r[0], r[1], r[2], r[3]);
-  if (a.rt_tendf && (add_row || a.rt_tendf_in != a.rt_tendf))
-    *reinterpret_cast<float4 *>(a.rt_tendf + e) = make_float4(tt[0], tt[1], tt[2], tt[3]);
+  put4(a.rt_tendf + e, tt, write);
 }
 
 __global__ void __launch_bounds__(kThreads) tendency_kernel_vec4(const TendArgs a) {
@@ -118,11 +137,12 @@ __device__ __forceinline__ void quad(const TendArgs &a, int n, int q, float4 lw,
   float r[4], tt[4] = {t.x, t.y, t.z, t.w};
   int row = e / a.ny, j = e - row * a.ny;
   int i = row / a.nk, k = row - i * a.nk;
+  unsigned write = 0u;
 #pragma unroll
   for (int v = 0; v < 4; ++v) {
     const float c1 = a.couple ? __ldg(a.c1 + k) : 0.0f, c2 = a.couple ? __ldg(a.c2 + k) : 0.0f;
     const float mut = a.couple ? __ldg(a.mut + static_cast<size_t>(i) * a.ny + j) : 0.0f;
-    element(a, i, k, j, l[v], s[v], c1, c2, mut, r[v], tt[v]);
+    write |= static_cast<unsigned>(element(a, i, k, j, l[v], s[v], c1, c2, mut, r[v], tt[v])) << v;
     if (++j == a.ny) {
       j = 0;
       if (++k == a.nk) {
@@ -132,7 +152,7 @@ __device__ __forceinline__ void quad(const TendArgs &a, int n, int q, float4 lw,
     }
   }
   if (a.rthraten) reinterpret_cast<float4 *>(a.rthraten)[q] = make_float4(r[0], r[1], r[2], r[3]);
-  if (a.rt_tendf) reinterpret_cast<float4 *>(a.rt_tendf)[q] = make_float4(tt[0], tt[1], tt[2], tt[3]);
+  put4(a.rt_tendf + e, tt, write);
 }
 
 __global__ void __launch_bounds__(kThreads) tendency_kernel_run4(const TendArgs a) {
@@ -160,9 +180,9 @@ __global__ void __launch_bounds__(kThreads) tendency_kernel_run4(const TendArgs 
     const float c1 = a.couple ? __ldg(a.c1 + k) : 0.0f, c2 = a.couple ? __ldg(a.c2 + k) : 0.0f;
     const float mut = a.couple ? __ldg(a.mut + static_cast<size_t>(i) * a.ny + j) : 0.0f;
     float r, tt = a.rt_tendf ? a.rt_tendf_in[e] : 0.0f;
-    element(a, i, k, j, __ldg(a.lw + e), a.sw ? __ldg(a.sw + e) : 0.0f, c1, c2, mut, r, tt);
+    const bool write = element(a, i, k, j, __ldg(a.lw + e), a.sw ? __ldg(a.sw + e) : 0.0f, c1, c2, mut, r, tt);
     if (a.rthraten) a.rthraten[e] = r;
-    if (a.rt_tendf) a.rt_tendf[e] = tt;
+    if (write) a.rt_tendf[e] = tt;
   }
 }
 
