@@ -706,9 +706,11 @@ struct SwOptics {
   float dbt, dbt_nd;
 };
 
-// The clear-sky layer's inputs that the cloudy one builds on.
+// The clear-sky layer's inputs that the cloudy one builds on, and whether the
+// checked form below served it.
 struct SwClear {
   float ztau, ztauc, zomcc, zgcc;
+  bool checked;
 };
 
 // Clear sky, any operands: gas + Rayleigh, no aerosol (sw:6923-6927).  Divisions
@@ -716,6 +718,7 @@ struct SwClear {
 template <bool kFp64>
 __device__ __forceinline__ SwOptics sw_clear_any(const Tables &T, float tg, float tr, float mu, SwClear &c) {
   SwOptics o;
+  c.checked = false;
   c.ztau = (tr + tg) + 0.0f;
   const float zom0 = tr + 0.0f * 1.0f;
   const float zgr = zero_over(zom0);  // 0 * 1 * 0 / zom
@@ -892,7 +895,8 @@ __device__ __forceinline__ SwOptics sw_cloudy_safe(const Tables &T, const SwClea
   const float scatg = tcld * wcld * gcld + 0.0f;  // the clear sky's share has zgcc = 0
   const float zg = quotient_in_range(scatg, scat);
   const float zw = quotient_in_range(scat, ztauo);
-  ok = ok && tcld >= 0.0f && taor >= 0.0f && taor <= kSafeHigh && ztauo <= kSafeHigh && scat >= kSafeLow &&
+  // (scat is at most ztauo where zw is at most 1: with 2^30 the quotient zg is at least 2^-120)
+  ok = ok && tcld >= 0.0f && taor >= 0.0f && taor <= kSafeHigh && ztauo <= 0x1p30f && scat >= kSafeLow &&
        scatg >= kSafeLow && zg <= 0.99f && zw >= 0x1p-30f && zw <= 1.0f;
   // whether zw / (1 - (1 - zw) (zg / (1 - zg))^2) reaches 0.9999995: far below
   // it by an approximate divisor, else by the reference's own quotients
@@ -1414,6 +1418,7 @@ __device__ __forceinline__ SwOptics sw_clear(const Tables &T, float tg, float tr
   } else {
     bool ok;
     SwOptics o = sw_clear_safe(T, tg, tr, mu, y_mu, c, ok);
+    c.checked = ok;
     if (!ok) o = sw_clear_slow(T, tg, tr, mu, c);
     return o;
   }
@@ -1425,7 +1430,7 @@ __device__ __forceinline__ SwOptics sw_cloudy(const Tables &T, const SwClear &c,
   if constexpr (kFp64) {
     return sw_cloudy_any<true>(T, c, oc, cld, mu);
   } else {
-    bool ok = c.zgcc == 0.0f && safe_size(c.ztau);
+    bool ok = c.checked;  // mu and the clear sky's operands
     SwOptics o = sw_cloudy_safe(T, c, cld, mu, y_mu, ok);
     if (!ok) o = sw_cloudy_slow(T, c, oc, cld, mu);
     return o;
