@@ -139,9 +139,10 @@ rrtmg_status rrtmg_swrad_live(rrtmg_ctx *ctx, const rrtmg_config *cfg, const rrt
  * which receives the workspace as one more result buffer from XLA's
  * allocator.  rrtmg_lw_workspace_bytes / rrtmg_sw_workspace_bytes return the
  * bytes a call with this config needs under the context's current schedule
- * (0 for an invalid config); they also build the context's McICA jump table
- * for the config's layer count, the one allocation a first call would
- * otherwise make, so call them during set-up.  The workspace is device memory
+ * (0 for an invalid config), no fewer for a larger domain, so that the largest
+ * one's workspace serves every smaller one.  They also build the context's
+ * McICA jump table for the config's layer count, the one allocation a first
+ * call would otherwise make, so call them during set-up.  The workspace is device memory
  * on the context's device, 256-byte aligned, at least that many bytes, and
  * must not be used by anything else until the call's work on `stream` is
  * done.  Results are those of rrtmg_lwrad / rrtmg_swrad bit for bit. */

@@ -85,6 +85,21 @@ def test_small_domains_equal_large_ones(ctx, nx, ny, nk, more, options):
         _assert_copies(small, big, nx, times, call.__name__)
 
 
+def test_a_larger_domains_workspace_serves_a_smaller_one(ctx):
+    """The workspace sizes do not fall as the domain grows, the end of the
+    small-chunk forms (2,048 columns) included."""
+    import ctypes
+    from wrf_jax_b200 import rrtmg
+    gases = dict(co2vmr=4.0e-4, n2ovmr=3.0e-7, ch4vmr=1.7e-6, yr=2024)
+    for name, config in (("lw", lambda n: rrtmg.lw_config(1, n, 50, p_top=5000.0, **gases)),
+                         ("sw", lambda n: rrtmg.sw_config(1, n, 50, solcon=1370.0, **gases))):
+        query = getattr(ctx.lib, f"rrtmg_{name}_workspace_bytes")
+        query.restype = ctypes.c_size_t
+        sizes = [query(ctx.handle, ctypes.byref(config(n)))
+                 for n in (1, 320, 384, 385, 2047, 2048, 2049, 2500, 3100, 5000, 16384, 16385, 32769, 100000)]
+        assert sizes[0] > 0 and sizes == sorted(sizes), (name, sizes)
+
+
 # kMaxBuf = 40 layers above the model top; a warp takes 30 of them (and two values of the top) at once
 @pytest.mark.parametrize("p_top", [500.0, 11600.0, 12000.0, 12400.0, 15900.0])
 def test_column_setup_by_warp_equals_by_thread(ctx, torch_cuda, p_top):

@@ -689,12 +689,20 @@ static size_t sw_chunk_columns(rrtmg_ctx *ctx, int ncol) {
   std::lock_guard<std::mutex> lk(ctx->mutex);
   return static_cast<size_t>(ncol < ctx->sw_chunk ? ncol : ctx->sw_chunk);
 }
+// Scratch floats of a chunk in a caller's workspace: `own`, what the chunk takes,
+// but no fewer than `small`, what one of kSmallColumns takes.  Chunks up to that
+// size need more per column (the small-chunk forms' records); so a workspace
+// serves every smaller domain of the same levels.
+static size_t workspace_floats(size_t chunk, size_t own, size_t small) {
+  return chunk > kSmallColumns && own < small ? small : own;
+}
 static size_t lw_workspace_bytes(rrtmg_ctx *ctx, const rrtmg_config *cfg) {
   const int nlay = rrtmg_lw_nlayers(cfg->p_top, cfg->nk);
   const size_t ncol = static_cast<size_t>(cfg->nx) * cfg->ny;
   const size_t chunk = lw_chunk_columns(ctx, static_cast<int>(ncol));
   return CallScratch::aligned(static_cast<size_t>(nlay) * kLwMaskWords * ncol * sizeof(uint32_t)) +
-         CallScratch::aligned(lw_scratch_floats(nlay, static_cast<int>(chunk)) * sizeof(float));
+         CallScratch::aligned(workspace_floats(chunk, lw_scratch_floats(nlay, static_cast<int>(chunk)),
+                                               lw_scratch_floats(nlay, kSmallColumns)) * sizeof(float));
 }
 static size_t sw_workspace_bytes(rrtmg_ctx *ctx, const rrtmg_config *cfg) {
   const int nlay = cfg->nk + 1;
@@ -702,7 +710,8 @@ static size_t sw_workspace_bytes(rrtmg_ctx *ctx, const rrtmg_config *cfg) {
   const size_t chunk = sw_chunk_columns(ctx, static_cast<int>(ncol));
   return CallScratch::aligned(static_cast<size_t>(nlay) * kSwMaskWords * ncol * sizeof(uint32_t)) +
          CallScratch::aligned((ncol + 1) * sizeof(int)) +
-         CallScratch::aligned(sw_record_floats(cfg->nk, static_cast<int>(chunk)) * sizeof(float));
+         CallScratch::aligned(workspace_floats(chunk, sw_record_floats(cfg->nk, static_cast<int>(chunk)),
+                                               sw_record_floats(cfg->nk, kSmallColumns)) * sizeof(float));
 }
 
 // live: null, or a device count; columns at or past it are skipped.  ws: null
