@@ -34,3 +34,41 @@ def test_trials_with_other_settings_are_not_candidates(pkg):
     best = {k: v for k, v in trials[0].items() if k != "ms"}
     pick, ms = prefer_fewer_streams(best, 310.0, trials)
     assert pick == best and ms == 310.0
+
+
+def test_autotune_leaves_the_gemm_tile_alone(pkg, monkeypatch):
+    """The GEMM's tile is a process-wide setting that no ensemble member uses: a
+    tuned ensemble leaves it as it was, by default the automatic choice, which
+    later training steps and unfused inference then take."""
+    import types
+
+    import torch
+    from wrf_jax_b200 import _capi, ensemble
+    tiles, clock = [], [0.0]
+    lib = types.SimpleNamespace(rrtmg_set_schedule=lambda handle, sch: 0,
+                                rrtmg_gemm_set_tile=lambda bn: tiles.append(bn) or 0)
+
+    class Event:
+        def __init__(self, enable_timing=False):
+            pass
+
+        def record(self):
+            self.at = clock[0]
+
+        def elapsed_time(self, end):
+            return end.at - self.at
+
+    class Runner:
+        ctx = types.SimpleNamespace(handle=None, check=lambda st: None)
+
+        def set_streams(self, n):
+            pass
+
+        def launch_all(self, fallback):
+            clock[0] += 1.0
+
+    monkeypatch.setattr(_capi, "load", lambda: lib)
+    monkeypatch.setattr(torch.cuda, "Event", Event)
+    monkeypatch.setattr(torch.cuda, "synchronize", lambda: None)
+    tuned = ensemble.autotune(Runner())
+    assert tuned["best_ms"] == 1.0 and not tiles

@@ -11,8 +11,8 @@ surrogate domain, are then gathered into one compact domain and solved by one
 plain LW + SW call (one fallback per step instead of one per domain).
 
 `autotune` picks the launch schedule (columns per launch of the plain kernels,
-the band-split limit of the SW kernel, the GEMM tile width, the number of
-streams) by timing candidate settings on the ensemble itself.
+the band-split limit of the SW kernel, the number of streams) by timing
+candidate settings on the ensemble itself.
 """
 
 from __future__ import annotations
@@ -315,7 +315,6 @@ def autotune(runner: EnsembleRunner, *, log=None) -> dict:
         sch = _capi.Schedule(lw_chunk_columns=cfg["lw_chunk"], sw_chunk_columns=cfg["sw_chunk"],
                              sw_split_max_columns=cfg["sw_split_max"], lw_split_max_columns=cfg["lw_split_max"])
         ctx.check(lib.rrtmg_set_schedule(ctx.handle, ctypes.byref(sch)))
-        S._check(lib.rrtmg_gemm_set_tile(cfg["gemm_tile"]), "gemm tile")
         runner.set_streams(cfg["streams"])
 
     def measure(cfg):
@@ -330,10 +329,10 @@ def autotune(runner: EnsembleRunner, *, log=None) -> dict:
         torch.cuda.synchronize()
         return ev0.elapsed_time(ev1) / 2
 
+    # (not the GEMM's tile: that setting is the process's, and no member runs the GEMM)
     space = dict(lw_chunk=[65536, 131072, 262144], sw_chunk=[65536, 131072, 262144],
-                 sw_split_max=[2048, 4096, 8192], lw_split_max=[1024, 2048, 4096], gemm_tile=[128, 256],
-                 streams=[1, 2, 4])
-    best = dict(lw_chunk=131072, sw_chunk=131072, sw_split_max=4096, lw_split_max=2048, gemm_tile=256, streams=4)
+                 sw_split_max=[2048, 4096, 8192], lw_split_max=[1024, 2048, 4096], streams=[1, 2, 4])
+    best = dict(lw_chunk=131072, sw_chunk=131072, sw_split_max=4096, lw_split_max=2048, streams=4)
     best_ms = measure(best)
     trials = [dict(best, ms=best_ms)]
     for key, values in space.items():
