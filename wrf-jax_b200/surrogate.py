@@ -294,8 +294,10 @@ class SurrogateModel:
             field = getattr(a, name)
             for i, t in enumerate(tensors):
                 field[i] = t.data_ptr()
-        if lib.rrtmg_sur_train_step(ctypes.byref(a), _stream()) != 0:
+        st = lib.rrtmg_sur_train_step(ctypes.byref(a), _stream())
+        if st == 1:  # RRTMG_BAD_ARG
             raise ValueError(f"rrtmg_sur_train_step rejected the arguments (batch {B}; a multiple of 128 is needed)")
+        _check(st, "rrtmg_sur_train_step")
         self.step = step
 
     # -- persistence ----------------------------------------------------------
