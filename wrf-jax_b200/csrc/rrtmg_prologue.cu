@@ -19,9 +19,11 @@ namespace {
 // 1000 x 50 x 1000, all outputs: 518 us before (five blocks of 256; the slopes
 // divided out in every column), 424 us so and 407 us with 32-bit indices; with
 // 64-bit ones 640 threads took 442 us, 768 596 us, five blocks of 256 610 us,
-// and inputs loaded two levels ahead 465 us.
-constexpr int kPrologueThreads = 512;
-constexpr int kPrologueBlocks = 2;  // per SM
+// and inputs loaded two levels ahead 465 us.  Without ozone there is no table
+// to stage and less to keep: five blocks of 256 (cloud fraction alone of 425 x
+// 50 x 425 59 us, of 1000 x 50 x 1000 304 us; two of 512 91 and 336 us).
+constexpr int prologue_threads(bool ozone) { return ozone ? 512 : 256; }
+constexpr int prologue_blocks(bool ozone) { return ozone ? 2 : 5; }  // per SM
 // Two blocks' slope rows and queues share an SM's 227 KB.
 constexpr size_t kSlopeRowsMax = 96 * 1024;
 
@@ -212,7 +214,7 @@ size_t slope_rows_bytes(int levsiz, int latsiz) {
 // Off: the type of an element's index, 32 bits where a field has fewer than 2^32
 // elements (424 us with 64 bits, 407 us with 32 at 1000 x 50 x 1000).
 template <bool kCld, bool kOz, bool kCz, bool kFlag, class Off>
-__global__ void __launch_bounds__(kPrologueThreads, kPrologueBlocks)
+__global__ void __launch_bounds__(prologue_threads(kOz), prologue_blocks(kOz))
 prologue_kernel(const PrologueArgs a, bool slopes) {
   // slopes: (latsiz - 1, levsiz) rows of OzoneColumn; otherwise
   // (2, latsiz, levsiz): month_lo, month_hi.  Then the levels and latitudes.
@@ -254,7 +256,7 @@ prologue_kernel(const PrologueArgs a, bool slopes) {
   // too, instead of read again, qv has to be read everywhere: 409 us at
   // 1000 x 50 x 1000 with 12% of the levels cloudy, 357 us instead of 334 us
   // with none.
-  __shared__ Off s_queue[kPrologueThreads / 32][64];
+  __shared__ Off s_queue[prologue_threads(kOz) / 32][64];
   Off *q = s_queue[threadIdx.x >> 5];
   int qn = 0, head = 0;  // warp-uniform
   auto drain = [&](int n) {
@@ -389,7 +391,7 @@ cudaError_t launch_variant(const PrologueArgs &a, int blocks, size_t smem, bool 
     cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(smem));
     if (e != cudaSuccess) return e;
   }
-  kern<<<blocks, kPrologueThreads, smem, stream>>>(a, slopes);
+  kern<<<blocks, prologue_threads(kOz), smem, stream>>>(a, slopes);
   return cudaGetLastError();
 }
 
@@ -414,8 +416,8 @@ cudaError_t launch_prologue(const PrologueArgs &a, cudaStream_t stream) {
                                : prologue_smem_bytes(a.levsiz, a.latsiz);
   // the ozone tables are staged once per block: a persistent grid of a few
   // blocks per SM when they are needed, one thread per column otherwise
-  const int need = (ncol + kPrologueThreads - 1) / kPrologueThreads;
-  const int blocks = oz ? std::min(need, sms * kPrologueBlocks) : need;
+  const int threads = prologue_threads(oz), need = (ncol + threads - 1) / threads;
+  const int blocks = oz ? std::min(need, sms * prologue_blocks(true)) : need;
   const int key = (cld ? 8 : 0) | (oz ? 4 : 0) | (cz ? 2 : 0) | (flag ? 1 : 0);
   switch (key) {
 #define RRTMG_PROLOGUE_CASE(K)                                                              \
