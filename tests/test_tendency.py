@@ -146,3 +146,23 @@ def test_gpu_in_place_tiles_on_two_streams(pkg, south_north, offset):
         want[b["its"] - 1:b["ite"], :nk - 1, b["jts"] - 1:b["jte"]] += passes
     assert torch.equal(t.cpu().view(nx, nk, ny), want)
     assert not flat[:offset].any() and not flat[offset + n:].any()
+
+
+@pytest.mark.gpu
+def test_gpu_result_stays_tied_to_a_tracked_input(pkg):
+    """rt_tendf with a gradient: the updated tendency is rt_tendf plus the heating,
+    with the gradient of a copy, and rt_tendf itself is left as it was."""
+    import torch
+    if not torch.cuda.is_available():
+        pytest.skip("no CUDA device")
+    from wrf_jax_b200 import tendency
+    b = dict(ids=1, ide=7, jds=1, jde=6, kds=1, kde=4, ims=1, ime=6, jms=1, jme=5, kms=1, kme=4, its=1, ite=6, jts=1,
+             jte=5, kts=1, kte=3)
+    lw, sw, t0 = (torch.randn(6, 4, 5, device="cuda") for _ in range(3))
+    c1, c2, mut = torch.rand(4, device="cuda"), torch.rand(4, device="cuda"), torch.rand(6, 5, device="cuda")
+    r, plain = tendency.radiation_tendency(lw, sw, c1, c2, mut, t0, {}, **b)
+    tracked = t0.clone().requires_grad_()
+    _, t = tendency.radiation_tendency(lw, sw, c1, c2, mut, tracked, {}, **b)
+    assert torch.equal(t, plain) and torch.equal(tracked, t0)
+    t.sum().backward()
+    assert torch.equal(tracked.grad, torch.ones_like(t0))

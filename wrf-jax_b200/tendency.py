@@ -70,7 +70,9 @@ def radiation_tendency(rthratenlw, rthratensw, c1, c2, mut, rt_tendf, config_fla
                    or tuple(d["mut"].shape) != (shape[0], shape[2])):
         raise ValueError("c1/c2 must have kme-kms+1 values and mut (ime-ims+1, jme-jms+1)")
     r = torch.empty(shape, dtype=torch.float32, device=d["lw"].device)
-    t = torch.empty_like(d["t"])
+    # a clone where rt_tendf takes part in a gradient: the result then stays tied to it
+    tied = torch.is_grad_enabled() and d["t"].requires_grad
+    t = d["t"].clone() if tied else torch.empty_like(d["t"])
     s = stream if stream is not None else torch.cuda.current_stream().cuda_stream
     lib = _capi.load()
     _check(lib.rrtmg_radiation_tendency_into(ctypes.byref(tb), d["lw"].data_ptr(), d["sw"].data_ptr(),
