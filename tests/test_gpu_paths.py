@@ -207,3 +207,26 @@ def test_training_step_batches(torch_cuda, batch):
     # the next step's weights: the master copies rounded, and their transposes
     for master, rounded, transposed in zip(model.w, model.wb, model.wbt):
         assert torch.equal(master.to(torch.bfloat16), rounded) and torch.equal(rounded.t(), transposed)
+
+
+@pytest.mark.parametrize("batch", [1024, 6272, 16384])
+def test_weight_gradients_of_large_batches(torch_cuda, batch):
+    """The weight gradients against the same products in 64 bits.  A split of the
+    batch sums at most 1,024 rows in the tensor cores, 64 instructions that may
+    each lose a binary32 unit (2^-24) of the running sum, half of one on average:
+    64 * 2^-25 = 1.9e-6 of the gradient's norm; 2e-6 with the splits' own sums."""
+    torch = torch_cuda
+    from wrf_jax_b200 import surrogate as S
+    model = S.SurrogateModel(seed=6)
+    g = torch.Generator(device="cuda").manual_seed(batch)
+    X = torch.randn(batch, S.K_IN, device="cuda", generator=g).bfloat16()
+    Tn = torch.randn(batch, S.N_OUT, device="cuda", generator=g)
+    idx = torch.randperm(batch, device="cuda", generator=g).to(torch.int32)
+    model.train_step(X, Tn, idx, S.target_weights(), lr=0.0)
+    torch.cuda.synchronize()
+    assert S.gemm_error() == 0
+    b = model._buf
+    for layer, (grad, inputs) in enumerate(zip([*b["dZt"], b["dYt"]], [b["Xbt"], *b["Ht"]])):
+        want = grad.double() @ inputs.double().t()
+        err = float((b["gw"][layer].double() - want).norm() / want.norm())
+        assert err < 2e-6, (layer, err)
