@@ -554,8 +554,11 @@ __device__ __forceinline__ float adam_element(const P &p, float g, float w0, flo
 }
 
 // Bias gradients and their Adam step: one block per bias sums its row of the
-// transposed gradient.  Bound by HBM / L2; one 2-byte load per thread took 32 us
-// per layer at 16,384 rows.
+// transposed gradient, eight values of a load pairwise and the warps' sums
+// likewise (error against 64 bits at 16,384 rows 4.0e-8 to 4.6e-8 of the layers'
+// gradients, as by row_sum_kernel; one value after the other 5.1e-8 to 6.2e-8).
+// Bound by HBM / L2; one 2-byte load per
+// thread took 32 us per layer at 16,384 rows.
 __global__ void __launch_bounds__(256) bias_update_kernel(const __grid_constant__ SurUpdateArgs a) {
   int layer = 0, row = blockIdx.x;
   while (row >= a.rows[layer]) row -= a.rows[layer++];
@@ -563,12 +566,8 @@ __global__ void __launch_bounds__(256) bias_update_kernel(const __grid_constant_
   float acc = 0.0f;
   for (int q = threadIdx.x; q < a.batch / 8; q += 256) {
     const uint4 v = __ldg(g + q);
-    const uint32_t u[4] = {v.x, v.y, v.z, v.w};
-#pragma unroll
-    for (int e = 0; e < 4; ++e) {
-      acc += __uint_as_float(u[e] << 16);
-      acc += __uint_as_float(u[e] & 0xffff0000u);
-    }
+    auto pair = [](uint32_t u) { return __uint_as_float(u << 16) + __uint_as_float(u & 0xffff0000u); };
+    acc += (pair(v.x) + pair(v.y)) + (pair(v.z) + pair(v.w));
   }
   __shared__ float part[8];
 #pragma unroll
@@ -576,9 +575,7 @@ __global__ void __launch_bounds__(256) bias_update_kernel(const __grid_constant_
   if ((threadIdx.x & 31) == 0) part[threadIdx.x >> 5] = acc;
   __syncthreads();
   if (threadIdx.x == 0) {
-    float s = part[0];
-#pragma unroll
-    for (int w = 1; w < 8; ++w) s += part[w];
+    const float s = ((part[0] + part[1]) + (part[2] + part[3])) + ((part[4] + part[5]) + (part[6] + part[7]));
     a.gb[layer][row] = s;
     float m = a.mb[layer][row], v = a.vb[layer][row];
     SurUpdateArgs p = a;
