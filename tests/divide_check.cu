@@ -33,8 +33,9 @@ __device__ __forceinline__ uint64_t next(uint64_t &s) {  // xorshift64
   return s;
 }
 
-// random operands, among them significands near 2 and near 1 and quotients next
-// to the midpoint of two neighbours
+// random operands over the whole ranges of rrtmg_divide.cuh, of either sign,
+// among them significands near 2 and near 1, quotients next to the midpoint of
+// two neighbours, and numerators, divisors and quotients at the ranges' ends
 __global__ void quotients(int n, uint64_t seed) {
   uint64_t s = seed + (blockIdx.x * blockDim.x + threadIdx.x + 1) * 0x9E3779B97F4A7C15ull;
   unsigned bad = 0;
@@ -43,9 +44,16 @@ __global__ void quotients(int n, uint64_t seed) {
     unsigned ma = static_cast<unsigned>(r >> 23) & 0x7fffffu, mb = static_cast<unsigned>(r) & 0x7fffffu;
     if ((i & 3) == 1) mb |= 0x7fff00u;
     if ((i & 3) == 2) ma &= 0xffu;
-    const float b = binary32(static_cast<int>(x % 81) - 40, mb);
-    float a = binary32(static_cast<int>((x / 81) % 81) - 40, ma);
+    int eb = static_cast<int>(x % 200) - 100, ea = static_cast<int>(x / 200 % 200) - 100;
+    if ((i & 28) == 4) eb = i & 32 ? 99 : -100;
+    if ((i & 28) == 8) ea = i & 32 ? 99 : -100;
+    if ((i & 28) == 12) eb = ea + 119;  // the smallest quotients
+    if ((i & 28) == 16) eb = ea - 117;  // the largest
+    if (eb < -100 || eb > 99 || ea - eb < -119 || ea - eb > 117) continue;
+    const float b = x >> 40 & 1u ? -binary32(eb, mb) : binary32(eb, mb);
+    float a = x >> 41 & 1u ? -binary32(ea, ma) : binary32(ea, ma);
     if ((i & 3) == 3) a = static_cast<float>(static_cast<double>(__fdiv_rn(a, b)) * (1.0 + 0x1p-24) * b);
+    if (fabsf(a) < 0x1p-100f) continue;
     if (i == 0) a = 0.0f;
     bad += __float_as_uint(rrtmg::quotient_in_range(a, b)) != __float_as_uint(__fdiv_rn(a, b));
   }

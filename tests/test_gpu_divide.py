@@ -1,6 +1,7 @@
 """csrc/rrtmg_divide.cuh against IEEE division, bit for bit: the reciprocal of
-every binary32 significand at all exponents of its range, and 2.5e9 quotients
-with operands chosen next to the hard cases."""
+every binary32 significand at all exponents of its range, and some 1.5e9
+quotients with operands chosen next to the hard cases and at the ends of their
+ranges; and the shortwave layer optics that use it against their general form."""
 
 from __future__ import annotations
 

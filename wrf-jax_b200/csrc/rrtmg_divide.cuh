@@ -11,8 +11,9 @@
 //     significand (checked exhaustively, tests/test_gpu_divide.py);
 //   * q = a y, corrected by its exact remainder, is within one unit in the
 //     last place, and corrected once more it is the correctly rounded a / b.
-// Ranges: |b| in [2^-100, 2^100], |a| in [2^-90, 2^100] (a positive zero is
-// fine), and the quotient within [2^-100, 2^100].
+// Ranges: |b| and |a| in [2^-100, 2^100] (a positive zero a is fine), and the
+// quotient's size in [2^-120, 2^117].  There no step leaves the normal numbers and
+// the remainder a - b q, a multiple of 2^-148, is exact.
 #pragma once
 
 namespace rrtmg {
