@@ -22,15 +22,16 @@ pytestmark = pytest.mark.gpu
 RRTMG_OK, RRTMG_BAD_ARG, RRTMG_TIMEOUT = 0, 1, 4
 
 
-@pytest.fixture()
-def gemm_env(pkg):
+@pytest.fixture(params=[0, 128, 256], ids=["auto", "tile128", "tile256"])
+def gemm_env(request, pkg):
     import torch
     if not torch.cuda.is_available():
         pytest.skip("no CUDA device")
     from wrf_jax_b200 import _capi, surrogate
     lib = _capi.load()
-    assert lib.rrtmg_gemm_set_tile(0) == RRTMG_OK
+    assert lib.rrtmg_gemm_set_tile(request.param) == RRTMG_OK
     yield torch, lib, surrogate, _capi
+    lib.rrtmg_gemm_set_tile(0)
     lib.rrtmg_gemm_test_withhold_commit(0)
     lib.rrtmg_gemm_set_wait_ns(0)
     torch.cuda.synchronize()
@@ -47,7 +48,7 @@ def _args(_capi, A, B, C, M, N, K):
 
 def test_withheld_commit_times_out_then_next_call_is_exact(gemm_env):
     torch, lib, surrogate, _capi = gemm_env
-    M, N, K = 256, 256, 256  # 4 K blocks > 3 pipeline stages of the 256-wide tile
+    M, N, K = 256, 256, 256  # 4 K blocks > 3 pipeline stages
     g = torch.Generator(device="cuda").manual_seed(3)
     A = torch.randn(M, K, device="cuda", generator=g).bfloat16()
     B = (torch.randn(N, K, device="cuda", generator=g) / K ** 0.5).bfloat16()

@@ -1,7 +1,9 @@
 """tcgen05 BF16 GEMM of the surrogate against a plain torch fp32 reference of
 the same op (fp32 matmul of the bf16-rounded operands).  Tolerances: fp32
 accumulation in a different order, |diff| <= 1e-4 * sqrt(K) * scale; bf16
-outputs within one bf16 rounding (relative 2^-8) of the reference value."""
+outputs within one bf16 rounding (relative 2^-8) of the reference value.  Every
+test runs with the automatic tile width (64, or 128 from 75 tiles of 128 on),
+with 128 and with 256 (where N allows it, else 128)."""
 
 from __future__ import annotations
 
@@ -18,6 +20,15 @@ def torch_cuda(pkg):
     return torch
 
 
+@pytest.fixture(params=[0, 128, 256], ids=["auto", "tile128", "tile256"], autouse=True)
+def tile(request, torch_cuda):
+    from wrf_jax_b200 import _capi
+    lib = _capi.load()
+    assert lib.rrtmg_gemm_set_tile(request.param) == 0
+    yield request.param
+    assert lib.rrtmg_gemm_set_tile(0) == 0
+
+
 def _operands(torch, M, N, K, seed):
     g = torch.Generator(device="cuda").manual_seed(seed)
     A = torch.randn(M, K, device="cuda", generator=g).bfloat16()
@@ -27,7 +38,8 @@ def _operands(torch, M, N, K, seed):
 
 
 @pytest.mark.parametrize("M,N,K,ksplit", [(128, 128, 64, 1), (256, 384, 512, 1), (512, 128, 1024, 4),
-                                         (384, 512, 192, 1), (256, 256, 2048, 8)])
+                                         (384, 512, 192, 1), (256, 256, 2048, 8), (9472, 128, 512, 1),
+                                         (9600, 128, 512, 1)])
 def test_gemm_f32_matches_torch(torch_cuda, M, N, K, ksplit):
     torch = torch_cuda
     from wrf_jax_b200 import surrogate, _capi
@@ -41,10 +53,11 @@ def test_gemm_f32_matches_torch(torch_cuda, M, N, K, ksplit):
     torch.testing.assert_close(got, ref, rtol=1e-4, atol=1e-4 * K ** 0.5)
 
 
-def test_gemm_gelu_epilogue(torch_cuda):
+@pytest.mark.parametrize("M", [256, 4864])  # 4 and 76 tiles of 128 x 128
+def test_gemm_gelu_epilogue(torch_cuda, M):
     torch = torch_cuda
     from wrf_jax_b200 import surrogate, _capi
-    M, N, K = 256, 256, 512
+    N, K = 256, 512
     A, B, bias = _operands(torch, M, N, K, 2)
     Z = torch.empty(M, N, device="cuda")
     H = torch.empty(M, N, device="cuda", dtype=torch.bfloat16)
@@ -61,10 +74,11 @@ def test_gemm_gelu_epilogue(torch_cuda):
     torch.testing.assert_close(Ht.float().T, H.float(), rtol=0, atol=0)
 
 
-def test_gemm_dgelu_epilogue(torch_cuda):
+@pytest.mark.parametrize("M", [128, 4864])
+def test_gemm_dgelu_epilogue(torch_cuda, M):
     torch = torch_cuda
     from wrf_jax_b200 import surrogate, _capi
-    M, N, K = 128, 256, 256
+    N, K = 256, 256
     A, B, _ = _operands(torch, M, N, K, 3)
     aux = torch.randn(M, N, device="cuda")
     H = torch.empty(M, N, device="cuda", dtype=torch.bfloat16)
