@@ -149,3 +149,17 @@ def test_set_ozone_rejects_bad_climatology_without_gpu(pkg):
     ptr = lambda a: a.ctypes.data_as(ctypes.c_void_p)
     assert lib.rrtmg_set_ozone_climatology(None, ptr(plev), 3, ptr(lat), 2, ptr(oz)) == 1
     assert lib.rrtmg_radiation_prologue(None, 1, 1, 1, None, None, None, None) == 1
+
+
+def test_fourth_root_by_two_square_roots():
+    """The cloud fraction's fourth root, two rounded binary32 square roots, over
+    every significand at four consecutive exponents (the pattern repeats with
+    them): within 0.5 + sqrt(2) / 4 units in the last place of the exact root."""
+    worst = 0.0
+    significand = np.arange(1 << 23, dtype=np.uint32)
+    for exponent in range(124, 128):
+        x = (significand | np.uint32(exponent << 23)).view(np.float32)
+        got = np.sqrt(np.sqrt(x))
+        want = np.sqrt(np.sqrt(x.astype(np.float64)))
+        worst = max(worst, float((np.abs(got - want) / np.spacing(want.astype(np.float32))).max()))
+    assert 0.8 < worst <= 0.5 + 2.0 ** 0.5 / 4.0

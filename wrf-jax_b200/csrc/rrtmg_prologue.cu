@@ -169,7 +169,8 @@ __device__ __forceinline__ float cal_cldfra1(float qv, float qc, float qi, float
   float arg = __fdiv_rn(__fmul_rn(-100.0f, qcld), powf(subsat, 0.49f));
   arg = (arg < -6.9f) ? -6.9f : arg;
   const float rpos = (rhum < 1.0e-10f) ? 1.0e-10f : rhum;
-  // the fourth root as two rounded square roots: within 0.75 units in the last place
+  // the fourth root as two rounded square roots: within 0.86 units in the last place (the first's half unit
+  // is at most sqrt(2) / 4 of one in the result, whose own rounding adds 0.5)
   const float partial = __fmul_rn(__fsqrt_rn(__fsqrt_rn(rpos)), __fsub_rn(1.0f, expf(arg)));
   return (partial < 0.01f) ? 0.0f : partial;
 }
