@@ -130,7 +130,8 @@ rrtmg_status rrtmg_sur_adam(const rrtmg_sur_adam_args *args, void *stream);
  * is a multiple of 128.  The buffers are the caller's: Xb, H, dZ [batch][512]
  * and dY [batch][128] BF16, their transposes Xbt, Ht, dZt [512][batch] and dYt
  * [128][batch], Z [batch][512], Tb and Y [batch][128] FP32, and part of
- * rrtmg_sur_train_part_floats(batch) floats; all 16-byte aligned. */
+ * rrtmg_sur_train_part_floats(batch) floats; these and wb, wbt are 16-byte
+ * aligned. */
 typedef struct {
     const void *X; int ldx;              /* normalized inputs (BF16), 512 columns */
     const float *T; int ldt;             /* normalized targets, 128 columns */

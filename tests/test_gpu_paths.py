@@ -230,3 +230,25 @@ def test_weight_gradients_of_large_batches(torch_cuda, batch):
         want = grad.double() @ inputs.double().t()
         err = float((b["gw"][layer].double() - want).norm() / want.norm())
         assert err < 2e-6, (layer, err)
+
+
+def test_training_step_with_weights_at_any_element(torch_cuda):
+    """FP32 weights and moments that are views at odd elements of larger buffers:
+    the same bits as with tensors of their own."""
+    torch = torch_cuda
+    from wrf_jax_b200 import surrogate as S
+    g = torch.Generator(device="cuda").manual_seed(4)
+    X = torch.randn(256, S.K_IN, device="cuda", generator=g).bfloat16()
+    Tn = torch.randn(256, S.N_OUT, device="cuda", generator=g)
+    idx = torch.arange(256, device="cuda", dtype=torch.int32)
+    own, views = S.SurrogateModel(seed=9), S.SurrogateModel(seed=9)
+    for name, shift in (("w", 1), ("mw", 2), ("vw", 3), ("b", 1), ("mb", 1), ("vb", 1)):
+        tensors = getattr(views, name)
+        for i, t in enumerate(tensors):
+            tensors[i] = torch.cat([torch.zeros(shift, device="cuda"), t.flatten()])[shift:].view(t.shape)
+            assert tensors[i].data_ptr() % 16
+    for model in (own, views):
+        model.train_step(X, Tn, idx, S.target_weights(), lr=1.0e-3, weight_decay=0.01)
+    for name in ("w", "mw", "vw", "b", "mb", "vb", "wb", "wbt"):
+        for a, b in zip(getattr(own, name), getattr(views, name)):
+            assert torch.equal(a, b), name

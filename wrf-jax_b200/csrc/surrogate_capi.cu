@@ -197,10 +197,9 @@ extern "C" rrtmg_status rrtmg_sur_train_step(const rrtmg_sur_train_args *a, void
     if (!p || !aligned16(p)) return RRTMG_BAD_ARG;
   if (!a->X || !a->T || !a->idx || !a->weights || !a->loss) return RRTMG_BAD_ARG;
   for (int i = 0; i < kTrainLayers; ++i) {
-    const void *per[] = {a->w[i], a->mw[i], a->vw[i], a->gw[i], a->wb[i], a->wbt[i]};
-    for (const void *p : per)
-      if (!p || !aligned16(p)) return RRTMG_BAD_ARG;
-    if (!a->b[i] || !a->mb[i] || !a->vb[i] || !a->gb[i]) return RRTMG_BAD_ARG;
+    if (!a->wb[i] || !aligned16(a->wb[i]) || !a->wbt[i] || !aligned16(a->wbt[i])) return RRTMG_BAD_ARG;
+    if (!a->w[i] || !a->mw[i] || !a->vw[i] || !a->gw[i] || !a->b[i] || !a->mb[i] || !a->vb[i] || !a->gb[i])
+      return RRTMG_BAD_ARG;
   }
   for (int i = 0; i < 3; ++i) {
     const void *per[] = {a->Z[i], a->H[i], a->Ht[i], a->dZ[i], a->dZt[i]};
@@ -286,6 +285,7 @@ extern "C" rrtmg_status rrtmg_sur_train_step(const rrtmg_sur_train_args *a, void
     group[i] = g;
     u.rows[i] = rows;
     u.cols[i] = kTrainWidth;
+    u.aligned[i] = aligned16(a->w[i]) && aligned16(a->mw[i]) && aligned16(a->vw[i]) && aligned16(a->gw[i]);
     u.gt[i] = g.A;
     u.part[i] = part;
     u.w[i] = a->w[i]; u.mw[i] = a->mw[i]; u.vw[i] = a->vw[i]; u.gw[i] = a->gw[i];

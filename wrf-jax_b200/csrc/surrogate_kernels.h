@@ -85,6 +85,7 @@ cudaError_t launch_sur_adam(const SurAdamArgs &a, cudaStream_t s);
 struct SurUpdateArgs {
   int layers, splits, batch;
   int rows[4], cols[4];
+  int aligned[4];              // w, mw, vw and gw are 16-byte aligned
   const __nv_bfloat16 *gt[4];  // d(pre-activation)^T [rows][batch]
   const float *part[4];        // splits slabs of rows x cols
   float *w[4], *mw[4], *vw[4], *gw[4], *b[4], *mb[4], *vb[4], *gb[4];

@@ -601,8 +601,21 @@ __global__ void __launch_bounds__(256) weight_update_kernel(const __grid_constan
   const int r0 = t / (cols / 32) * 32, c0 = t % (cols / 32) * 32;
   const int r = threadIdx.x >> 3, c = (threadIdx.x & 7) * 4;
   const size_t at = static_cast<size_t>(r0 + r) * cols + c0 + c;
-  auto ld = [&](const float *p) { return *reinterpret_cast<const float4 *>(p + at); };
-  auto st = [&](float *p, const float (&v)[4]) { *reinterpret_cast<float4 *>(p + at) = make_float4(v[0], v[1], v[2], v[3]); };
+  // (the caller's weights and moments may lie at any element)
+  const bool vec = a.aligned[layer] != 0;
+  auto ld = [&](const float *p) {
+    p += at;
+    return vec ? *reinterpret_cast<const float4 *>(p) : make_float4(p[0], p[1], p[2], p[3]);
+  };
+  auto st = [&](float *p, const float (&v)[4]) {
+    p += at;
+    if (vec) {
+      *reinterpret_cast<float4 *>(p) = make_float4(v[0], v[1], v[2], v[3]);
+    } else {
+#pragma unroll
+      for (int e = 0; e < 4; ++e) p[e] = v[e];
+    }
+  };
   const size_t slab = static_cast<size_t>(rows) * cols;
   float4 s = ld(a.part[layer]);
   for (int z = 1; z < a.splits; ++z) {
