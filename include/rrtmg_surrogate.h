@@ -232,8 +232,8 @@ rrtmg_status rrtmg_sur_move_fields(const int *list, const int *count, int max_n,
                                    int to_compact, int stride, int offset, void *stream);
 
 /* GEMM tile width: 0 = automatic (128 columns, 64 where 128 would leave SMs
- * idle), or 128 / 256 (256 needs N % 256 == 0; narrower N falls back to 128).  Process-
- * wide; set by the ensemble autotuner. */
+ * idle), or 128 / 256 (256 needs N % 256 == 0; narrower N falls back to 128).
+ * Process-wide. */
 rrtmg_status rrtmg_gemm_set_tile(int bn);
 
 /* Synchronous: reads the sticky flag that a CTA of rrtmg_gemm_bf16 or

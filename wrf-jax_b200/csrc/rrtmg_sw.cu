@@ -1,5 +1,5 @@
-// RRTMG shortwave on the GPU: one thread per column, fused from the WRF adapter
-// to the theta tendencies and the 2-D surface/TOA fields.
+// RRTMG shortwave on the GPU: the sweep schedule, from the WRF adapter to the
+// theta tendencies and the 2-D surface/TOA fields.
 //
 // Reference call: rrtmg_swrad_wrf_columns (src/wrf_jax/physics/module_ra_rrtmg_sw.py:2386)
 // and below it: inatm_sw (sw:1250), cldprmc_sw (sw:1409), setcoef_sw (sw:7101),
@@ -8,14 +8,13 @@
 // The adapter passes rounding_token=None, so every statement is one binary32
 // operation in the order written.
 //
-// Schedule.  Night columns (coszr <= 0) write zeros and exit: the reference
-// masks every output of such columns.  For a day column the thread walks the
-// 14 bands; per band it evaluates the band's gas optics for all layers once
-// (thread-local tables of taug/taur and the band's cloud optics), then for each
-// g-point runs a top-down pass (delta-Eddington layer reflectance and
+// Night columns (coszr <= 0) get zeros: the reference masks every output of such
+// columns.  Day columns are listed and taken in chunks; per chunk the column and
+// layer set-up, then every band's gas and cloud optics into layer records, then
+// per g-point a top-down pass (delta-Eddington layer reflectance and
 // transmittance, direct beam, downward adding recurrence) and a bottom-up pass
-// (upward adding recurrence, level fluxes) that accumulates the spectral sums
-// in g-point order.
+// (upward adding recurrence, level fluxes) whose spectral sums are taken in
+// g-point order (see "Sweep schedule" below).
 #include "rrtmg_device.cuh"
 #include "rrtmg_divide.cuh"
 #include "rrtmg_kernels.h"
